@@ -610,6 +610,33 @@ def test_sampler_against_plain(V):
     assert all(logits[4, t] >= kth for t in got)
 
 
+@pytest.mark.parametrize("V, ld", [(5, 8), (31, 33), (517, 517), (50257, 50257), (151936, 151936), (400004, 400004)])
+def test_sampler_shares_of_a_row(V, ld):
+    """A row is shared out to eight CTAs: shares without tokens, rows that are not 16-byte aligned, shares that shared
+    memory does not hold; draws from the first to the last token; rows whose masses are all one number, rows with two
+    tokens left, with nothing but minus infinity, with values that are not numbers."""
+    import struct
+
+    k = _k()
+    g = torch.Generator().manual_seed(43)
+    wide = torch.randn(9, ld, generator=g) * 3
+    logits = wide[:, :V]
+    logits[2] = 1.5
+    logits[3] = -float("inf")
+    logits[3, V // 2] = logits[3, V - 1] = 0.0
+    logits[4] = -float("inf")
+    logits[5, : V // 3] = float("nan")
+    rows = [(0.8, 0, 0.9, 0.0), (0.8, 0, 0.9, 0.99999994), (1.0, 0, 0.95, 0.51), (1.0, 0, 0.9, 0.75), (1.0, 0, 0.9, 0.4),
+            (1.0, 0, 1.0, 0.3), (1.2, 3, 1.0, 0.6), (0.5, 4, 0.7, 0.2), (0.0, 0, 0.9, 0.3)]
+    params = torch.frombuffer(bytearray(b"".join(struct.pack("<fiff", *r) for r in rows)), dtype=torch.uint8).to(DEV)
+    out = torch.full((9,), -1, dtype=torch.int32, device=DEV)
+    k.sample(wide.to(DEV)[:, :V], params, out)
+    got = out.cpu().tolist()
+    clean = torch.where(torch.isnan(logits), torch.full_like(logits, -float("inf")), logits)
+    want = [0 if i == 4 else P.sample_plain(clean[i], *rows[i]) for i in range(9)]
+    assert got == want and got[3] == V - 1
+
+
 @pytest.mark.parametrize("V, ld", [(517, 517), (1000, 1003), (151936, 151936), (5, 8), (64, 64)])
 def test_argmax_rows(V, ld):
     """Greedy sampling of every row by clusters of eight CTAs: the largest value, ties to the lowest id, the same
