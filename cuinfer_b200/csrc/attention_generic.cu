@@ -3,13 +3,13 @@
 //
 // Reference counterpart: csrc/ops/paged_attention.cu:133-383 (one kernel for prompt portions and
 // decoded tokens; queries are the last n positions of seq_len, keys 0..seq_len-1 come from pages;
-// scale 1/sqrt(d); causal mask; online softmax in 32 bits).  This kernel is the 32-bit path and the
-// fallback for head sizes the tensor-core kernels do not take: any head_dim up to 256, any head
+// scale 1/sqrt(d); causal mask; online softmax in 32 bits).  This kernel is the fallback for head sizes that the
+// tensor-core kernels and, in 32 bits, attention_f32.cu do not take: any head_dim up to 256, any head
 // counts, any page size, an optional window.  Scores, softmax and the weighted sum are 32-bit with
 // the exact exponential; the weights are not rounded before they multiply the values.
 //
 // Cache layout of one layer: [page][0 = keys, 1 = values][kv head][slot in page][d].
-#include "common.cuh"
+#include "attention_f32.cuh"
 
 namespace cib {
 
@@ -112,6 +112,11 @@ extern "C" int cib_paged_attention_generic(const void* q, int dtype, int q_strid
     CIB_REQUIRE(page_size > 0 && num_pages > 0 && table_stride > 0, "paged_attention: bad cache geometry");
     CIB_REQUIRE(window >= 0, "paged_attention: window must be >= 0 (0 = all keys)");
     if (num_tokens == 0) return 0;
+    if (dtype == kF32) {
+        const AttnF32 p{(const float*)q, (float*)out, (const float*)cache, block_table, query_start_loc, seq_lens, token_request,
+                        q_stride, out_stride, num_pages, page_size, table_stride, num_tokens, nq, nkv, window, scale};
+        if (const int rc = attention_f32_try(p, d, stream)) return rc > 0 ? 0 : rc;
+    }
     dim3 grid(num_tokens, (nq + kAttnWarps - 1) / kAttnWarps);
     const size_t smem = (size_t)kAttnWarps * d * sizeof(float);
     if (dtype == kF32) {

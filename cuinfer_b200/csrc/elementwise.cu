@@ -74,6 +74,7 @@ template <typename TD, typename TO, int V>
 __global__ void add_rmsnorm_kernel(float* __restrict__ residual, const TD* __restrict__ delta,
                                    AnyVec weight, float eps, TO* __restrict__ out, int hidden) {
     __shared__ float scratch[33];
+    griddep_launch();        // the product after this one may ask for its weights meanwhile
     const size_t row = (size_t)blockIdx.x * hidden;
     float* res = residual + row;
     float ss = 0.f;
@@ -190,6 +191,7 @@ __global__ void gather_rows_kernel(const float* __restrict__ residual, const TD*
 // exact exponential.
 template <typename T, int V>
 __global__ void silu_mul_kernel(const T* __restrict__ gate_up, T* __restrict__ act, int inter, int rows, int gelu) {
+    griddep_launch();        // the product after this one may ask for its weights meanwhile
     const int per_row = inter / V;
     const size_t total = (size_t)rows * per_row;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;

@@ -1,16 +1,15 @@
 // out[M, N] = a[M, K] · w[N, K]^T on the ordinary 32-bit FMA pipe, for any M, N, K.
 //
 // The reference sends every projection to cuBLAS with 32-bit accumulation
-// (csrc/ops/projection.cu:13-45).  This kernel is the true 32-bit path (no tensor cores, no reduced
-// precision mode) and the fallback for shapes the tensor-core kernels refuse.  Every output element
-// is a sum of fused-multiply-add chains of kBK values each, in the order of k (a chain of its own per
-// tile keeps the rounding of a long K from growing with its running sum), so a row's result does not
-// depend on how many other rows are in the batch.
-#include "common.cuh"
+// (csrc/ops/projection.cu:13-45).  This kernel is the fallback for shapes that the tensor-core kernels and the
+// 32-bit kernels of gemm_f32.cu refuse (rows off 16-byte boundaries).  Every output element adds in the order that
+// gemm_f32.cuh lays down, so a row's result depends neither on how many other rows are in the batch nor, in 32 bits, on
+// which kernel its address lets through.
+#include "gemm_f32.cuh"
 
 namespace cib {
 
-constexpr int kBM = 64, kBN = 64, kBK = 16;
+constexpr int kBM = 64, kBN = 64, kBK = kF32Chain;
 
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
@@ -27,11 +26,8 @@ gemm_generic_kernel(const TI* __restrict__ a, int lda, const TI* __restrict__ w,
     const int tid = threadIdx.x;
     const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
     const int tx = tid & 15, ty = tid >> 4;       // 16 x 16 threads, 4 x 4 outputs each
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const int group_k = f32_group_slices(K) * kF32Slice;
+    float slice[4][4] = {}, group[4][4] = {}, total[4][4] = {};
 
     // each thread loads 4 elements of each tile per step: row = tid / 4, k = (tid % 4) * 4 ..
     const int lrow = tid >> 2, lk = (tid & 3) * 4;
@@ -60,7 +56,20 @@ gemm_generic_kernel(const TI* __restrict__ a, int lda, const TI* __restrict__ w,
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+            for (int j = 0; j < 4; ++j) slice[i][j] += part[i][j];
+        const int done = k0 + kBK;
+        if (done % kF32Slice == 0 || done >= K) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { group[i][j] += slice[i][j]; slice[i][j] = 0.f; }
+            if (done % group_k == 0 || done >= K) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { total[i][j] += group[i][j]; group[i][j] = 0.f; }
+            }
+        }
         __syncthreads();
     }
 #pragma unroll
@@ -70,7 +79,7 @@ gemm_generic_kernel(const TI* __restrict__ a, int lda, const TI* __restrict__ w,
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
-            if (n < N) out[(size_t)m * ldo + n] = from_f32<TO>(acc[i][j]);
+            if (n < N) out[(size_t)m * ldo + n] = from_f32<TO>(total[i][j]);
         }
     }
 }
@@ -85,6 +94,10 @@ static int gemm_generic_launch(const void* a, int lda, long long a_batch, const 
     CIB_REQUIRE(M >= 0 && N > 0 && K > 0 && batch > 0, "gemm: bad sizes M=%d N=%d K=%d batch=%d", M, N, K, batch);
     CIB_REQUIRE(lda >= K && ldw >= K && ldo >= N, "gemm: leading dimensions too small (lda=%d ldw=%d ldo=%d)", lda, ldw, ldo);
     if (M == 0) return 0;
+    if (in_dtype == kF32 && out_dtype == kF32) {
+        const GemmF32 p{(const float*)a, (const float*)w, (float*)out, lda, ldw, ldo, M, N, K, a_batch, w_batch, o_batch};
+        if (gemm_f32_takes(p, batch)) return gemm_f32_launch(p, batch, stream);
+    }
     dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, batch);
     CIB_REQUIRE(grid.y <= 65535 && batch <= 65535, "gemm: M=%d or batch=%d too large for this kernel", M, batch);
     if (in_dtype == kF32 && out_dtype == kF32)

@@ -4,7 +4,7 @@ gate/up the same way and has no bias).
 
 Which kernel multiplies is decided here, per call, from the engine dtype and the shape:
 
-* float32: the FMA kernel (``gemm_generic``), true 32-bit, any shape;
+* float32: the FMA kernels behind ``gemm_generic``, true 32-bit, any shape (few rows, tiles, or rows off 16-byte boundaries);
 * bfloat16: the tensor-core kernels of this package where they take the shape; otherwise the library
   product (cuBLAS through ``torch.mm``), which is what the reference uses for every projection
   (csrc/ops/projection.cu:32-44); shapes that are not a multiple of 8 go to ``gemm_generic``.

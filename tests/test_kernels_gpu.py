@@ -140,6 +140,33 @@ def test_gemm_generic(M, N, K, dtypes):
     assert torch.equal(one[0].cpu(), out[M // 2].cpu())
 
 
+@pytest.mark.parametrize("N, K", [(8, 16), (1001, 132), (520, 1028), (4096, 1024), (1024, 3072), (72, 5000), (40, 16384)])
+def test_gemm_32bit_paths(N, K):
+    """Few rows, tiles with and without K split over a cluster, and rows off 16-byte boundaries: one order of additions, so
+    the same bits; sums of 16-long chains of K products are within (16 + 8 + 12 + 8) roundings of the exact one, each at
+    most 2^-24 of the sum of magnitudes."""
+    k = _k()
+    M = 700
+    a, w = rand(M, K, seed=91).to(DEV), rand(N, K, seed=92).to(DEV)
+    full = torch.empty(M, N, device=DEV)
+    k.gemm_generic(a, w, full)
+    bound = (a.double().abs() @ w.double().abs().T) * 44 * 2.0 ** -24
+    assert bool(((full.double() - a.double() @ w.double().T).abs() <= bound).all())
+    for rows in (1, 3, 8, 9, 31, 33, 64, 257):
+        wide = torch.full((rows, N + 3), 7.0, device=DEV)                # output rows off 16-byte boundaries
+        k.gemm_generic(a[:rows], w, wide[:, :N])
+        assert torch.equal(wide[:, :N], full[:rows]) and bool((wide[:, N:] == 7.0).all()), rows
+    shifted = torch.zeros(5, K + 1, device=DEV)
+    shifted[:, 1:] = a[:5]
+    out = torch.empty(5, N, device=DEV)
+    k.gemm_generic(shifted[:, 1:], w, out)
+    assert torch.equal(out, full[:5])
+    # several products at once
+    batch = torch.empty(3, 40, N, device=DEV)
+    k.gemm_generic_batched(a[:120].view(3, 40, K), w.expand(3, N, K).contiguous(), batch)
+    assert torch.equal(batch.view(120, N), full[:120])
+
+
 @pytest.mark.parametrize("M, N, K", [(128, 128, 64), (128, 256, 128), (17, 1000, 96), (300, 517 + 3, 72),
                                      (2048, 4096, 1024), (640, 1024, 3072), (129, 6144, 1024), (200, 136, 2048)])
 @pytest.mark.parametrize("f32_out", [False, True])
@@ -436,6 +463,37 @@ def test_paged_attention_generic(dtype, nq, nkv, d, ps, window):
     k.paged_attention_generic(case["wide"].to(DEV), out, case["cache"].to(DEV), case["bt"].to(DEV), i32(case["qsl"]),
                               i32(lens), i32(case["treq"]), nq, nkv, d, scale, window or 0)
     close(out, attention_reference(case, lens, new, scale, window), 2e-5 if dtype == torch.float32 else 1.5e-2)
+
+
+@pytest.mark.parametrize("nq, nkv, d, ps", [(16, 8, 128, 16), (8, 1, 64, 32), (6, 3, 128, 5), (3, 3, 64, 1), (32, 2, 128, 128)])
+@pytest.mark.parametrize("window", [None, 50])
+@pytest.mark.parametrize("decode", [False, True])
+def test_paged_attention_32bit(nq, nkv, d, ps, window, decode):
+    """Both 32-bit kernels: tiles that end inside a request and hold several, contexts of more than one round of the warps,
+    empty slots that are NaN, later tokens whose values are infinite, and pages a window has given back."""
+    k = _k()
+    lens = [1, 37, 64, 130, 5, 600, 31, 32, 33]
+    new = [1] * len(lens) if decode else [1, 37, 1, 17, 2, 300, 31, 9, 1]
+    case = attention_case(torch.float32, nq, nkv, d, lens, new, ps, seed=21, sharp=True, poison=True)
+    scale = 0.7 / math.sqrt(d)
+    want = attention_reference(case, lens, new, scale, window)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    bt = case["bt"].clone()
+    if window and decode:                                    # request 5 sees keys 550 .. 599 only
+        bt[5, :(600 - window) // ps] = -1
+    qsl, lens_, treq = case["qsl"], list(lens), case["treq"]
+    out = torch.full((sum(new), nq * d), 5.0, device=DEV)
+    k.paged_attention_generic(case["wide"].to(DEV), out, case["cache"].to(DEV), bt.to(DEV), i32(qsl), i32(lens_), i32(treq), nq,
+                              nkv, d, scale, window or 0)
+    close(out, want, 2e-5)
+    # the last token of request 5 becomes infinite: only its own row may notice
+    cache, last = case["cache"].clone(), lens[5] - 1
+    cache[int(case["bt"][5, last // ps]), :, :, last % ps] = math.inf
+    out2 = torch.full_like(out, 5.0)
+    k.paged_attention_generic(case["wide"].to(DEV), out2, cache.to(DEV), bt.to(DEV), i32(qsl), i32(lens_), i32(treq), nq, nkv, d,
+                              scale, window or 0)
+    others = torch.arange(sum(new), device=DEV) != qsl[6] - 1
+    assert torch.equal(out2[others], out[others])
 
 
 @pytest.mark.parametrize("nq, nkv, d, ps", [(16, 8, 128, 16), (8, 1, 64, 32), (12, 3, 128, 5), (32, 2, 256, 16),
