@@ -8,10 +8,12 @@
 // (rows of one m16 tile) with them on the tensor cores, and keeps a running softmax in base 2.  Warps are
 // merged in shared memory, CTAs through a scratch buffer: every CTA writes its partial (max, sum, weighted
 // values) and bumps a counter; the last CTA of a (request, kv head) combines all partials and writes the
-// output, then resets the counter so that the kernel can be replayed from a CUDA graph.  Where the splits are few and
-// their partials small (`cluster_combine_fits`), the CTAs of a (request, kv head) are one thread-block cluster instead
+// output, then resets the counter so that the kernel can be replayed from a CUDA graph.  Where the launch allows it
+// (`cluster_combines`), the CTAs of a (request, kv head) are one thread-block cluster instead
 // and meet in the shared memory of its first CTA: the others write their partials there (distributed shared memory),
 // signal with a release on the cluster's barrier and leave; no scratch, fence, counter or second trip to the L2.
+// A launch is made for the longest context its graph may meet: a CTA that this request leaves without keys goes at once,
+// and a request whose keys fit one CTA is not merged at all.
 //
 // Scratch layout (float32): part_o[(request * nkv + kvh) * splits + split][g][D], part_ml[...][g][2].
 // Cache layout of one layer: [page][0 = keys, 1 = values][kv head][slot in page][D].
@@ -101,10 +103,17 @@ __device__ __forceinline__ void load_block(__nv_bfloat16* sK, __nv_bfloat16* sV,
 // Shared memory the first CTA of a cluster keeps for the partials of all its CTAs: [splits][g][D + 2] floats, in a
 // region of its own behind everything else (the other CTAs may write while the first still streams keys).
 __host__ __device__ inline size_t cluster_inbox_bytes(int splits, int g, int d) { return (size_t)splits * g * (d + 2) * sizeof(float); }
-// The cluster path is taken for up to 4 CTAs per (request, kv head) whose partials fit 9 KB: two CTAs of head size 128
-// then still share an SM.  (Clusters of 8 measured slower than the combine through memory once they fill the GPU: 4
-// requests x 8 heads x 8 splits ran a decode step in 1.42 ms against 1.17.)
-inline bool cluster_combine_fits(int splits, int g, int d) { return splits > 1 && splits <= 4 && cluster_inbox_bytes(splits, g, d) <= 9 * 1024; }
+// Whether a launch may merge in clusters: up to 8 CTAs per (request, kv head) where the whole launch has at most a CTA for
+// each of the 148 SMs, and up to 4 on the TMA path; partials of 9 KB at most, so that two CTAs of head size 128 still share
+// an SM.  The merge through memory costs 3.6 us more than none, a cluster 1.2 (one request with 256 keys: 8.4 us against
+// 6.1, with the kernel before it).  But a cluster's CTAs start together, and where they do not all find a free SM that costs
+// more: on the cp.async path, whose launches begin under the tail of the kernel before them, a step of 8 requests x 8 heads x
+// 4 splits with 1 050 keys took 3 % longer in clusters; 4 requests x 8 x 8 with 2 040 keys 18.1 us a layer against 13.6.
+// The host's choice of splits knows this rule (decode_merges_in_cluster in kernels.py).
+inline bool cluster_combines(long long pairs, int splits, int g, int d, bool tma) {
+    const bool one_round = splits <= 8 && pairs * splits <= 148;
+    return splits > 1 && (one_round || (tma && splits <= 4)) && cluster_inbox_bytes(splits, g, d) <= 9 * 1024;
+}
 
 template <int D, bool TMA, bool CL>
 __global__ void __launch_bounds__(kDecWarps * 32)
@@ -133,7 +142,9 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
     const int span = max(0, seq_len - lo);
     int chunk = (span + splits - 1) / splits;
-    chunk = (chunk + kDecKeys - 1) / kDecKeys * kDecKeys;
+    chunk = max(kDecWarps * kDecKeys, (chunk + kDecKeys - 1) / kDecKeys * kDecKeys);       // a block for every warp at least
+    const int active = max(1, (span + chunk - 1) / chunk);        // CTAs with keys
+    if (split >= active) return;
     const int k_begin = lo + split * chunk;
     const int k_end = min(seq_len, k_begin + chunk);
     const int* table = block_table + (size_t)r * table_stride;
@@ -359,7 +370,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     // cluster path: the partials go to the first CTA's shared memory, [split][g][D] values then [split][g][2] maxima and sums
     float* inbox_o = nullptr;
     float* inbox_ml = nullptr;
-    if (CL) {
+    if (CL && active > 1) {
         namespace cg = cooperative_groups;
         float* inbox = reinterpret_cast<float*>(smem_raw + inbox_offset);
         if (split != 0) inbox = cg::this_cluster().map_shared_rank(inbox, 0);
@@ -382,7 +393,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
                 O += sm_o[((size_t)(w * g + row)) * D + dim] * f;
             }
         }
-        if (splits == 1) {
+        if (active == 1) {
             out[(size_t)r * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
         } else if (CL) {
             inbox_o[row * D + dim] = O;
@@ -398,7 +409,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
             }
         }
     }
-    if (splits == 1) return;
+    if (active == 1) return;
     if (CL) {
         // ---- the first CTA of the cluster combines what the others have written into its shared memory ----
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -410,9 +421,9 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         for (int idx = threadIdx.x; idx < g * D; idx += blockDim.x) {
             const int row = idx / D, dim = idx - row * D;
             float M = -INFINITY;
-            for (int sp = 0; sp < splits; ++sp) M = fmaxf(M, all_ml[(sp * g + row) * 2]);
+            for (int sp = 0; sp < active; ++sp) M = fmaxf(M, all_ml[(sp * g + row) * 2]);
             float L = 0.f, O = 0.f;
-            for (int sp = 0; sp < splits; ++sp) {
+            for (int sp = 0; sp < active; ++sp) {
                 const float ms = all_ml[(sp * g + row) * 2];
                 const float f = (ms == -INFINITY || M == -INFINITY) ? 0.f : exp2f(ms - M);
                 L = fmaf(all_ml[(sp * g + row) * 2 + 1], f, L);
@@ -429,7 +440,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     __syncthreads();
     if (threadIdx.x == 0) {
         const int done = atomicAdd(&counters[r * nkv + kvh], 1);
-        s_last = done == splits - 1;
+        s_last = done == active - 1;
     }
     __syncthreads();
     if (!s_last) return;
@@ -438,11 +449,11 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     // the splits); then the weighted sums with up to sixteen loads in flight per thread.  (Read one by one in a loop
     // over the splits, the sums cost a round trip to the L2 each: some 5 us with 32 splits.)
     const size_t base = ((size_t)r * nkv + kvh) * splits;
-    float* sm_w = reinterpret_cast<float*>(smem_raw);            // [g][splits] maximum, then weight of each split
-    float* sm_ls = sm_w + (size_t)g * splits;                     // [g][splits] sum of each split
-    float* sm_inv = sm_ls + (size_t)g * splits;                   // [g] 1 / total
-    for (int idx = threadIdx.x; idx < g * splits; idx += blockDim.x) {
-        const int row = idx / splits, sp = idx - row * splits;
+    float* sm_w = reinterpret_cast<float*>(smem_raw);            // [g][active] maximum, then weight of each split
+    float* sm_ls = sm_w + (size_t)g * active;                     // [g][active] sum of each split
+    float* sm_inv = sm_ls + (size_t)g * active;                   // [g] 1 / total
+    for (int idx = threadIdx.x; idx < g * active; idx += blockDim.x) {
+        const int row = idx / active, sp = idx - row * active;
         const float2 ml = __ldcg(reinterpret_cast<const float2*>(&part_ml[((base + sp) * g + row) * 2]));
         sm_w[idx] = ml.x;
         sm_ls[idx] = ml.y;
@@ -450,15 +461,15 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     __syncthreads();
     for (int row = warp; row < g; row += kDecWarps) {
         float M = -INFINITY;
-        for (int sp = lane; sp < splits; sp += 32) M = fmaxf(M, sm_w[row * splits + sp]);
+        for (int sp = lane; sp < active; sp += 32) M = fmaxf(M, sm_w[row * active + sp]);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
         float L = 0.f;
-        for (int sp = lane; sp < splits; sp += 32) {
-            const float ms = sm_w[row * splits + sp];
+        for (int sp = lane; sp < active; sp += 32) {
+            const float ms = sm_w[row * active + sp];
             const float f = (ms == -INFINITY || M == -INFINITY) ? 0.f : exp2f(ms - M);
-            sm_w[row * splits + sp] = f;
-            L += sm_ls[row * splits + sp] * f;
+            sm_w[row * active + sp] = f;
+            L += sm_ls[row * active + sp] * f;
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
@@ -469,21 +480,21 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         const int row = idx / D, dim = idx - row * D;
         float O = 0.f;
         int sp = 0;
-        for (; sp + 16 <= splits; sp += 16) {
+        for (; sp + 16 <= active; sp += 16) {
             float v[16];
 #pragma unroll
             for (int u = 0; u < 16; ++u) v[u] = __ldcg(&part_o[((base + sp + u) * g + row) * D + dim]);
 #pragma unroll
-            for (int u = 0; u < 16; ++u) O = fmaf(v[u], sm_w[row * splits + sp + u], O);
+            for (int u = 0; u < 16; ++u) O = fmaf(v[u], sm_w[row * active + sp + u], O);
         }
-        for (; sp + 4 <= splits; sp += 4) {
+        for (; sp + 4 <= active; sp += 4) {
             float v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) v[u] = __ldcg(&part_o[((base + sp + u) * g + row) * D + dim]);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) O = fmaf(v[u], sm_w[row * splits + sp + u], O);
+            for (int u = 0; u < 4; ++u) O = fmaf(v[u], sm_w[row * active + sp + u], O);
         }
-        for (; sp < splits; ++sp) O = fmaf(__ldcg(&part_o[((base + sp) * g + row) * D + dim]), sm_w[row * splits + sp], O);
+        for (; sp < active; ++sp) O = fmaf(__ldcg(&part_o[((base + sp) * g + row) * D + dim]), sm_w[row * active + sp], O);
         out[(size_t)r * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(O * sm_inv[row]);
     }
     if (threadIdx.x == 0) counters[r * nkv + kvh] = 0;
@@ -491,8 +502,8 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
 
 // How many clusters of `cluster_x` CTAs of this kernel the device runs at one time (0 if that cannot be told); asked
 // once per cluster size and kernel, then remembered.
-template <typename Kernel>
-static int max_resident_clusters(Kernel kernel, int cluster_x, size_t smem) {
+template <auto kernel>
+static int max_resident_clusters(int cluster_x, size_t smem) {
     static std::mutex mutex;
     static int known[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};     // by cluster size; 0: not asked yet, -1: the query failed
     if (cluster_x < 2 || cluster_x > 8) return 0;
@@ -547,10 +558,11 @@ static int launch_decode(const void* q, int q_stride, void* out, int out_stride,
     // The cluster path only where all clusters of the launch run at once: a cluster needs its CTAs on SMs of one GPC, so
     // fewer fit than single CTAs would, and a second round of clusters costs far more than the combine through memory
     // (12 requests x 8 heads x 3 splits: 51 us against 37).
-    bool cluster = tma && cluster_combine_fits(splits, g, D);
+    bool cluster = cluster_combines((long long)num_requests * nkv, splits, g, D, tma) && smem + cluster_inbox_bytes(splits, g, D) <= 225 * 1024;
     if (cluster) {
         const size_t with_inbox = smem + cluster_inbox_bytes(splits, g, D);
-        const int resident = max_resident_clusters(paged_attention_decode_kernel<D, true, true>, splits, with_inbox);
+        const int resident = tma ? max_resident_clusters<paged_attention_decode_kernel<D, true, true>>(splits, with_inbox)
+                                 : max_resident_clusters<paged_attention_decode_kernel<D, false, true>>(splits, with_inbox);
         cluster = resident >= nkv * num_requests;
         if (cluster) smem = with_inbox;
     }
@@ -565,12 +577,12 @@ static int launch_decode(const void* q, int q_stride, void* out, int out_stride,
                                   nkv, scale_log2, window, splits, part_o, part_ml, counters, kv_map, error_flag, warm,
                                   warm_bytes, inbox_offset);
     };
-    static SmemLimit limits[3];          // one per instantiation of this head size
+    static SmemLimit limits[4];          // one per instantiation of this head size
     cudaError_t e = cudaSuccess;
     if (cluster) {
         // should the cluster launch be refused after all (the occupancy query is a forecast), the step is not lost:
         // the same work runs without clusters, combined through the scratch
-        e = launch(paged_attention_decode_kernel<D, true, true>, limits[0]);
+        e = tma ? launch(paged_attention_decode_kernel<D, true, true>, limits[0]) : launch(paged_attention_decode_kernel<D, false, true>, limits[3]);
         if (e != cudaSuccess && e != cudaErrorUnknown) {
             (void)cudaGetLastError();
             cluster = false;

@@ -605,6 +605,13 @@ def decode_slots(head_dim: int) -> int:
     return 148 * (1 if head_dim > 128 else 2 if head_dim > 64 else 3)
 
 
+def decode_merges_in_cluster(pairs: int, splits: int) -> bool:
+    """Whether the CTAs that share the keys of a (request, kv head) merge in a cluster, which costs little, on either path
+    of the kernel (``cluster_combines`` in attention_decode.cu; larger launches merge so on the TMA path only, which
+    the estimates below do not count on)."""
+    return splits <= 8 and pairs * splits <= 148
+
+
 def decode_splits(num_requests: int, num_kv_heads: int, max_seq_len: int, slots: int = 296, tma: bool = False,
                   head_dim: int = 128) -> int:
     """How many CTAs share the keys of one (request, kv head).  ``tma``: the cache layout allows the TMA path, which
@@ -614,7 +621,7 @@ def decode_splits(num_requests: int, num_kv_heads: int, max_seq_len: int, slots:
     16-key blocks in turn, so a CTA's share counts in steps of 64 keys.  A launch is estimated, in nanoseconds, round
     of CTAs by round: a round of n CTAs takes keys per CTA x (the larger of a CTA's own pace per key and n x 0.072, the
     memory's pace when n CTAs stream at once) plus a fixed cost for a CTA's start and its partial results; splitting
-    adds 3000 for the combine and 40 per split.  A CTA's own pace is 16 per key and 3000 fixed on the TMA path, 18 and
+    adds 3000 for the combine and 40 per split, or 1200 where the combine is a cluster's.  A CTA's own pace is 16 per key and 3000 fixed on the TMA path, 18 and
     4000 on the cp.async path.  The constants were fitted to timings at batch 1 to 128 with 300 to 9000 keys of head
     size 128 (largest miss 1.7 us, 9 % r.m.s. error of the estimate); for another head size the costs per key scale
     with the bytes of a key.  The smallest estimate wins.
@@ -632,7 +639,7 @@ def decode_splits(num_requests: int, num_kv_heads: int, max_seq_len: int, slots:
         if rest:
             cost += keys * max(per_key, 0.072 * width * rest) + fixed
         if s > 1:
-            cost += 3000.0 + 40.0 * s
+            cost += 1200.0 if decode_merges_in_cluster(pairs, s) else 3000.0 + 40.0 * s
         if best_cost is None or cost < best_cost:
             best, best_cost = s, cost
     return best
