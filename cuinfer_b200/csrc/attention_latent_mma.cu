@@ -300,30 +300,61 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q_abs, int qa_stri
 
 // Merge the splits of a (token, head): M = max(sink, m_s), L = 2^(sink - M) + sum l_s 2^(m_s - M),
 // out = sum acc_s 2^(m_s - M) / L.  A block per (token, head), a thread per column.
-__global__ void latent_attention_merge_kernel(const float* __restrict__ part, const float* __restrict__ sinks,
-                                              __nv_bfloat16* __restrict__ out, int out_stride, int H, int rk, int splits,
-                                              int rows) {
-    const int w = blockIdx.x, lane = threadIdx.x;
+// The splits' maxima and sums are read by as many threads at once and turned into weights in shared memory; the rows are then
+// a stream of independent 8-byte loads, eight in flight a thread.  (Every thread used to read the maxima one by one, twice:
+// 32 splits of 8 rows x 32 heads x 512 took 18 us.)
+constexpr int kMergeChunk = 512;
+__global__ void __launch_bounds__(256)
+latent_attention_merge_kernel(const float* __restrict__ part, const float* __restrict__ sinks,
+                              __nv_bfloat16* __restrict__ out, int out_stride, int H, int rk, int splits, int rows) {
+    __shared__ float s_w[kMergeChunk];
+    __shared__ float s_red[33];
+    const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
     if (w >= rows) return;
     const int token = w / H, head = w % H;
-    const float* p = part + (size_t)w * splits * (rk + 2);
+    const size_t stride = rk + 2;
+    const float* p = part + (size_t)w * splits * stride;
     const float sink = sinks ? sinks[head] * kLog2e : -INFINITY;
-    float M = sink;
-    for (int s = 0; s < splits; ++s) M = fmaxf(M, p[(size_t)s * (rk + 2)]);
-    float L = sink == -INFINITY ? 0.f : exp2f(sink - M);
-    for (int s = 0; s < splits; ++s) {
-        const float m = p[(size_t)s * (rk + 2)];
-        if (m != -INFINITY) L += p[(size_t)s * (rk + 2) + 1] * exp2f(m - M);
+    float M = sink, used = 0.f;                                  // used: the splits up to the last one with keys
+    for (int s = tid; s < splits; s += blockDim.x) {
+        const float m = p[s * stride];
+        M = fmaxf(M, m);
+        if (m != -INFINITY) used = (float)(s + 1);
     }
-    const float inv = L > 0.f ? 1.f / L : 0.f;
-    for (int c = lane; c < rk; c += blockDim.x) {
-        float acc = 0.f;
-#pragma unroll 4
-        for (int s = 0; s < splits; ++s) {
-            const float m = p[(size_t)s * (rk + 2)];
-            if (m != -INFINITY) acc += p[(size_t)s * (rk + 2) + 2 + c] * exp2f(m - M);
+    M = warp_max(M);
+    used = warp_max(used);
+    if (lane == 0) { s_red[warp] = M; s_w[warp] = used; }
+    __syncthreads();
+    M = warp_max(lane < warps ? s_red[lane] : -INFINITY);
+    const int end = (int)warp_max(lane < warps ? s_w[lane] : 0.f);
+    float L = 0.f;
+    float2 acc = make_float2(0.f, 0.f);
+    const int c = 2 * tid;                                      // rk is at most twice the threads
+    for (int first = 0; first < end; first += kMergeChunk) {
+        const int count = min(kMergeChunk, end - first);
+        __syncthreads();
+        for (int s = tid; s < count; s += blockDim.x) {
+            const float2 ml = *reinterpret_cast<const float2*>(p + (first + s) * stride);
+            const float f = ml.x == -INFINITY ? 0.f : exp2f(ml.x - M);
+            s_w[s] = f;
+            if (f != 0.f) L += ml.y * f;
         }
-        out[(size_t)token * out_stride + (size_t)head * rk + c] = __float2bfloat16_rn(acc * inv);
+        __syncthreads();
+        if (c < rk) {
+            const float* src = p + first * stride + 2 + c;
+#pragma unroll 8
+            for (int s = 0; s < count; ++s) {
+                const float f = s_w[s];
+                const float2 v = *reinterpret_cast<const float2*>(src + s * stride);
+                acc.x = fmaf(f != 0.f ? v.x : 0.f, f, acc.x);   // a split without keys may not have written its row
+                acc.y = fmaf(f != 0.f ? v.y : 0.f, f, acc.y);
+            }
+        }
+    }
+    L = block_sum(L, s_red) + (sink == -INFINITY ? 0.f : exp2f(sink - M));
+    if (c < rk) {
+        const float inv = L > 0.f ? 1.f / L : 0.f;
+        *reinterpret_cast<__nv_bfloat162*>(out + (size_t)token * out_stride + (size_t)head * rk + c) = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
     }
 }
 
@@ -405,7 +436,7 @@ extern "C" int cib_latent_attention_mma(const void* q_abs, int qa_stride, const 
     CIB_LAUNCH_CHECK("latent_attention_mma");
     if (splits > 1) {
         const int rows = num_tokens * H;
-        latent_attention_merge_kernel<<<rows, rk >= 256 ? 256 : 128, 0, stream>>>(scratch, sinks, (__nv_bfloat16*)out, out_stride, H, rk,
+        latent_attention_merge_kernel<<<rows, rk > 256 ? 256 : 128, 0, stream>>>(scratch, sinks, (__nv_bfloat16*)out, out_stride, H, rk,
                                                                            splits, rows);
         CIB_LAUNCH_CHECK("latent_attention_merge");
     }

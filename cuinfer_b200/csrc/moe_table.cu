@@ -50,104 +50,93 @@ struct ExpertAct {
 
 __device__ __forceinline__ float base_factor(float g) { return 1.f / (1.f + expf(-g)); }
 
+// Where value i of a 32-bit vector of n lies in shared memory.  bfloat16 weights are read eight to a lane, so the vector's
+// eights are split into two planes of fours: a warp's two 16-byte reads then hit every bank once.  (In natural order the
+// lanes' eights lay 32 bytes apart and each of their eight 4-byte reads took eight turns at the banks: with 8 tokens of two
+// experts 12.6 MB each, the down projection of a decode step ran at 2.9 TB/s whatever the memory could deliver.)
 template <typename T>
-__device__ __forceinline__ float dot_row(const T* __restrict__ w, const float* __restrict__ x, int n, int lane) {
-    float s = 0.f;
-    for (int i = lane; i < n; i += 32) s = fmaf(to_f32(w[i]), x[i], s);
-    return warp_sum(s);
-}
-// bfloat16 rows of a multiple of 8 values that start on a 16-byte boundary: a lane reads 16 bytes at a time (a warp
-// 512 bytes per load instead of 64), four loads issued before the first is used.
-template <>
-__device__ __forceinline__ float dot_row<__nv_bfloat16>(const __nv_bfloat16* __restrict__ w, const float* __restrict__ x, int n,
-                                                        int lane) {
-    float s = 0.f;
-    if ((n & 7) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
-        const uint4* w8 = reinterpret_cast<const uint4*>(w);
-        const int chunks = n >> 3;
-        int c = lane;
-        for (; c + 96 < chunks; c += 128) {
-            uint4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = __ldg(w8 + c + 32 * u);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[u]);
-                const float* xs = x + (c + 32 * u) * 8;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    s = fmaf(__low2float(h[k]), xs[2 * k], s);
-                    s = fmaf(__high2float(h[k]), xs[2 * k + 1], s);
-                }
-            }
-        }
-        for (; c < chunks; c += 32) {
-            const uint4 v = __ldg(w8 + c);
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-            const float* xs = x + c * 8;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                s = fmaf(__low2float(h[k]), xs[2 * k], s);
-                s = fmaf(__high2float(h[k]), xs[2 * k + 1], s);
-            }
-        }
-    } else {
-        for (int i = lane; i < n; i += 32) s = fmaf(__bfloat162float(w[i]), x[i], s);
-    }
-    return warp_sum(s);
+__device__ __forceinline__ bool in_planes(int n) { return sizeof(T) == 2 && (n & 7) == 0; }
+template <typename T>
+__device__ __forceinline__ int vec_at(int i, int n) {
+    return in_planes<T>(n) ? ((i >> 3) << 2 | (i & 3)) + (i >> 2 & 1) * (n >> 1) : i;
 }
 
-// Two rows at once, each against its own vector: the loads of both rows are issued before either is used, so a lane
-// keeps eight 16-byte loads in flight instead of four (a decode step has too few warps an SM for four to fill the
-// memory pipe: two rows at a time took a call of the large experts from 180 to 107 us).  Every row is summed in the
-// order `dot_row` sums it, so the results are the same to the last bit.
 template <typename T>
-__device__ __forceinline__ void dot_rows2(const T* __restrict__ w0, const float* __restrict__ x0, const T* __restrict__ w1,
-                                          const float* __restrict__ x1, int n, int lane, float& r0, float& r1) {
-    r0 = dot_row(w0, x0, n, lane);
-    r1 = dot_row(w1, x1, n, lane);
+__device__ __forceinline__ float dot_row_plain(const T* __restrict__ w, const float* __restrict__ x, int n, int lane) {
+    float s = 0.f;
+    for (int i = lane; i < n; i += 32) s = fmaf(to_f32(w[i]), x[vec_at<T>(i, n)], s);
+    return warp_sum(s);
 }
-__device__ __forceinline__ float dot_chunk(const uint4& v, const float* __restrict__ xs, float s) {
+__device__ __forceinline__ float dot_chunk(const uint4& v, const float4& lo, const float4& hi, float s) {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        s = fmaf(__low2float(h[k]), xs[2 * k], s);
-        s = fmaf(__high2float(h[k]), xs[2 * k + 1], s);
-    }
-    return s;
+    s = fmaf(__low2float(h[0]), lo.x, s);
+    s = fmaf(__high2float(h[0]), lo.y, s);
+    s = fmaf(__low2float(h[1]), lo.z, s);
+    s = fmaf(__high2float(h[1]), lo.w, s);
+    s = fmaf(__low2float(h[2]), hi.x, s);
+    s = fmaf(__high2float(h[2]), hi.y, s);
+    s = fmaf(__low2float(h[3]), hi.z, s);
+    return fmaf(__high2float(h[3]), hi.w, s);
 }
-template <>
-__device__ __forceinline__ void dot_rows2<__nv_bfloat16>(const __nv_bfloat16* __restrict__ w0, const float* __restrict__ x0,
-                                                         const __nv_bfloat16* __restrict__ w1, const float* __restrict__ x1, int n,
-                                                         int lane, float& r0, float& r1) {
-    if ((n & 7) != 0 || ((reinterpret_cast<uintptr_t>(w0) | reinterpret_cast<uintptr_t>(w1)) & 15) != 0) {
-        r0 = dot_row(w0, x0, n, lane);
-        r1 = dot_row(w1, x1, n, lane);
+
+// ROWS rows (one or two) times the same vector.  bfloat16 rows of a multiple of 8 values that start on a 16-byte boundary: a
+// lane reads 16 bytes at a time, four loads of every row issued before the first is used (a decode step has too few warps
+// an SM for fewer to fill the memory pipe: two rows at a time took a call of the large experts from 180 to 107 us), and the
+// vector is read once for both rows.  Every row is summed in the same order whether it comes alone or not.
+template <int ROWS, typename T>
+__device__ __forceinline__ void dot_rows(const T* const (&w)[ROWS], const float* __restrict__ x, int n, int lane, float (&r)[ROWS]) {
+    bool wide = in_planes<T>(n);
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) wide = wide && (reinterpret_cast<uintptr_t>(w[k]) & 15) == 0;
+    if (!wide) {
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k) r[k] = dot_row_plain(w[k], x, n, lane);
         return;
     }
-    const uint4* a8 = reinterpret_cast<const uint4*>(w0);
-    const uint4* b8 = reinterpret_cast<const uint4*>(w1);
     const int chunks = n >> 3;
-    float s0 = 0.f, s1 = 0.f;
+    const float4* lo = reinterpret_cast<const float4*>(x);
+    const float4* hi = reinterpret_cast<const float4*>(x + (n >> 1));
+    float s[ROWS] = {};
     int c = lane;
     for (; c + 96 < chunks; c += 128) {
-        uint4 a[4], b[4];
+        uint4 v[ROWS][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) a[u] = __ldg(a8 + c + 32 * u);
+        for (int k = 0; k < ROWS; ++k)
 #pragma unroll
-        for (int u = 0; u < 4; ++u) b[u] = __ldg(b8 + c + 32 * u);
+            for (int u = 0; u < 4; ++u) v[k][u] = __ldg(reinterpret_cast<const uint4*>(w[k]) + c + 32 * u);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) s0 = dot_chunk(a[u], x0 + (c + 32 * u) * 8, s0);
+        for (int u = 0; u < 4; ++u) {
+            const float4 a = lo[c + 32 * u], b = hi[c + 32 * u];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) s1 = dot_chunk(b[u], x1 + (c + 32 * u) * 8, s1);
+            for (int k = 0; k < ROWS; ++k) s[k] = dot_chunk(v[k][u], a, b, s[k]);
+        }
     }
     for (; c < chunks; c += 32) {
-        const uint4 a = __ldg(a8 + c), b = __ldg(b8 + c);
-        s0 = dot_chunk(a, x0 + c * 8, s0);
-        s1 = dot_chunk(b, x1 + c * 8, s1);
+        uint4 v[ROWS];
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k) v[k] = __ldg(reinterpret_cast<const uint4*>(w[k]) + c);
+        const float4 a = lo[c], b = hi[c];
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k) s[k] = dot_chunk(v[k], a, b, s[k]);
     }
-    r0 = warp_sum(s0);
-    r1 = warp_sum(s1);
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) r[k] = warp_sum(s[k]);
+}
+
+template <typename T>
+__device__ __forceinline__ float dot_row(const T* w, const float* __restrict__ x, int n, int lane) {
+    const T* const rows[1] = {w};
+    float r[1];
+    dot_rows<1, T>(rows, x, n, lane, r);
+    return r[0];
+}
+template <typename T>
+__device__ __forceinline__ void dot_rows2(const T* w0, const T* w1, const float* __restrict__ x, int n, int lane, float& r0, float& r1) {
+    const T* const rows[2] = {w0, w1};
+    float r[2];
+    dot_rows<2, T>(rows, x, n, lane, r);
+    r0 = r[0];
+    r1 = r[1];
 }
 
 template <typename T>
@@ -155,10 +144,10 @@ __global__ void __launch_bounds__(kMoeWarps * 32)
 moe_table_gate_up_kernel(const T* __restrict__ h, int h_stride, const int* __restrict__ ids,
                          const int* __restrict__ table, int vocab, int top, int experts,
                          const T* __restrict__ gate_up, T* __restrict__ act, int width, int ff, ExpertAct fn, int outs) {
-    extern __shared__ float hs[];
+    extern __shared__ __align__(16) float hs[];
     const int t = blockIdx.x / top, k = blockIdx.x % top;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < width; i += blockDim.x) hs[i] = to_f32(h[(size_t)t * h_stride + i]);
+    for (int i = threadIdx.x; i < width; i += blockDim.x) hs[vec_at<T>(i, width)] = to_f32(h[(size_t)t * h_stride + i]);
     __syncthreads();
     const int id = ids ? ids[t] : t;
     const int e = (id >= 0 && id < vocab) ? table[(size_t)id * top + k] : -1;
@@ -171,7 +160,7 @@ moe_table_gate_up_kernel(const T* __restrict__ h, int h_stride, const int* __res
     if (gated) {                                      // a gate row and its up row together
         for (int j = j0 + warp; j < j_end; j += kMoeWarps) {
             float g = 0.f, u = 0.f;
-            if (ok) dot_rows2(wg + (size_t)j * width, hs, wu + (size_t)j * width, hs, width, lane, g, u);
+            if (ok) dot_rows2(wg + (size_t)j * width, wu + (size_t)j * width, hs, width, lane, g, u);
             if (lane == 0) dst[j] = from_f32<T>(ok ? fn(g, u) : 0.f);
         }
         return;
@@ -180,7 +169,7 @@ moe_table_gate_up_kernel(const T* __restrict__ h, int h_stride, const int* __res
         const int j2 = j + kMoeWarps;
         float a = 0.f, b = 0.f;
         if (ok) {
-            if (j2 < j_end) dot_rows2(wg + (size_t)j * width, hs, wg + (size_t)j2 * width, hs, width, lane, a, b);
+            if (j2 < j_end) dot_rows2(wg + (size_t)j * width, wg + (size_t)j2 * width, hs, width, lane, a, b);
             else a = dot_row(wg + (size_t)j * width, hs, width, lane);
         }
         if (lane == 0) {
@@ -197,10 +186,11 @@ moe_table_down_kernel(const T* __restrict__ act, const int* __restrict__ ids, co
                       float weight, const float* __restrict__ weights, const float* __restrict__ base_gate, int base_gate_stride,
                       const T* __restrict__ h, int h_stride, const float* __restrict__ self_weight, T* __restrict__ out, int width,
                       int ff, int outs) {
-    extern __shared__ float as[];                       // [top][ff]
+    extern __shared__ __align__(16) float as[];         // [top][ff], each as `vec_at` lays it out
     const int t = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < top * ff; i += blockDim.x) as[i] = to_f32(act[(size_t)t * top * ff + i]);
+    for (int i = threadIdx.x; i < top * ff; i += blockDim.x)
+        as[i / ff * ff + vec_at<T>(i % ff, ff)] = to_f32(act[(size_t)t * top * ff + i]);
     __syncthreads();
     const int id = ids ? ids[t] : t;
     const bool id_ok = id >= 0 && id < vocab;
@@ -213,7 +203,7 @@ moe_table_down_kernel(const T* __restrict__ act, const int* __restrict__ ids, co
             const int e = id_ok ? table[(size_t)id * top + k] : -1;
             if (e < 0 || e >= experts) continue;
             float d0, d1 = 0.f;
-            if (i2 < i_end) dot_rows2(down + ((size_t)e * width + i) * ff, as + k * ff, down + ((size_t)e * width + i2) * ff, as + k * ff, ff, lane, d0, d1);
+            if (i2 < i_end) dot_rows2(down + ((size_t)e * width + i) * ff, down + ((size_t)e * width + i2) * ff, as + k * ff, ff, lane, d0, d1);
             else d0 = dot_row(down + ((size_t)e * width + i) * ff, as + k * ff, ff, lane);
             const float wk = weights ? weights[(size_t)t * top + k] : 1.f;
             sum[0] += wk * d0;
