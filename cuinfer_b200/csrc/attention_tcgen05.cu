@@ -4,32 +4,33 @@
 // request, keys 0..position come from its pages, rows of a tile are query token x query head of one kv head), on
 // Blackwell's own path instead of mma.sync:
 //
-//   * a CTA owns a 128-row query tile (128 / g tokens x g heads of one kv head) and walks over 128-key tiles;
+//   * a CTA owns a 128-row query tile (128 / g tokens x g heads of one kv head) and walks over 64-key tiles; two CTAs share
+//     an SM (256 columns of tensor memory and 97 KB of shared memory each), so that one takes exponentials while the other
+//     starts, waits for its first keys or stores (8 prompts of 1 024 tokens, 16 heads over 8: 67.5 us a layer, 510 TFLOP/s,
+//     where one CTA an SM, 128-key tiles and sixteen softmax warps took 88.7; one of 8 192: 268.6 us, 1 024 TFLOP/s, for 327).
+//     Launches of few CTAs run that other variant (attention_tcgen05_wide.cu);
 //   * keys and values come page by page through TMA (`cp.async.bulk.tensor.2d`, one box of 64 columns x one page per
 //     copy, 128-byte swizzle: the layout the tensor cores read), issued by the lanes of the producer warps,
-//     double-buffered, completion counted in bytes on mbarriers.  (Copies issued by ordinary loads or `cp.async` kept
-//     too few bytes in flight per SM: a tile took longer to arrive than its softmax takes.)  The page size must be a
-//     power of two of at least 8 slots, so that a box starts on a 1024-byte swizzle atom;
+//     double-buffered, completion counted in bytes on mbarriers (four buffers each changed nothing).  (Copies issued by
+//     ordinary loads or `cp.async` kept too few bytes in flight per SM: a tile took longer to arrive than its softmax takes.)
+//     The page size must be a power of two of at least 8 slots, so that a box starts on a 1024-byte swizzle atom;
 //   * S = Q K^T and O += P V are `tcgen05.mma.cta_group::1.kind::f16` with accumulators in tensor memory; K is a
 //     K-major operand, V an MN-major one, straight from the page layout; P is the A operand of P V straight from tensor
 //     memory (bfloat16, written with `tcgen05.st` over the scores it was made from), so it never touches shared memory;
-//   * key tiles alternate between two sets of S, running maximum, running sum and O in tensor memory (4 x 128 columns),
-//     merged at the end like the splits of a split-key kernel: S of tile j+1 is computed and P V of tile j-1 runs while
-//     the sixteen softmax warps take the exponentials of tile j.  Four threads share a row (TMEM lane = row, 32 columns
-//     each): they read S with one `tcgen05.ld`, keep the running maximum in base 2 and raise it only when it grows by
-//     more than 8 (so O is rescaled rarely, with `tcgen05.ld`/`tcgen05.st`);
-//   * a seventeenth warp's first lane issues the MMAs.
+//   * key tiles alternate between two buffers of S: S of tile j+1 is computed while the four softmax warps take the
+//     exponentials of tile j.  A thread owns a row (TMEM lane = row): no exchange with other threads; it keeps the running
+//     maximum in base 2 and raises it only when it grows by more than 8 (so O is rescaled rarely, with
+//     `tcgen05.ld`/`tcgen05.st`);
+//   * a fifth warp's first lane issues the MMAs.
 //
 // Two options serve attention layers that keep a token's key and value side by side in one cache row and put a learned
 // number per head into the softmax's denominator: `joined` (the cache is [pages][kv heads][slots][key 128 | value 128];
-// keys and values are boxes of the same tensor map, 128 columns apart) and `sinks` (32-bit, one per query head: when the
-// two sets are merged, exp(sink) joins the denominator once, with no value).
+// keys and values are boxes of the same tensor map, 128 columns apart) and `sinks` (32-bit, one per query head: at the
+// end exp(sink) joins the denominator once, with no value).
 //
 // Every mbarrier wait is bounded; on a time-out the kernel raises the error flag, stops, frees its tensor memory
 // and returns.
-#include <type_traits>
-
-#include "common.cuh"
+#include "attention_tcgen05_wide.cuh"
 #include "mma_utils.cuh"
 #include "tcgen05_utils.cuh"
 
@@ -38,17 +39,18 @@ namespace fa {
 
 constexpr int kD = 128;          // head size
 constexpr int kM = 128;          // rows per CTA
-constexpr int kN = 128;          // keys per tile
-constexpr int kPanel = kM * 128; // bytes of one 64-column panel of a 128-row tile
+constexpr int kN = 64;           // keys per tile
+constexpr int kPanel = kM * 128; // bytes of one 64-column panel of the 128 query rows
+constexpr int kKvPanel = kN * 128;
 
 // MN-major operand (values: [key][d], d contiguous), 128-byte swizzle: 64-element panels `panel_bytes` apart (leading
 // offset), 8-key groups 1024 bytes apart (stride offset).
 __device__ __forceinline__ uint64_t desc_mnmajor(const void* smem, uint32_t panel_bytes) {
     return (uint64_t)((tc_smem_u32(smem) & 0x3ffff) >> 4) | ((uint64_t)(panel_bytes >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// D = F32, A = B = BF16, M = 128, N = 128; b_mn: B is MN-major.
-__host__ __device__ constexpr uint32_t idesc(bool b_mn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+// D = F32, A = B = BF16, M = 128; b_mn: B is MN-major.
+__host__ __device__ constexpr uint32_t idesc(bool b_mn, int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 __device__ __forceinline__ void tst32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
@@ -61,23 +63,16 @@ __device__ __forceinline__ void tst32(uint32_t taddr, const uint32_t (&r)[32]) {
           "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
-__device__ __forceinline__ void tst16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 __device__ __forceinline__ void tst_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// shared memory: Q | K0 | K1 | V0 | V1, each 128 rows x 128 columns bf16 = 32 KB as two 64-column panels.  (A third key
-// buffer changed nothing: what a tile waits for is the 64 KB of its keys and values crossing from the L2.)
-constexpr int kTileBytes = 2 * kPanel;
+// shared memory: Q | K0 | K1 | V0 | V1; Q has 128 rows x 128 columns bf16 = 32 KB as two 64-column panels, a key or value tile
+// 64 rows = 16 KB
+constexpr int kQBytes = 2 * kPanel, kTileBytes = 2 * kKvPanel;
 constexpr int kKBufs = 2, kVBufs = 2;
-constexpr int kSmemBytes = (1 + kKBufs + kVBufs) * kTileBytes + 1024 + 256;
+constexpr int kSmemBytes = kQBytes + (kKBufs + kVBufs) * kTileBytes + 1024 + 256;
+constexpr int kTmemCols = 256;                     // S of buffer 0 | S of buffer 1 | O
 
-constexpr int kMmaWarp = 16;                       // warps 0-15: the softmax
+constexpr int kMmaWarp = 4;                        // warps 0-3: the softmax, a thread per row
 constexpr int kThreads = (kMmaWarp + 3) * 32;      // + the MMA warp, a producer warp for keys and one for values
 
 // A operand from tensor memory (P, bfloat16, two keys to a column), B from shared memory
@@ -86,7 +81,7 @@ __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a_tmem, uint64_t b, 
                  ::"r"(d), "r"(a_tmem), "l"(b), "r"(id), "r"(acc) : "memory");
 }
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pages, const __nv_bfloat16* __restrict__ q, int q_stride,
                          __nv_bfloat16* __restrict__ out, int out_stride, int page_size,
                          const int* __restrict__ block_table, int table_stride, const int* __restrict__ query_start_loc,
@@ -95,23 +90,21 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* sQ = base;
-    unsigned char* sK = base + kTileBytes;                      // kKBufs buffers: tile j in buffer j % kKBufs
-    unsigned char* sV = base + (1 + kKBufs) * kTileBytes;       // kVBufs buffers
-    uint64_t* bars = reinterpret_cast<uint64_t*>(base + (1 + kKBufs + kVBufs) * kTileBytes);
-    // one barrier per buffer; key tile j uses key and value buffer and tensor-memory set j % 2
+    unsigned char* sK = base + kQBytes;                         // kKBufs buffers: tile j in buffer j % kKBufs
+    unsigned char* sV = sK + kKBufs * kTileBytes;         // kVBufs buffers
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + kVBufs * kTileBytes);
+    // one barrier per buffer; key tile j uses key, value and score buffer j % 2
     uint64_t* k_full = bars;           // [kKBufs <= 3] a key tile has landed (bytes counted)
     uint64_t* v_full = bars + 3;       // [2] a value tile has landed
     uint64_t* s_full = bars + 5;       // [2] S of a tile is in tensor memory
-    uint64_t* p_ready = bars + 7;      // [2] P of a tile is in tensor memory (16 warps arrive)
-    uint64_t* pv_done = bars + 9;      // [2] the set's O includes a tile
+    uint64_t* p_ready = bars + 7;      // [2] P of a tile is in tensor memory (the softmax warps arrive)
+    uint64_t* pv_done = bars + 9;      // [2] O includes a tile
     // With two key and two value buffers, tile j's buffers are free again exactly when s_full[j % 2] (S has read the
     // keys) and pv_done[j % 2] (P V has read the values) complete: the producers wait on those, and the thread that
     // issues the MMAs, which every tile waits for in turn, has two commits fewer per tile to issue.
     static_assert(kKBufs == 2 && kVBufs == 2, "the producers take s_full and pv_done for the buffers' release");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     __shared__ int s_req, s_tile, s_abort, s_q0, s_n, s_seq;
-    __shared__ float s_mx[2][4][128];      // [tile parity][column quarter][row]: the quarters' maxima
-    __shared__ float s_l[2][4][128];       // [tile parity][column quarter][row]: the quarters' sums at the end
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = blockIdx.x;     // heads vary fastest: every head's longest tile starts before any shorter one
@@ -153,17 +146,18 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
             asm volatile("prefetch.tensormap [%0];" ::"l"(&kv_map) : "memory");
         }
     } else if (warp == 1 && lane < 16) {
-        // a thread per barrier: p_ready (at 7 and 8) counts the sixteen softmax warps, all others one arrival
+        // a thread per barrier: p_ready (at 7 and 8) counts the softmax warps, all others one arrival
         mbar_init(&bars[lane], lane == 7 || lane == 8 ? kMmaWarp : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tmem_slot)), "r"((uint32_t)kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // stale shared memory must at least be finite: rows of a tile that no page covers are multiplied by P = 0
-    for (int i = tid; i < (kKBufs + kVBufs) * kTileBytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(sK)[i] = make_uint4(0, 0, 0, 0);
+    // stale values must at least be finite: rows of a tile that no page covers are multiplied by P = 0 (stale keys need not
+    // be: their scores are replaced, not multiplied)
+    for (int i = tid; i < kVBufs * kTileBytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(sV)[i] = make_uint4(0, 0, 0, 0);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // before the bulk copies write the same bytes
     tcgen05_fence_before();
     __syncthreads();
@@ -190,7 +184,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
 
     if (active && warp < kMmaWarp) {
         // ---- the query tile: row = token_local * g + head_in_group, two swizzled 64-column panels ----
-        // (a thread's four loads are all on their way before the first is stored: one round trip, not four)
+        // (a thread's loads are all on their way before the first is stored: one round trip)
         constexpr int kPer = kM * 16 / (kMmaWarp * 32);
         uint4 v[kPer];
 #pragma unroll
@@ -216,8 +210,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
     // way while the queries are still being copied
     if (warp <= kMmaWarp) asm volatile("bar.sync 10, %0;" ::"r"((kMmaWarp + 1) * 32) : "memory");
 
-    // tensor memory: S of set 0 | S of set 1 | O of set 0 | O of set 1, 128 columns each; P of a set (bfloat16,
-    // two keys to a column) takes the first 64 columns of the set's S once the softmax holds S in registers
+    // tensor memory: S of buffer 0 | S of buffer 1, 64 columns each, | O, 128 columns; P (bfloat16, two keys to a column)
+    // takes the first 32 columns of its S once the softmax holds S in registers
     if (active && warp == kMmaWarp) {
         // ---- the MMAs: the whole warp walks the loop, lane 0 issues ----
         auto issue_s = [&](int j) {
@@ -226,8 +220,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
             const uint64_t qd = umma_desc_k_major_sw128(sQ), kd = umma_desc_k_major_sw128(sK + (j % kKBufs) * kTileBytes);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                const uint64_t off = (uint64_t)(((k >> 2) * kPanel + (k & 3) * 32) >> 4);
-                umma_bf16(tmem + (uint32_t)(b * kN), qd + off, kd + off, idesc(false), k != 0);
+                const uint64_t q_off = (uint64_t)(((k >> 2) * kPanel + (k & 3) * 32) >> 4), k_off = (uint64_t)(((k >> 2) * kKvPanel + (k & 3) * 32) >> 4);
+                umma_bf16(tmem + (uint32_t)(b * kN), qd + q_off, kd + k_off, idesc(false, kN), k != 0);
             }
             umma_commit(&s_full[b]);            // also: the key buffer can be refilled
         };
@@ -243,7 +237,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
             const int b = j & 1;
             const uint32_t parity = (j >> 1) & 1;
             if (j + 1 < num_tiles) {
-                // S(j+1) overwrites S and P of tile j-1 (same set): P V(j-1) was issued before, and the tensor pipe
+                // S(j+1) overwrites S and P of tile j-1 (same buffer): P V(j-1) was issued before, and the tensor pipe
                 // runs what one thread issues in order
                 ok = wait_all(&k_full[(j + 1) % kKBufs], ((j + 1) / kKBufs) & 1, 12);
                 if (!ok) break;
@@ -262,7 +256,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
                     unsigned char* vb = sV + b * kTileBytes;
                     for (int idx = valid_rows * 16 + lane; idx < end * 16; idx += 32) {
                         const int row = idx >> 4, c = idx & 15;
-                        *reinterpret_cast<uint4*>(vb + (c >> 3) * kPanel + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+                        *reinterpret_cast<uint4*>(vb + (c >> 3) * kKvPanel + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
@@ -270,19 +264,18 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
             }
             tcgen05_fence_after();
             if (lane == 0) {
-                // O_b += P V: P is the A operand straight from tensor memory (16 keys = 8 columns per step)
+                // O += P V: P is the A operand straight from tensor memory (16 keys = 8 columns per step)
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const uint64_t vd = desc_mnmajor(sV + b * kTileBytes + k * 16 * 128, kPanel);
-                    mma_ts(tmem + (uint32_t)(2 * kN + b * kN), tmem + (uint32_t)(b * kN + k * 8), vd, idesc(true), (j >= 2) || k != 0);
+                for (int k = 0; k < kN / 16; ++k) {
+                    const uint64_t vd = desc_mnmajor(sV + b * kTileBytes + k * 16 * 128, kKvPanel);
+                    mma_ts(tmem + (uint32_t)(2 * kN), tmem + (uint32_t)(b * kN + k * 8), vd, idesc(true, kD), j > 0 || k != 0);
                 }
                 umma_commit(&pv_done[b]);        // also: the value buffer can be refilled
             }
             __syncwarp();
         }
     } else if (active && warp > kMmaWarp) {
-        // ---- producer warps (first: keys, second: values; two more warps did not make the copies of a tile land sooner:
-        // 64 KB per tile is what an SM fetches from the L2 in about 1.6 k cycles): a lane issues one TMA copy per (page
+        // ---- producer warps (first: keys, second: values): a lane issues one TMA copy per (page
         // of the tile, 64-column panel); keys of tile j+2 as soon as S(j) has read its buffer, values of tile j+2 after P V(j).  Rows of a tile past the
         // request's last page are not copied: their columns of S are masked and P is 0 there.  A page number outside the
         // pool turns into a row outside the tensor map, which reads as zeros and still counts its bytes. ----
@@ -291,7 +284,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
         const int boxes = kN / box_rows;
         // joined: a token's key and value lie side by side in one row of 2 x 128 values (one plane), else in two planes
         const long long total_rows = (long long)num_pages * (joined ? 1 : 2) * nkv * page_size;
-        // a tile has at most 32 boxes (16 pages of 8 slots x 2 panels): lane = box * 2 + panel.  The page number of
+        // a tile has at most 16 boxes (8 pages of 8 slots x 2 panels): lane = box * 2 + panel.  The page number of
         // a lane's box is fetched a tile ahead, so that no copy waits for a round trip to the table.
         const int kv = warp - kMmaWarp - 1;
         const int box = lane >> 1, panel = lane & 1;
@@ -314,7 +307,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
                                           ? (joined ? ((long long)page * nkv + kvh) * page_size + off
                                                     : (((long long)page * 2 + kv) * nkv + kvh) * page_size + off)
                                           : total_rows;
-                tma_load_2d((kv ? sV : sK) + b * kTileBytes + panel * kPanel + box * box_rows * 128, &kv_map, bar,
+                tma_load_2d((kv ? sV : sK) + b * kTileBytes + panel * kKvPanel + box * box_rows * 128, &kv_map, bar,
                             (joined ? kv * kD : 0) + panel * 64, (int)row);
             }
         };
@@ -335,173 +328,124 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
             lookup(j + depth + 1);
         }
     } else if (active && warp < kMmaWarp) {
-        // ---- softmax: all sixteen warps take every key tile, four threads to a row (TMEM lane) with 32 of the 128
-        // columns each; warps w, w + 4, w + 8 and w + 12 share the lanes 32 * (w % 4) .. + 31 and meet at a named barrier
-        // to combine a row's maxima.  Tiles alternate between two sets of scores, running maximum, running sum and
-        // output accumulator (set j % 2), so that the scores of tile j + 1 are computed and the P V of tile j - 1 runs
-        // while the exponentials of tile j are taken; the two sets are merged at the end. ----
-        const int quarter = warp & 3, cq = warp >> 2;
-        const int cb = cq * 32;
-        const int row_local = quarter * 32 + lane;
+        // ---- softmax: a thread per row (TMEM lane 32 * warp + lane); S of the next tile is computed meanwhile ----
+        const int row_local = tid;
         const int grow = row0 + row_local;
         const bool row_ok = grow < rows_total;
         const int pos = row_ok ? seq_len - n + (grow >> g_shift) : -1;
-        const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-        auto row_barrier = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory"); };
-        float m_set[2] = {-INFINITY, -INFINITY}, l_set[2] = {0.f, 0.f};     // indexed by constants only
+        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16), o_addr = lane_addr + 2 * kN;
+        float m_used = -INFINITY, l = 0.f;
         bool ok = true;
-        // one key tile of set B (a constant after inlining); false if a wait ran out
-        auto softmax_tile = [&](int j, auto set) -> bool {
-            constexpr int B = decltype(set)::value;
-            float& m_used = m_set[B];
-            float& l = l_set[B];
-            const uint32_t s_col = (uint32_t)(B * kN), o_col = (uint32_t)(2 * kN + B * kN);
-            const int done = j >> 1;                    // tiles of this set before this one
+        auto wait_here = [&](uint64_t* bar, uint32_t parity, int code) {       // false if the wait ran out
+            bool good = mbar_wait(bar, parity);
+            if (!good && lane == 0) { atomicExch(error_flag, code); s_abort = 1; }
+            return __all_sync(0xffffffffu, good) != 0;
+        };
+        for (int j = 0; j < num_tiles; ++j) {
+            const int b = j & 1;
             const int key0 = k_lo + j * kN;
-            bool good = mbar_wait(&s_full[B], (uint32_t)(done & 1));
-            if (!good && lane == 0) { atomicExch(error_flag, 15); s_abort = 1; }
-            good = __shfl_sync(0xffffffffu, good ? 1 : 0, 0) != 0 && !(*(volatile int*)&s_abort);
-            if (!good) {
-                row_barrier();      // a warp that gives up still meets the row's other warps at every barrier they reach
-                return false;
-            }
+            ok = wait_here(&s_full[b], (uint32_t)((j >> 1) & 1), 15);
+            ok = __all_sync(0xffffffffu, ok && !(*(volatile int*)&s_abort)) != 0;
+            if (!ok) break;
             tcgen05_fence_after();
             const bool need_mask = key0 + kN - 1 > pos || window > 0;
             const int hi = pos - key0;                              // columns <= hi are visible ...
             const int lo = window > 0 ? hi - window : -1;           // ... and > lo
-            // this thread's 32 scores, read from tensor memory once; masked ones become -inf here, so that the
+            // the row's 64 scores, read from tensor memory once; masked ones become -inf here, so that the
             // maximum (the scale is positive: applied afterwards) and the exponentials need no second look at the mask
-            uint32_t v[32];
-            tmem_ld_32x32b_x32(lane_addr + s_col + (uint32_t)cb, v);
+            uint32_t v[2][32];
+            tmem_ld_32x32b_x32(lane_addr + (uint32_t)(b * kN), v[0]);
+            tmem_ld_32x32b_x32(lane_addr + (uint32_t)(b * kN + 32), v[1]);
             tmem_ld_wait();
-            float mx = -INFINITY;
             if (need_mask) {
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    const int col = cb + e;
-                    if (!(col <= hi && col > lo)) v[e] = __float_as_uint(-INFINITY);
-                }
+                for (int e = 0; e < kN; ++e)
+                    if (!(e <= hi && e > lo)) v[e / 32][e % 32] = __float_as_uint(-INFINITY);
             }
+            float part[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(v[e]));
-            s_mx[B][cq][row_local] = mx;
-            row_barrier();                          // all four threads of the row hold their scores in registers from here on
-            mx = fmaxf(fmaxf(s_mx[B][0][row_local], s_mx[B][1][row_local]), fmaxf(s_mx[B][2][row_local], s_mx[B][3][row_local])) * scale_log2;
-            // raise the reference maximum only when it would grow by more than 8 (values stay below 2^8); the
-            // threads of a row see the same numbers and decide alike
+            for (int e = 0; e < kN; ++e) part[e & 3] = fmaxf(part[e & 3], __uint_as_float(v[e / 32][e % 32]));
+            const float mx = fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3])) * scale_log2;
+            // raise the reference maximum only when it would grow by more than 8 (values stay below 2^8)
             float corr = 1.f;
             bool rescale = false;
             if (mx > m_used + 8.f || (m_used == -INFINITY && mx != -INFINITY)) {
                 corr = m_used == -INFINITY ? 0.f : exp2f(m_used - mx);
                 m_used = mx;
                 l *= corr;
-                rescale = done > 0;
+                rescale = j > 0;
             }
             // P = 2^(s * scale - m): one fused multiply-add and one ex2 per score, packed two to a register
             const float m_eff = m_used == -INFINITY ? 0.f : m_used;
-            uint32_t p[16];
+            uint32_t p[32];
+            float sums[2] = {0.f, 0.f};
 #pragma unroll
-            for (int e = 0; e < 32; e += 2) {
+            for (int e = 0; e < kN; e += 2) {
                 float pe[2];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    const float x = fmaf(__uint_as_float(v[e + u]), scale_log2, -m_eff);
+                    const float x = fmaf(__uint_as_float(v[e / 32][e % 32 + u]), scale_log2, -m_eff);
                     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(pe[u]) : "f"(x));
+                    sums[u] += pe[u];
                 }
-                l += pe[0] + pe[1];
                 __nv_bfloat162 pk = __floats2bfloat162_rn(pe[0], pe[1]);
                 p[e / 2] = *reinterpret_cast<uint32_t*>(&pk);
             }
-            // the set's O is only touched once P V of its tile before has finished
-            if (done > 0 && __any_sync(0xffffffffu, rescale)) {
-                good = mbar_wait(&pv_done[B], (uint32_t)((done - 1) & 1));
-                if (!good && lane == 0) { atomicExch(error_flag, 16); s_abort = 1; }
-                good = __shfl_sync(0xffffffffu, good ? 1 : 0, 0) != 0;
-                if (!good) return false;
+            l += sums[0] + sums[1];
+            // O is only touched once P V of the tile before has finished
+            if (j > 0 && __any_sync(0xffffffffu, rescale)) {
+                ok = wait_here(&pv_done[b ^ 1], (uint32_t)(((j - 1) >> 1) & 1), 16);
+                if (!ok) break;
                 tcgen05_fence_after();
-                uint32_t o[32];
-                tmem_ld_32x32b_x32(lane_addr + o_col + (uint32_t)cb, o);
-                tmem_ld_wait();
+#pragma unroll 1
+                for (int c = 0; c < kD; c += 32) {
+                    uint32_t o[32];
+                    tmem_ld_32x32b_x32(o_addr + (uint32_t)c, o);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * (rescale ? corr : 1.f));
-                tst32(lane_addr + o_col + (uint32_t)cb, o);
+                    for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
+                    tst32(o_addr + (uint32_t)c, o);
+                }
             }
-            // P (bfloat16, two keys to a column): this thread's 32 keys take the columns 16 cq .. + 15, over scores
-            // that the row's threads hold in registers since the barrier above
-            tst16(lane_addr + s_col + (uint32_t)(cq * 16), p);
+            // P (bfloat16, two keys to a column) over the scores, which this row's thread holds in registers
+            tst32(lane_addr + (uint32_t)(b * kN), p);
             tst_wait();
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&p_ready[B]);
-            return true;
-        };
-        for (int j = 0; j < num_tiles; j += 2) {
-            // after a wait has run out (never in a healthy run) only the tiles' barriers are kept, so that no warp of
-            // the row is left waiting at one
-            if (ok) ok = softmax_tile(j, std::integral_constant<int, 0>{});
-            else row_barrier();
-            if (j + 1 < num_tiles) {
-                if (ok) ok = softmax_tile(j + 1, std::integral_constant<int, 1>{});
-                else row_barrier();
-            }
+            if (lane == 0) mbar_arrive(&p_ready[b]);
         }
-        // ---- merge the two sets: O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)) ----
-        // every thread waits for the last P V of both sets itself: behind them no MMA reads shared or tensor memory
-#pragma unroll
-        for (int B = 0; B < 2; ++B) {
-            if (ok && num_tiles > B) {
-                const int last = ((num_tiles - 1 - B) >> 1);        // the set's last tile is its (last + 1)-th
-                ok = mbar_wait(&pv_done[B], (uint32_t)(last & 1));
-                if (!ok && lane == 0) { atomicExch(error_flag, 17); s_abort = 1; }
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            }
-        }
-        s_l[0][cq][row_local] = l_set[0];
-        s_l[1][cq][row_local] = l_set[1];
-        tcgen05_fence_before();
-        row_barrier();                  // the four threads of a row
+        // every thread waits for the last P V itself: behind it no MMA reads shared or tensor memory
+        if (ok && num_tiles > 0) ok = wait_here(&pv_done[(num_tiles - 1) & 1], (uint32_t)(((num_tiles - 1) >> 1) & 1), 17);
         tcgen05_fence_after();
         if (!(*(volatile int*)&s_abort) && num_tiles > 0) {
-            // this thread stores the output columns 32 cq .. + 31 of its row
-            const float m0 = m_set[0], m1 = m_set[1];
-            const float l0 = (s_l[0][0][row_local] + s_l[0][1][row_local]) + (s_l[0][2][row_local] + s_l[0][3][row_local]);
-            const float l1 = (s_l[1][0][row_local] + s_l[1][1][row_local]) + (s_l[1][2][row_local] + s_l[1][3][row_local]);
-            const float m = fmaxf(m0, m1);
-            const float w0 = m0 == -INFINITY ? 0.f : exp2f(m0 - m), w1 = m1 == -INFINITY ? 0.f : exp2f(m1 - m);
-            float total = l0 * w0 + l1 * w1;
+            float total = l;
             // a sink is a score of the row's head without key or value: it joins the denominator once, unscaled
             float keep = 1.f;
             if (sinks != nullptr && row_ok) {
                 const float sink = sinks[kvh * g + (grow & (g - 1))] * 1.4426950408889634f;
-                const float top = fmaxf(m, sink);
-                keep = m == -INFINITY ? 0.f : exp2f(m - top);
+                const float top = fmaxf(m_used, sink);
+                keep = m_used == -INFINITY ? 0.f : exp2f(m_used - top);
                 total = total * keep + exp2f(sink - top);
             }
             // (total is at least 2^-8 for a row with a visible key and at most a few thousand)
-            const float inv = total > 0.f ? __fdividef(1.f, total) : 0.f;
-            const float f0 = w0 * keep * inv, f1 = w1 * keep * inv;
-            const bool has1 = num_tiles > 1;        // set 1 has an accumulator only if there was a second tile
-            uint32_t a[32], b[32];
-            tmem_ld_32x32b_x32(lane_addr + (uint32_t)(2 * kN + cb), a);
-            if (has1) tmem_ld_32x32b_x32(lane_addr + (uint32_t)(3 * kN + cb), b);
-            tmem_ld_wait();
+            const float f = keep * (total > 0.f ? __fdividef(1.f, total) : 0.f);
             // into the query tile's shared memory (every S has read it), a row's 256 bytes together, its 16-byte pieces
             // swapped by the row number so that neither these stores nor the loads below meet in a bank
+#pragma unroll 1
+            for (int c = 0; c < kD; c += 32) {
+                uint32_t o[32];
+                tmem_ld_32x32b_x32(o_addr + (uint32_t)c, o);
+                tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-                float y[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    y[u] = __uint_as_float(a[e + u]) * f0;
-                    if (has1) y[u] = fmaf(__uint_as_float(b[e + u]), f1, y[u]);
+                for (int e = 0; e < 32; e += 8) {
+                    uint4 pk;
+                    pk.x = pack_bf16(__uint_as_float(o[e]) * f, __uint_as_float(o[e + 1]) * f);
+                    pk.y = pack_bf16(__uint_as_float(o[e + 2]) * f, __uint_as_float(o[e + 3]) * f);
+                    pk.z = pack_bf16(__uint_as_float(o[e + 4]) * f, __uint_as_float(o[e + 5]) * f);
+                    pk.w = pack_bf16(__uint_as_float(o[e + 6]) * f, __uint_as_float(o[e + 7]) * f);
+                    const int piece = (c + e) >> 3;
+                    *reinterpret_cast<uint4*>(sQ + row_local * 256 + ((piece ^ (row_local & 15)) << 4)) = pk;
                 }
-                uint4 pk;
-                __nv_bfloat162 t0 = __floats2bfloat162_rn(y[0], y[1]), t1 = __floats2bfloat162_rn(y[2], y[3]);
-                __nv_bfloat162 t2 = __floats2bfloat162_rn(y[4], y[5]), t3 = __floats2bfloat162_rn(y[6], y[7]);
-                pk.x = *reinterpret_cast<uint32_t*>(&t0); pk.y = *reinterpret_cast<uint32_t*>(&t1);
-                pk.z = *reinterpret_cast<uint32_t*>(&t2); pk.w = *reinterpret_cast<uint32_t*>(&t3);
-                const int piece = (cb + e) >> 3;
-                *reinterpret_cast<uint4*>(sQ + row_local * 256 + ((piece ^ (row_local & 15)) << 4)) = pk;
             }
         }
         // out to global memory sixteen threads to a row: a thread that stored its own row's pieces sent 32 partial
@@ -523,7 +467,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
     }
     tcgen05_fence_before();
     __syncthreads();
-    if (warp == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    if (warp == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTmemCols) : "memory");
 }
 
 }  // namespace fa
@@ -556,21 +500,25 @@ extern "C" int cib_attention_tcgen05(const void* q, int q_stride, void* out, int
     // page_size, 256] with the key in the first and the value in the second half of a row; a box is one page x 64 columns
     const long long total_rows = (long long)num_pages * (joined ? 1 : 2) * nkv * page_size;
     CIB_REQUIRE(total_rows < (1ll << 31), "attention_tcgen05: %lld cache rows do not fit a 32-bit coordinate", total_rows);
+    // few CTAs: the variant that has an SM alone (attention_tcgen05_wide.cu says why the line lies here)
+    const bool wide = (long long)nkv * num_tiles <= 2 * 148;
+    const int tile_keys = wide ? kWideKeys : fa::kN;
     CUtensorMap kv_map;
     const int row_values = joined ? 2 * fa::kD : fa::kD;
     if (encode_tensor_map_bf16_2d(&kv_map, cache, (unsigned long long)total_rows, row_values, row_values, 64,
-                                  page_size < fa::kN ? page_size : fa::kN, "attention_tcgen05") != 0)
+                                  page_size < tile_keys ? page_size : tile_keys, "attention_tcgen05") != 0)
         return -1;
+    const float scale_log2 = scale * 1.4426950408889634f;
+    if (wide)
+        return attention_tcgen05_wide(kv_map, num_pages, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, page_size, block_table,
+                                      table_stride, query_start_loc, seq_lens, num_requests, num_tiles, nq, nkv, scale_log2, window, joined,
+                                      sinks, error_flag, stream);
     static SmemLimit limit;
     if (int rc = raise_smem_limit(limit, fa::attention_tcgen05_kernel, fa::kSmemBytes, "attention_tcgen05")) return rc;
-    dim3 grid(nkv, num_tiles);
-    cudaError_t e = launch_pdl(fa::attention_tcgen05_kernel, grid, dim3(fa::kThreads), (size_t)fa::kSmemBytes, stream, prompt_pdl(),
-                               kv_map, num_pages, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, page_size,
-                               block_table, table_stride, query_start_loc, seq_lens, num_requests, nq, nkv,
-                               scale * 1.4426950408889634f, window, joined, sinks, error_flag);
-    if (e != cudaSuccess) {
-        set_error("attention_tcgen05: launch failed: %s", cudaGetErrorString(e));
-        return -2;
-    }
+    const cudaError_t e = launch_pdl(fa::attention_tcgen05_kernel, dim3(nkv, num_tiles), dim3(fa::kThreads), (size_t)fa::kSmemBytes, stream,
+                                     prompt_pdl(), kv_map, num_pages, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride,
+                                     page_size, block_table, table_stride, query_start_loc, seq_lens, num_requests, nq, nkv, scale_log2,
+                                     window, joined, sinks, error_flag);
+    CIB_REQUIRE(e == cudaSuccess, "attention_tcgen05: launch failed: %s", cudaGetErrorString(e));
     return 0;
 }

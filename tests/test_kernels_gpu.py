@@ -544,6 +544,26 @@ def test_paged_attention_prefill(nq, nkv, d, ps, window):
     close(out, attention_reference(case, lens, new, scale, window), 1.5e-2)
 
 
+@pytest.mark.parametrize("nq, nkv, ps", [(16, 8, 16), (20, 20, 8), (32, 16, 64), (16, 8, 256)])
+@pytest.mark.parametrize("window", [None, 100])
+def test_attention_tcgen05_many_ctas(nq, nkv, ps, window):
+    """Launches of more than two CTAs a SM: tiles of 64 keys whose ends the contexts meet, miss by one and cross, late
+    portions, and a far key that dominates after weaker ones; empty slots are NaN."""
+    k = _k()
+    d, lens, new = 128, [64, 65, 63, 128, 129, 1000, 700, 513, 1, 900], [64, 65, 63, 128, 1, 700, 77, 513, 1, 640]
+    if sum((n * (nq // nkv) + 127) // 128 for n in new) * nkv <= 296:
+        lens, new = lens * 2, new * 2
+    assert sum((n * (nq // nkv) + 127) // 128 for n in new) * nkv > 296
+    case = attention_case(torch.bfloat16, nq, nkv, d, lens, new, ps, seed=81, sharp=True, poison=True)
+    scale = 1.0 / math.sqrt(d)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    out = torch.full((sum(new), nq * d), 5.0, dtype=torch.bfloat16, device=DEV)
+    k.attention_tcgen05(case["wide"].to(DEV), out, case["cache"].to(DEV), case["bt"].to(DEV), i32(case["qsl"]), i32(lens), new, nq, nkv,
+                        d, scale, window or 0)
+    k.check_error_flags()
+    close(out, attention_reference(case, lens, new, scale, window), 1.5e-2)
+
+
 @pytest.mark.parametrize("nq, nkv, ps", [(16, 8, 16), (8, 1, 32), (4, 4, 8), (32, 2, 128), (2, 1, 256)])
 @pytest.mark.parametrize("window", [None, 200])
 def test_attention_tcgen05(nq, nkv, ps, window):
