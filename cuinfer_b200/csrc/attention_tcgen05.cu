@@ -6,8 +6,8 @@
 //
 //   * a CTA owns a 128-row query tile (128 / g tokens x g heads of one kv head) and walks over 64-key tiles; two CTAs share
 //     an SM (256 columns of tensor memory and 97 KB of shared memory each), so that one takes exponentials while the other
-//     starts, waits for its first keys or stores (8 prompts of 1 024 tokens, 16 heads over 8: 67.5 us a layer, 510 TFLOP/s,
-//     where one CTA an SM, 128-key tiles and sixteen softmax warps took 88.7; one of 8 192: 268.6 us, 1 024 TFLOP/s, for 327).
+//     starts, waits for its first keys or stores (8 prompts of 1 024 tokens, 16 heads over 8: 72 us a layer, 475 TFLOP/s,
+//     where one CTA an SM, 128-key tiles and sixteen softmax warps took 89; one of 8 192: 275 us, 1 000 TFLOP/s, for 328).
 //     Launches of few CTAs run that other variant (attention_tcgen05_wide.cu);
 //   * keys and values come page by page through TMA (`cp.async.bulk.tensor.2d`, one box of 64 columns x one page per
 //     copy, 128-byte swizzle: the layout the tensor cores read), issued by the lanes of the producer warps,
@@ -366,16 +366,19 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
 #pragma unroll
             for (int e = 0; e < kN; ++e) part[e & 3] = fmaxf(part[e & 3], __uint_as_float(v[e / 32][e % 32]));
             const float mx = fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3])) * scale_log2;
-            // raise the reference maximum only when it would grow by more than 8 (values stay below 2^8)
+            // raise the reference maximum only when it would grow by more than 8 (values stay below 2^8) — but whenever it grows
+            // over the first 256 keys, so that a short context's largest weight is 1 and not rounded
             float corr = 1.f;
             bool rescale = false;
-            if (mx > m_used + 8.f || (m_used == -INFINITY && mx != -INFINITY)) {
+            if (mx > m_used + (j < 256 / kN ? 0.f : 8.f) || (m_used == -INFINITY && mx != -INFINITY)) {
                 corr = m_used == -INFINITY ? 0.f : exp2f(m_used - mx);
                 m_used = mx;
                 l *= corr;
                 rescale = j > 0;
             }
-            // P = 2^(s * scale - m): one fused multiply-add and one ex2 per score, packed two to a register
+            // P = 2^(s * scale - m): one fused multiply-add and one ex2 per score, packed two to a register.  The sum is of the
+            // weights as they are multiplied, rounded: the reference maximum lags behind, so that even a row's largest weight
+            // is rounded, and only a sum that has the same rounding takes it out again
             const float m_eff = m_used == -INFINITY ? 0.f : m_used;
             uint32_t p[32];
             float sums[2] = {0.f, 0.f};
@@ -386,10 +389,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
                 for (int u = 0; u < 2; ++u) {
                     const float x = fmaf(__uint_as_float(v[e / 32][e % 32 + u]), scale_log2, -m_eff);
                     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(pe[u]) : "f"(x));
-                    sums[u] += pe[u];
                 }
-                __nv_bfloat162 pk = __floats2bfloat162_rn(pe[0], pe[1]);
-                p[e / 2] = *reinterpret_cast<uint32_t*>(&pk);
+                p[e / 2] = pack_bf16(pe[0], pe[1]);
+                sums[0] += __uint_as_float(p[e / 2] << 16);
+                sums[1] += __uint_as_float(p[e / 2] & 0xffff0000u);
             }
             l += sums[0] + sums[1];
             // O is only touched once P V of the tile before has finished
@@ -501,7 +504,7 @@ extern "C" int cib_attention_tcgen05(const void* q, int q_stride, void* out, int
     const long long total_rows = (long long)num_pages * (joined ? 1 : 2) * nkv * page_size;
     CIB_REQUIRE(total_rows < (1ll << 31), "attention_tcgen05: %lld cache rows do not fit a 32-bit coordinate", total_rows);
     // few CTAs: the variant that has an SM alone (attention_tcgen05_wide.cu says why the line lies here)
-    const bool wide = (long long)nkv * num_tiles <= 2 * 148;
+    const bool wide = (long long)nkv * num_tiles <= 3 * 148;
     const int tile_keys = wide ? kWideKeys : fa::kN;
     CUtensorMap kv_map;
     const int row_values = joined ? 2 * fa::kD : fa::kD;

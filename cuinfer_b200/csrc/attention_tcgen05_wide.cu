@@ -7,9 +7,10 @@
 //   * four threads share a row (TMEM lane = row, 32 columns each): they read S with one `tcgen05.ld`, keep the running
 //     maximum in base 2 and raise it only when it grows by more than 8.
 //
-// A tile of 128 keys takes it about 1.9 us; one CTA of the other variant takes 2.2 us for 128 keys, but an SM has two of
-// them.  So this one is better while a launch has at most two CTAs for each SM and its longest row tile decides (one prompt
-// of 2 048 tokens, 256 CTAs: 31.9 us a layer against 39.8), the other beyond.
+// A tile of 128 keys takes it about 1.9 us; one CTA of the other variant takes 2.2 us or more for 128 keys, but an SM has two
+// of them.  So this one is better while a launch has at most three CTAs for each SM and its longest row tile decides (one
+// prompt of 2 048 tokens, 256 CTAs: 31.9 us a layer against 39.8; of 2 560, 320 CTAs: 48.8 against 50.6), the other beyond
+// (one of 8 192, 1 024 CTAs: 328 us against 275).
 //
 // Every mbarrier wait is bounded; on a time-out the kernel raises the error flag, stops, frees its tensor memory
 // and returns.

@@ -547,13 +547,13 @@ def test_paged_attention_prefill(nq, nkv, d, ps, window):
 @pytest.mark.parametrize("nq, nkv, ps", [(16, 8, 16), (20, 20, 8), (32, 16, 64), (16, 8, 256)])
 @pytest.mark.parametrize("window", [None, 100])
 def test_attention_tcgen05_many_ctas(nq, nkv, ps, window):
-    """Launches of more than two CTAs a SM: tiles of 64 keys whose ends the contexts meet, miss by one and cross, late
+    """Launches of more than three CTAs a SM: tiles of 64 keys whose ends the contexts meet, miss by one and cross, late
     portions, and a far key that dominates after weaker ones; empty slots are NaN."""
     k = _k()
     d, lens, new = 128, [64, 65, 63, 128, 129, 1000, 700, 513, 1, 900], [64, 65, 63, 128, 1, 700, 77, 513, 1, 640]
-    if sum((n * (nq // nkv) + 127) // 128 for n in new) * nkv <= 296:
+    if sum((n * (nq // nkv) + 127) // 128 for n in new) * nkv <= 444:
         lens, new = lens * 2, new * 2
-    assert sum((n * (nq // nkv) + 127) // 128 for n in new) * nkv > 296
+    assert sum((n * (nq // nkv) + 127) // 128 for n in new) * nkv > 444
     case = attention_case(torch.bfloat16, nq, nkv, d, lens, new, ps, seed=81, sharp=True, poison=True)
     scale = 1.0 / math.sqrt(d)
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
