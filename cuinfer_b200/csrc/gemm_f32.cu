@@ -16,7 +16,8 @@ namespace cib {
 
 // ---- few rows ----------------------------------------------------------------------------------------------------------
 // A warp takes 8 output features x 512 of K: all of its 16 KB of weights are on their way to shared memory before it looks
-// at the activations (with programmatic dependent launch before the kernel that computes them has ended), so an SM has its
+// at the activations (with programmatic dependent launch, and where the caller says that nothing in flight writes the
+// weights, before the kernel that computes the activations has ended), so an SM has its
 // whole share of a projection in flight at once.  A lane then owns one feature and one slice of 128: its chains need no
 // exchange with other lanes, and only the slices' sums meet in shared memory, once.  Rows of the weights lie 2 064 bytes
 // apart and slices of the activations 528: eight lanes read eight weight rows without a bank conflict, and the warp's
@@ -42,6 +43,7 @@ gemm_f32_few_kernel(const GemmF32 p, int rounds) {
     const int n0 = blockIdx.x * kFewFeatures;
     const int feature = lane & 7, slice = lane >> 3;
 
+    if (!p.w_constant) griddep_wait();
     for (int m0 = 0; m0 < p.M; m0 += MT) {
         for (int r = 0; r < rounds; ++r) {
             const int chunk = warp + r * warps, k0 = chunk * kFewChunk;

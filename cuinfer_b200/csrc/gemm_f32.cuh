@@ -27,6 +27,7 @@ struct GemmF32 {
     const float* a; const float* w; float* out;
     int lda, ldw, ldo, M, N, K;
     long long a_batch, w_batch, o_batch;
+    bool w_constant;             // no kernel still in flight writes `w` (a model's loaded weights): it may be read before the wait
 };
 
 // Whether the kernels of gemm_f32.cu take these operands: every row of both starts on a 16-byte boundary.

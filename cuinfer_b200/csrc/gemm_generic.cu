@@ -90,12 +90,12 @@ using namespace cib;
 
 static int gemm_generic_launch(const void* a, int lda, long long a_batch, const void* w, int ldw, long long w_batch,
                                int in_dtype, void* out, int ldo, long long o_batch, int out_dtype, int M, int N, int K,
-                               int batch, cudaStream_t stream) {
+                               int batch, int w_constant, cudaStream_t stream) {
     CIB_REQUIRE(M >= 0 && N > 0 && K > 0 && batch > 0, "gemm: bad sizes M=%d N=%d K=%d batch=%d", M, N, K, batch);
     CIB_REQUIRE(lda >= K && ldw >= K && ldo >= N, "gemm: leading dimensions too small (lda=%d ldw=%d ldo=%d)", lda, ldw, ldo);
     if (M == 0) return 0;
     if (in_dtype == kF32 && out_dtype == kF32) {
-        const GemmF32 p{(const float*)a, (const float*)w, (float*)out, lda, ldw, ldo, M, N, K, a_batch, w_batch, o_batch};
+        const GemmF32 p{(const float*)a, (const float*)w, (float*)out, lda, ldw, ldo, M, N, K, a_batch, w_batch, o_batch, w_constant != 0};
         if (gemm_f32_takes(p, batch)) return gemm_f32_launch(p, batch, stream);
     }
     dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, batch);
@@ -112,15 +112,16 @@ static int gemm_generic_launch(const void* a, int lda, long long a_batch, const 
     return 0;
 }
 
+// w_constant: no kernel still in flight in the stream writes `w`; without it a kernel launched early waits before it reads `w`.
 extern "C" int cib_gemm_generic(const void* a, int lda, const void* w, int ldw, int in_dtype, void* out, int ldo,
-                                int out_dtype, int M, int N, int K, cudaStream_t stream) {
-    return gemm_generic_launch(a, lda, 0, w, ldw, 0, in_dtype, out, ldo, 0, out_dtype, M, N, K, 1, stream);
+                                int out_dtype, int M, int N, int K, int w_constant, cudaStream_t stream) {
+    return gemm_generic_launch(a, lda, 0, w, ldw, 0, in_dtype, out, ldo, 0, out_dtype, M, N, K, 1, w_constant, stream);
 }
 
 // `batch` independent products out[b] = a[b] . w[b]^T whose operands lie a_batch / w_batch / o_batch elements apart
 // (heads side by side inside wider rows: the batch stride is then smaller than the leading dimension).
 extern "C" int cib_gemm_generic_batched(const void* a, int lda, long long a_batch, const void* w, int ldw,
                                         long long w_batch, int in_dtype, void* out, int ldo, long long o_batch,
-                                        int out_dtype, int M, int N, int K, int batch, cudaStream_t stream) {
-    return gemm_generic_launch(a, lda, a_batch, w, ldw, w_batch, in_dtype, out, ldo, o_batch, out_dtype, M, N, K, batch, stream);
+                                        int out_dtype, int M, int N, int K, int batch, int w_constant, cudaStream_t stream) {
+    return gemm_generic_launch(a, lda, a_batch, w, ldw, w_batch, in_dtype, out, ldo, o_batch, out_dtype, M, N, K, batch, w_constant, stream);
 }

@@ -86,7 +86,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cib_latent_attention_mma": [_P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _P, _I, _P, _I, _I, _I, _I,
                                      _F, _I, _F, _I, _P],
         "cib_gemm_generic_batched": [_P, _I, ctypes.c_longlong, _P, _I, ctypes.c_longlong, _I, _P, _I, ctypes.c_longlong, _I,
-                                     _I, _I, _I, _I, _P],
+                                     _I, _I, _I, _I, _I, _P],
         "cib_moe_table_gate_up": [_P, _I, _I, _P, _P, _I, _I, _I, _P, _P, _I, _I, _I, _I, _F, _P],
         "cib_moe_table_grouped": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _F, _P, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _F, _P],
         "cib_moe_table_down": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _F, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _P],
@@ -122,7 +122,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cib_gemm_skinny": [_P, _I, _I, _I, _P, _I, _P, _P, _I, _P, _I, _F, _P, _P, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P],
         "cib_gemm_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
         "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
-        "cib_gemm_generic": [_P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _P],
+        "cib_gemm_generic": [_P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P],
         "cib_sample": [_P, _I, _I, _I, _P, _P, _P],
         "cib_argmax_rows": [_P, _I, _I, _I, _P, _P],
         "cib_selftest_bounded_wait": [ctypes.c_longlong, _P, _P, _P],
@@ -733,8 +733,9 @@ def paged_attention_prefill(q: torch.Tensor, out: torch.Tensor, cache: torch.Ten
 
 # ---- matrix product ----------------------------------------------------------------------------------
 
-def gemm_generic(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M, N] = a[M, K] @ w[N, K]^T with 32-bit FMA accumulation, any sizes."""
+def gemm_generic(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, constant_w: bool = False) -> None:
+    """out[M, N] = a[M, K] @ w[N, K]^T with 32-bit FMA accumulation, any sizes.  ``constant_w``: no kernel still in flight
+    writes ``w`` (a model's loaded weights), so that it may be read before the kernel ahead in the stream has ended."""
     M, K = a.shape
     N, K2 = w.shape
     if K != K2 or out.shape != (M, N) or a.dtype != w.dtype:
@@ -743,14 +744,15 @@ def gemm_generic(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         raise KernelError("gemm: rows must be dense")
     rc = library().cib_gemm_generic(
         _cuda(a, "a", contiguous=False), a.stride(0), _cuda(w, "w", contiguous=False), w.stride(0), _code(a, "a"),
-        _cuda(out, "out", contiguous=False), out.stride(0), _code(out, "out"), M, N, K, _stream())
+        _cuda(out, "out", contiguous=False), out.stride(0), _code(out, "out"), M, N, K, int(constant_w), _stream())
     _check(rc, "gemm_generic")
     _count()
 
 
-def gemm_generic_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+def gemm_generic_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, constant_w: bool = False) -> None:
     """out[b, M, N] = a[b, M, K] @ w[b, N, K]^T for every b, 32-bit FMA accumulation, any sizes.  The three tensors
-    may be strided views (heads side by side inside wider rows); only their last axis must be dense."""
+    may be strided views (heads side by side inside wider rows); only their last axis must be dense.  ``constant_w`` as for
+    :func:`gemm_generic`."""
     B, M, K = a.shape
     B2, N, K2 = w.shape
     if B != B2 or K != K2 or out.shape != (B, M, N) or a.dtype != w.dtype:
@@ -759,7 +761,8 @@ def gemm_generic_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) ->
         raise KernelError("gemm: rows must be dense")
     rc = library().cib_gemm_generic_batched(
         _cuda(a, "a", contiguous=False), a.stride(1), a.stride(0), _cuda(w, "w", contiguous=False), w.stride(1), w.stride(0),
-        _code(a, "a"), _cuda(out, "out", contiguous=False), out.stride(1), out.stride(0), _code(out, "out"), M, N, K, B, _stream())
+        _code(a, "a"), _cuda(out, "out", contiguous=False), out.stride(1), out.stride(0), _code(out, "out"), M, N, K, B,
+        int(constant_w), _stream())
     _check(rc, "gemm_generic_batched")
     _count()
 

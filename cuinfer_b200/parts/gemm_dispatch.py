@@ -104,4 +104,4 @@ def bf16_matmul_nt(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> 
         if out.dtype == torch.float32:
             torch.mm(x, weight.t(), out_dtype=torch.float32, out=out)
             return
-    kernels.gemm_generic(x, weight, out)
+    kernels.gemm_generic(x, weight, out, constant_w=True)

@@ -21,7 +21,8 @@ from .spec import TensorSpec
 
 
 def matmul_nt(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """``x[M, K] @ weight[N, K]^T`` → ``[M, N]`` in ``out_dtype`` (default: x's dtype)."""
+    """``x[M, K] @ weight[N, K]^T`` → ``[M, N]`` in ``out_dtype`` (default: x's dtype); ``weight`` is loaded, not computed by
+    the kernels in flight."""
     M, K = x.shape
     N = weight.shape[0]
     out_dtype = out_dtype or x.dtype
@@ -29,7 +30,7 @@ def matmul_nt(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.d
     if M == 0:
         return out
     if x.dtype == torch.float32:
-        kernels.gemm_generic(x, weight, out)
+        kernels.gemm_generic(x, weight, out, constant_w=True)
         return out
     from . import gemm_dispatch
     gemm_dispatch.bf16_matmul_nt(x, weight, out)
@@ -38,7 +39,8 @@ def matmul_nt(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.d
 
 def per_head_products(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     """``out[h] = a[h] @ w[h]^T`` for every head h, or for every one of several products of one size; ``a [H, T, K]`` and
-    ``out [H, T, N]`` may be views of rows in which the heads lie side by side, ``w [H, N, K]`` is dense.  bfloat16 with
+    ``out [H, T, N]`` may be views of rows in which the heads lie side by side, ``w [H, N, K]`` is dense and loaded, not
+    computed by the kernels in flight.  bfloat16 with
     sizes in multiples of 8: the library's strided batched product (as for the plain projections); else the FMA kernel,
     which is also the 32-bit path."""
     from . import gemm_dispatch  # noqa: F401  (sets the library products to 32-bit accumulation before the first one runs)
@@ -49,7 +51,7 @@ def per_head_products(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
         torch.bmm(a, w.transpose(1, 2), out=out)
         kernels.launch_count += 1
         return
-    kernels.gemm_generic_batched(a, w, out)
+    kernels.gemm_generic_batched(a, w, out, constant_w=True)
 
 
 def padded_rows(weight: torch.Tensor, multiple: int = 8) -> torch.Tensor:

@@ -167,6 +167,27 @@ def test_gemm_32bit_paths(N, K):
     assert torch.equal(batch.view(120, N), full[:120])
 
 
+@pytest.mark.parametrize("M", [1, 8, 33, 200])
+@pytest.mark.parametrize("batched", [False, True])
+def test_gemm_32bit_waits_for_a_computed_operand(M, batched):
+    """A second operand that the kernel ahead in the stream is still writing, when that kernel lets the next one start
+    early: every kernel of the 32-bit products waits for it unless the caller says that it is constant."""
+    k = _k()
+    N, K = 24576, 1024
+    gate_up, a = rand(N, 2 * K, seed=93).to(DEV), rand(M, K, seed=94).to(DEV)
+    w = torch.zeros(N, K, device=DEV)
+    product = (lambda c, o: k.gemm_generic_batched(a[None], c[None], o[None])) if batched else (lambda c, o: k.gemm_generic(a, c, o))
+    want, got = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    k.silu_mul(gate_up, w)
+    torch.cuda.synchronize()
+    product(w, want)
+    for _ in range(3):
+        w.zero_()
+        k.silu_mul(gate_up, w)
+        product(w, got)
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("M, N, K", [(128, 128, 64), (128, 256, 128), (17, 1000, 96), (300, 517 + 3, 72),
                                      (2048, 4096, 1024), (640, 1024, 3072), (129, 6144, 1024), (200, 136, 2048)])
 @pytest.mark.parametrize("f32_out", [False, True])
