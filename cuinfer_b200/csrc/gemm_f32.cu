@@ -346,6 +346,7 @@ static_assert(kFewMaxWarps * (kFewFeatures * kFewWRow + kFewRows * kFewARow) + 5
               "shared memory of the largest few-rows launch");
 
 int gemm_f32_launch(const GemmF32& p, int batch, cudaStream_t stream) {
+    CIB_REQUIRE((p.M + kTileM - 1) / kTileM <= 65535 && batch <= 65535, "gemm: M=%d or batch=%d too large for this kernel", p.M, batch);
     const bool one_round = p.K <= kFewChunk * kFewMaxWarps;
     if (p.K <= kFewMaxK && (p.M <= kFewRows || (p.M <= kFewMaxRows && one_round))) {
         switch (p.M) {
@@ -361,10 +362,10 @@ int gemm_f32_launch(const GemmF32& p, int batch, cudaStream_t stream) {
     }
     const int groups = f32_groups(p.K);
     const dim3 grid((p.N + kTileN - 1) / kTileN, (p.M + kTileM - 1) / kTileM, batch);
-    CIB_REQUIRE(grid.y <= 65535 && (long long)batch * groups <= 65535, "gemm: M=%d or batch=%d too large for this kernel", p.M, batch);
-    // rounds of resident CTAs, in groups of K: a tile whole, or its groups apart where that fills the last round better
+    // rounds of resident CTAs, in groups of K: a tile whole, or its groups apart where that fills the last round better (and
+    // the launch's z extent holds them)
     const long long tiles = (long long)grid.x * grid.y * batch;
-    const bool split = groups > 1 && (tiles * groups + kTileCtas - 1) / kTileCtas < (tiles + kTileCtas - 1) / kTileCtas * groups;
+    const bool split = groups > 1 && (long long)batch * groups <= 65535 && (tiles * groups + kTileCtas - 1) / kTileCtas < (tiles + kTileCtas - 1) / kTileCtas * groups;
     static SmemLimit limit_split, limit_whole;
     cudaError_t e;
     if (split) {

@@ -167,6 +167,26 @@ def test_gemm_32bit_paths(N, K):
     assert torch.equal(batch.view(120, N), full[:120])
 
 
+def test_gemm_32bit_many_products():
+    """As many products at once as a launch's extent holds, also where every one of them divides K into groups; one more is
+    refused by every kernel before it launches, and the next call runs."""
+    k = _k()
+    N, K = 4, 1028                                                        # three groups of K
+    w = rand(N, K, seed=95).to(DEV)
+    for M in (1, 65):
+        a = rand(M, K, seed=96).to(DEV)
+        want = torch.empty(M, N, device=DEV)
+        k.gemm_generic(a, w, want)
+        for B in (21846, 65535):
+            out = torch.empty(B, M, N, device=DEV)
+            k.gemm_generic_batched(a.expand(B, M, K), w.expand(B, N, K), out)
+            assert bool((out == want).all()), (M, B)
+        with pytest.raises(k.KernelError, match="too large"):
+            k.gemm_generic_batched(a.expand(65536, M, K), w.expand(65536, N, K), torch.empty(65536, M, N, device=DEV))
+        k.gemm_generic(a, w, want)
+        assert torch.equal(want, out[7])
+
+
 @pytest.mark.parametrize("M", [1, 8, 33, 200])
 @pytest.mark.parametrize("batched", [False, True])
 def test_gemm_32bit_waits_for_a_computed_operand(M, batched):
