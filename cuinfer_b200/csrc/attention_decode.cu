@@ -115,6 +115,22 @@ inline bool cluster_combines(long long pairs, int splits, int g, int d, bool tma
     return splits > 1 && (one_round || (tma && splits <= 4)) && cluster_inbox_bytes(splits, g, d) <= 9 * 1024;
 }
 
+// The last `count` <= N splits of an output: one batch of loads whatever their number (those past the end read the last one
+// again and are left out).  The CTAs with keys are any number; batches of 4 and then single loads behind the full ones cost
+// a round trip each (two requests, 64 heads over 8, 15 of 16 CTAs with keys: 25 us against 15).
+template <int N>
+__device__ __forceinline__ float add_last_splits(float sum, const float* __restrict__ part, size_t stride, const float* weight, int count) {
+    float v[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) v[u] = __ldcg(part + (size_t)min(u, count - 1) * stride);
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const float more = fmaf(v[u], weight[min(u, count - 1)], sum);
+        sum = u < count ? more : sum;
+    }
+    return sum;
+}
+
 template <int D, bool TMA, bool CL>
 __global__ void __launch_bounds__(kDecWarps * 32)
 paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_bfloat16* __restrict__ out,
@@ -487,14 +503,8 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
 #pragma unroll
             for (int u = 0; u < 16; ++u) O = fmaf(v[u], sm_w[row * active + sp + u], O);
         }
-        for (; sp + 4 <= active; sp += 4) {
-            float v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = __ldcg(&part_o[((base + sp + u) * g + row) * D + dim]);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) O = fmaf(v[u], sm_w[row * active + sp + u], O);
-        }
-        for (; sp < active; ++sp) O = fmaf(__ldcg(&part_o[((base + sp) * g + row) * D + dim]), sm_w[row * active + sp], O);
+        if (active - sp > 4) O = add_last_splits<16>(O, part_o + ((base + sp) * g + row) * D + dim, (size_t)g * D, sm_w + row * active + sp, active - sp);
+        else if (active > sp) O = add_last_splits<4>(O, part_o + ((base + sp) * g + row) * D + dim, (size_t)g * D, sm_w + row * active + sp, active - sp);
         out[(size_t)r * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(O * sm_inv[row]);
     }
     if (threadIdx.x == 0) counters[r * nkv + kvh] = 0;

@@ -658,6 +658,21 @@ def test_attention_tcgen05_random_batches(seed):
         close(out, attention_reference(case, lens, new, scale, window), 1.5e-2)
 
 
+@pytest.mark.parametrize("nq, nkv, d", [(16, 8, 128), (16, 1, 128), (6, 3, 64), (8, 4, 256)])
+@pytest.mark.parametrize("splits, tma", [(16, False), (16, True), (37, False)])
+def test_paged_attention_decode_any_number_of_ctas_with_keys(nq, nkv, d, splits, tma):
+    """Partial results of one, some and all CTAs of a launch, merged through memory: every count up to the splits, with the
+    last CTA's share full, one key short and a single key."""
+    k = _k()
+    lens = [64 * n + extra for n in range(splits) for extra in (1, 63, 64)]
+    case = attention_case(torch.bfloat16, nq, nkv, d, lens, [1] * len(lens), 16, seed=97, sharp=True, poison=True)
+    out = torch.full((len(lens), nq * d), 5.0, dtype=torch.bfloat16, device=DEV)
+    k.paged_attention_decode(case["wide"].to(DEV), out, case["cache"].to(DEV), case["bt"].to(DEV),
+                             torch.tensor(lens, dtype=torch.int32, device=DEV), nq, nkv, d, 1.0 / math.sqrt(d), 0, splits, tma=tma)
+    k.check_error_flags()
+    close(out, attention_reference(case, lens, [1] * len(lens), 1.0 / math.sqrt(d)), 1.5e-2)
+
+
 @pytest.mark.parametrize("requests", [3, 45])
 @pytest.mark.parametrize("splits", [2, 4])
 def test_paged_attention_decode_cluster_and_memory_combine(requests, splits):
