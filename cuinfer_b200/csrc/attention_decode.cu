@@ -154,13 +154,24 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     const int quad = lane & 3, qrow = lane >> 2;
 
     const int seq_len = seq_lens[r];
+    // (while that load is on its way)
+    if (TMA) {
+        if (threadIdx.x == 0) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&kv_map) : "memory");
+            for (int i = 0; i < kDecWarps * kDecStages; ++i) mbar_init(&s_full[i], 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncthreads();
+    }
     const int pos = seq_len - 1;
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
     const int span = max(0, seq_len - lo);
-    int chunk = (span + splits - 1) / splits;
+    // (nothing else can start before a CTA knows its keys: no division here that the merge can make later)
+    int chunk = splits == 1 ? span : (span + splits - 1) / splits;
     chunk = max(kDecWarps * kDecKeys, (chunk + kDecKeys - 1) / kDecKeys * kDecKeys);       // a block for every warp at least
-    const int active = max(1, (span + chunk - 1) / chunk);        // CTAs with keys
-    if (split >= active) return;
+    if (split != 0 && split * chunk >= span) return;              // no keys for this CTA
+    const bool alone = chunk >= span;                             // all keys are the first CTA's
     const int k_begin = lo + split * chunk;
     const int k_end = min(seq_len, k_begin + chunk);
     const int* table = block_table + (size_t)r * table_stride;
@@ -179,15 +190,6 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     const int my_blocks = total_blocks > warp ? (total_blocks - warp + kDecWarps - 1) / kDecWarps : 0;
     auto block_key = [&](int i) { return k_begin + (i * kDecWarps + warp) * kDecKeys; };
 
-    if (TMA) {
-        if (threadIdx.x == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&kv_map) : "memory");
-            for (int i = 0; i < kDecWarps * kDecStages; ++i) mbar_init(&s_full[i], 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-        __syncthreads();
-    }
     // TMA path: lane 0 asks for the four boxes of a block (keys and values, two 64-column panels each for D = 128);
     // a block is 16 slots of one page (pages hold a multiple of 16 slots, blocks start at multiples of 16).  A page
     // number outside the pool becomes a row outside the tensor map: zeros, with the bytes still counted.
@@ -386,7 +388,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     // cluster path: the partials go to the first CTA's shared memory, [split][g][D] values then [split][g][2] maxima and sums
     float* inbox_o = nullptr;
     float* inbox_ml = nullptr;
-    if (CL && active > 1) {
+    if (CL && !alone) {
         namespace cg = cooperative_groups;
         float* inbox = reinterpret_cast<float*>(smem_raw + inbox_offset);
         if (split != 0) inbox = cg::this_cluster().map_shared_rank(inbox, 0);
@@ -409,7 +411,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
                 O += sm_o[((size_t)(w * g + row)) * D + dim] * f;
             }
         }
-        if (active == 1) {
+        if (alone) {
             out[(size_t)r * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
         } else if (CL) {
             inbox_o[row * D + dim] = O;
@@ -425,7 +427,10 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
             }
         }
     }
-    if (active == 1) return;
+    if (alone) return;
+    int active = splits;                                          // CTAs with keys
+    if (CL) while ((active - 1) * chunk >= span) --active;
+    else active = (span + chunk - 1) / chunk;
     if (CL) {
         // ---- the first CTA of the cluster combines what the others have written into its shared memory ----
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
