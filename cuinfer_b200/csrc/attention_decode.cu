@@ -625,6 +625,11 @@ extern "C" int cib_paged_attention_decode_supports(int head_dim, int nq, int nkv
     return (head_dim == 64 || head_dim == 128 || head_dim == 256) && nkv > 0 && nq % nkv == 0 && nq / nkv <= 16;
 }
 
+// Whether a launch merges its splits in clusters as far as its sizes decide that (the device's room for clusters decides the rest).
+extern "C" int cib_decode_merges_in_cluster(long long pairs, int splits, int group, int head_dim, int tma) {
+    return cluster_combines(pairs, splits, group, head_dim, tma != 0);
+}
+
 // Floats of scratch that `splits` splits need: part_o then part_ml, laid out one after the other.
 extern "C" long long cib_paged_attention_decode_scratch_floats(int num_requests, int nq, int head_dim, int splits) {
     return (long long)num_requests * nq * splits * (head_dim + 2);

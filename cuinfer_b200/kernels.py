@@ -123,6 +123,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cib_gemm_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
         "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
         "cib_gemm_generic": [_P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P],
+        "cib_decode_merges_in_cluster": [ctypes.c_longlong, _I, _I, _I, _I],
         "cib_sample": [_P, _I, _I, _I, _P, _P, _P],
         "cib_argmax_rows": [_P, _I, _I, _I, _P, _P],
         "cib_selftest_bounded_wait": [ctypes.c_longlong, _P, _P, _P],
@@ -605,17 +606,18 @@ def decode_slots(head_dim: int) -> int:
     return 148 * (1 if head_dim > 128 else 2 if head_dim > 64 else 3)
 
 
-def decode_merges_in_cluster(pairs: int, splits: int) -> bool:
-    """Whether the CTAs that share the keys of a (request, kv head) merge in a cluster, which costs little, on either path
-    of the kernel (``cluster_combines`` in attention_decode.cu; larger launches merge so on the TMA path only, which
-    the estimates below do not count on)."""
-    return splits <= 8 and pairs * splits <= 148
+def decode_merges_in_cluster(pairs: int, splits: int, group: int, head_dim: int, tma: bool = False) -> bool:
+    """Whether the CTAs that share the keys of a (request, kv head) merge in a cluster, which costs little: the rule of
+    ``cluster_combines`` in attention_decode.cu (``cib_decode_merges_in_cluster`` answers for the kernel).  Launches of more
+    CTAs than SMs merge so on the TMA path only, which the estimates below do not count on."""
+    one_round = splits <= 8 and pairs * splits <= 148
+    return splits > 1 and (one_round or (tma and splits <= 4)) and splits * group * (head_dim + 2) * 4 <= 9 * 1024
 
 
 def decode_splits(num_requests: int, num_kv_heads: int, max_seq_len: int, slots: int = 296, tma: bool = False,
-                  head_dim: int = 128) -> int:
+                  head_dim: int = 128, group: int = 1) -> int:
     """How many CTAs share the keys of one (request, kv head).  ``tma``: the cache layout allows the TMA path, which
-    a split then takes if it leaves a CTA ``DECODE_TMA_MIN_KEYS`` keys or more.
+    a split then takes if it leaves a CTA ``DECODE_TMA_MIN_KEYS`` keys or more.  ``group``: query heads per kv head.
 
     The GPU runs ``slots`` CTAs of this kernel at a time (two on each of the 148 SMs); a CTA's four warps take
     16-key blocks in turn, so a CTA's share counts in steps of 64 keys.  A launch is estimated, in nanoseconds, round
@@ -639,7 +641,7 @@ def decode_splits(num_requests: int, num_kv_heads: int, max_seq_len: int, slots:
         if rest:
             cost += keys * max(per_key, 0.072 * width * rest) + fixed
         if s > 1:
-            cost += 1200.0 if decode_merges_in_cluster(pairs, s) else 3000.0 + 40.0 * s
+            cost += 1200.0 if decode_merges_in_cluster(pairs, s, group, head_dim) else 3000.0 + 40.0 * s
         if best_cost is None or cost < best_cost:
             best, best_cost = s, cost
     return best

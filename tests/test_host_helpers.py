@@ -35,6 +35,23 @@ def test_decode_splits_is_sane_for_every_shape():
         assert counts == sorted(counts)
 
 
+def test_the_choice_of_splits_knows_which_launches_merge_in_clusters():
+    """The host's estimate and the kernel's launch take the same launches for clusters, whatever the group and head size; the
+    choice is the one that the merge really taken calls for."""
+    lib = kernels.library()
+    for pairs in (1, 2, 3, 8, 16, 18, 19, 24, 37, 49, 50, 74, 75, 148, 149, 500):
+        for splits in (1, 2, 3, 4, 5, 6, 7, 8, 9, 16):
+            for group in (1, 2, 3, 4, 6, 8, 16):
+                for head_dim in (64, 128, 256):
+                    for tma in (False, True):
+                        assert kernels.decode_merges_in_cluster(pairs, splits, group, head_dim, tma) == bool(
+                            lib.cib_decode_merges_in_cluster(pairs, splits, group, head_dim, int(tma))), (pairs, splits, group, head_dim, tma)
+    # groups of two heads of 128 meet in clusters of eight; the partials of groups of four and more do not fit, and the merge
+    # through memory that they then take asks for more and shorter shares
+    assert kernels.decode_splits(2, 8, 2048, group=2) == 8 and kernels.decode_splits(2, 8, 2048, group=4) == 16
+    assert kernels.decode_splits(1, 8, 512, group=4) == 4 and kernels.decode_splits(1, 8, 1500, group=4) == 24
+
+
 def test_uniform_numbers_depend_on_seed_request_and_index_only():
     seen = set()
     for seed in (0, 1, 12345):
