@@ -170,8 +170,12 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     // (nothing else can start before a CTA knows its keys: no division here that the merge can make later)
     int chunk = splits == 1 ? span : (span + splits - 1) / splits;
     chunk = max(kDecWarps * kDecKeys, (chunk + kDecKeys - 1) / kDecKeys * kDecKeys);       // a block for every warp at least
-    if (split != 0 && split * chunk >= span) return;              // no keys for this CTA
-    const bool alone = chunk >= span;                             // all keys are the first CTA's
+    // Clusters on the TMA path are launched for streams of a thousand keys a CTA, and their merge costs little: there a CTA
+    // without keys sends an empty partial, and the loops of the merge run over a number that the launch knows (over a
+    // computed one 8 requests of 2 049 keys took 13.4 us instead of 13.0, 16 of 200 6.05 instead of 5.85).
+    constexpr bool kLeave = !(CL && TMA);
+    if (kLeave && split != 0 && split * chunk >= span) return;    // no keys for this CTA
+    const bool alone = kLeave ? chunk >= span : splits == 1;      // all keys are the first CTA's
     const int k_begin = lo + split * chunk;
     const int k_end = min(seq_len, k_begin + chunk);
     const int* table = block_table + (size_t)r * table_stride;
@@ -428,9 +432,9 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         }
     }
     if (alone) return;
-    int active = splits;                                          // CTAs with keys
-    if (CL) while ((active - 1) * chunk >= span) --active;
-    else active = (span + chunk - 1) / chunk;
+    int active = splits;                                          // CTAs that have sent a partial
+    if (CL && kLeave) while ((active - 1) * chunk >= span) --active;
+    else if (!CL) active = (span + chunk - 1) / chunk;
     if (CL) {
         // ---- the first CTA of the cluster combines what the others have written into its shared memory ----
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
