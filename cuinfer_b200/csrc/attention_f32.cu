@@ -73,7 +73,7 @@ attention_f32_few_kernel(const AttnF32 p, int splits) {
             if (page >= 0 && page < p.num_pages) row = (long long)(page * page_stride + (size_t)(j % p.page_size) * D);
         }
         float4 k[2][Q4];
-        float v[kFewAttnKeys][VD];
+        __align__(16) float v[kFewAttnKeys][VD];
         bool in[2];
 #pragma unroll
         for (int step = 0; step < 2; ++step) {
@@ -319,7 +319,7 @@ attention_f32_tile_kernel(const AttnF32 p) {
                     for (int k = 0; k < kWarpRows; ++k) w4[k] = *reinterpret_cast<const float4*>(&s.p[warp * kWarpRows + k][j4]);
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        float v[VD];
+                        __align__(16) float v[VD];
                         const float* vp = &s.v[buffer][j4 + u][lane * VD];
                         if (VD == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(vp);
                         else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(vp);

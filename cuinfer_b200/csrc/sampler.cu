@@ -130,7 +130,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int s
                       int* __restrict__ out_ids) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ float s_row[];
+    extern __shared__ __align__(16) float s_row[];
     __shared__ SampleShared s;
     const int row = blockIdx.x / kSampleCtas, rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
