@@ -8,7 +8,7 @@ namespace cib {
 struct AttnF32 {
     const float* q; float* out; const float* cache; const int* block_table; const int* query_start_loc; const int* seq_lens;
     const int* token_request;
-    int q_stride, out_stride, num_pages, page_size, table_stride, num_tokens, nq, nkv, window;
+    int q_stride, out_stride, num_pages, page_size, table_stride, num_tokens, num_requests, nq, nkv, window;
     float scale;
 };
 

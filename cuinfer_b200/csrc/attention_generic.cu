@@ -100,21 +100,23 @@ __global__ void paged_attention_generic_kernel(
 
 using namespace cib;
 
+// query_start_loc holds num_requests + 1 boundaries of the num_tokens rows; token_request names the same requests row by row.
 extern "C" int cib_paged_attention_generic(const void* q, int dtype, int q_stride, void* out, int out_stride,
                                            const void* cache, int num_pages, int page_size,
                                            const int* block_table, int table_stride,
                                            const int* query_start_loc, const int* seq_lens,
-                                           const int* token_request, int num_tokens, int nq, int nkv, int d,
+                                           const int* token_request, int num_tokens, int num_requests, int nq, int nkv, int d,
                                            float scale, int window, cudaStream_t stream) {
     CIB_REQUIRE(num_tokens >= 0 && nq > 0 && nkv > 0 && d > 0 && nq % nkv == 0,
                 "paged_attention: bad sizes T=%d nq=%d nkv=%d d=%d", num_tokens, nq, nkv, d);
+    CIB_REQUIRE(num_requests > 0 || num_tokens == 0, "paged_attention: tokens without requests");
     CIB_REQUIRE(d <= kMaxHeadDim, "paged_attention: head_dim %d exceeds %d", d, kMaxHeadDim);
     CIB_REQUIRE(page_size > 0 && num_pages > 0 && table_stride > 0, "paged_attention: bad cache geometry");
     CIB_REQUIRE(window >= 0, "paged_attention: window must be >= 0 (0 = all keys)");
     if (num_tokens == 0) return 0;
     if (dtype == kF32) {
         const AttnF32 p{(const float*)q, (float*)out, (const float*)cache, block_table, query_start_loc, seq_lens, token_request,
-                        q_stride, out_stride, num_pages, page_size, table_stride, num_tokens, nq, nkv, window, scale};
+                        q_stride, out_stride, num_pages, page_size, table_stride, num_tokens, num_requests, nq, nkv, window, scale};
         if (const int rc = attention_f32_try(p, d, stream)) return rc > 0 ? 0 : rc;
     }
     dim3 grid(num_tokens, (nq + kAttnWarps - 1) / kAttnWarps);

@@ -548,6 +548,31 @@ def test_paged_attention_32bit(nq, nkv, d, ps, window, decode):
     assert torch.equal(out2[others], out[others])
 
 
+@pytest.mark.parametrize("nq, nkv, d", [(8, 8, 64), (16, 8, 128), (12, 3, 64)])
+@pytest.mark.parametrize("portion", [None, 70])
+def test_paged_attention_32bit_many_requests(nq, nkv, d, portion):
+    """Decoded tokens of more requests than the few-tokens kernel would take by its CTAs, alone and beside a prompt, with
+    requests that bring nothing in between and at the end (as a recorded step pads)."""
+    k = _k()
+    lens, new = [], []
+    for r in range(70):
+        lens.append(1 + r * 37 % 190)
+        new.append(0 if r in (0, 31, 32, 50) else 1)
+    if portion:
+        lens[40], new[40] = portion + 20, portion
+    live = [r for r in range(70) if new[r]]
+    case = attention_case(torch.float32, nq, nkv, d, [lens[r] for r in live], [new[r] for r in live], 16, seed=27, sharp=True, poison=True)
+    scale, T = 0.7 / math.sqrt(d), sum(new)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    bt = torch.full((90, case["bt"].shape[1]), -1, dtype=torch.int32)
+    bt[live] = case["bt"]
+    qsl = [sum(new[:r]) for r in range(71)] + [T] * 20
+    out = torch.full((T, nq * d), 5.0, device=DEV)
+    k.paged_attention_generic(case["wide"].to(DEV), out, case["cache"].to(DEV), bt.to(DEV), i32(qsl), i32(lens + [0] * 20),
+                              i32([r for r in range(70) for _ in range(new[r])]), nq, nkv, d, scale, 0)
+    close(out, attention_reference(case, [lens[r] for r in live], [new[r] for r in live], scale), 2e-5)
+
+
 @pytest.mark.parametrize("nq, nkv, d, ps", [(16, 8, 128, 16), (8, 1, 64, 32), (12, 3, 128, 5), (32, 2, 256, 16),
                                             (4, 4, 64, 16)])
 @pytest.mark.parametrize("splits", [1, 3, 8])
