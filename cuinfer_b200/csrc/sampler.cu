@@ -1,4 +1,4 @@
-// Next-token sampling from 32-bit logits: greedy, temperature, top-k, top-p.  A cluster of eight CTAs per row.
+// Next-token sampling from 32-bit logits: greedy, temperature, top-k, top-p.  A cluster of up to eight CTAs per row.
 //
 // Meaning of the options follows the reference's sampler (csrc/ops/sampler.cu:134-387):
 //   temperature == 0   -> argmax, ties to the lowest id (:207-212)
@@ -18,7 +18,7 @@
 
 namespace cib {
 
-// A cluster of eight CTAs takes a row, an eighth of the vocabulary each, kept in shared memory: the logits are read from
+// A cluster of up to eight CTAs takes a row, a share of the vocabulary each, kept in shared memory: the logits are read from
 // device memory once, the exponentials are taken once, and every level of a descent walks shared memory.  What bounds it
 // is the chain of levels (a histogram of the share, a cluster barrier, a scan of 256 sums), not the bytes.  Two things keep
 // the histograms from serialising on one bin: the lowest digit's sum is never needed (it is what is left when no other digit
@@ -28,10 +28,22 @@ namespace cib {
 // Rows of 151 936 tokens, microseconds with the L2 flushed, against one CTA a row with 64-bit sums of every digit: 32 rows
 // with top_p 0.9 55 (10 749), 1 row 39 (10 699), 128 rows 184 (10 770); 32 rows with top_k 50 59 (1 912), with neither 29
 // (141); 32 rows of 400 000 tokens, which shared memory does not hold, 363 (5 273).
-constexpr int kSampleCtas = 8;
+constexpr int kSampleCtas = 8;                  // at most
 constexpr int kSampleThreads = 512;
 constexpr int kSampleWarps = kSampleThreads / 32;
 constexpr int kSampleShareMax = 49152;          // tokens of a share that shared memory holds (192 KB); longer ones are re-read
+constexpr int kSampleShareFour = 12800;         // tokens of a share with which four CTAs fit an SM, all its threads
+
+// CTAs of a row: as few as leave an SM four of them, since every CTA of a large batch costs its start and its part of every
+// barrier; more, down to 512 tokens each, while the whole batch still has at most two for each SM.  (With eight at every
+// size 512 rows of 128 tokens took 29 us greedily and 193 with top_p, one CTA each 5 and 15; 128 rows of 8 192 with
+// top_p 58, now 20.)
+inline int sample_ctas(int rows, int vocab) {
+    int ctas = 1;
+    while (ctas < kSampleCtas && vocab > ctas * kSampleShareFour) ctas *= 2;
+    while (ctas < kSampleCtas && (long long)rows * ctas * 2 <= 2 * 148 && vocab >= 2 * ctas * 512) ctas *= 2;
+    return ctas;
+}
 
 struct SampleParams {
     float temperature;
@@ -78,24 +90,31 @@ struct SampleShared {
     u64 above;
 };
 
+template <int CTAS>
 __device__ __forceinline__ void cluster_barrier() {
+    if (CTAS == 1) { __syncthreads(); return; }
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// `p`, a place in this CTA's shared memory, in that of CTA `rank` of the row.
+template <int CTAS, typename T>
+__device__ __forceinline__ T* of_rank(T* p, int rank) {
+    return CTAS == 1 ? p : cooperative_groups::this_cluster().map_shared_rank(p, rank);
 }
 
 // One level of a descent: the sums of this CTA's histogram and its peers' are joined by every CTA for itself, and the highest
 // digit d is found with above + sum of the digits >= d reaching `need` (0 if none does).  `above` becomes the sum of the
 // digits above it.  kWide: the two words of the histogram are one 64-bit sum.
-template <bool kWide>
+template <int CTAS, bool kWide>
 __device__ __forceinline__ unsigned int descend(SampleShared& s, int parity, u64 need, u64& above) {
-    namespace cg = cooperative_groups;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    cluster_barrier();                                           // every CTA's histogram is complete
+    cluster_barrier<CTAS>();                                     // every CTA's histogram is complete
     u64 suffix = 0ull;
     if (tid < 256) {
         u64 v = 0ull;
 #pragma unroll
-        for (int r = 0; r < kSampleCtas; ++r) {
-            const unsigned int* h = cg::this_cluster().map_shared_rank(&s.hist[parity][0][0], r);
+        for (int r = 0; r < CTAS; ++r) {
+            const unsigned int* h = of_rank<CTAS>(&s.hist[parity][0][0], r);
             v += kWide ? reinterpret_cast<const u64*>(h)[tid] : (u64)h[tid] + ((u64)h[256 + tid] << 16);
         }
         suffix = v;                                              // sum over the digits >= tid of this warp
@@ -124,17 +143,15 @@ __device__ __forceinline__ unsigned int descend(SampleShared& s, int parity, u64
 
 // kCached: the share lies in shared memory (logits first, masses in their place later); else the row is re-read and the
 // masses are taken again at every level.
-template <bool kCached>
+template <int CTAS, bool kCached>
 __global__ void __launch_bounds__(kSampleThreads)
 sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int share, const SampleParams* __restrict__ params,
                       int* __restrict__ out_ids) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) float s_row[];
     __shared__ SampleShared s;
-    const int row = blockIdx.x / kSampleCtas, rank = (int)cluster.block_rank();
+    const int row = blockIdx.x / CTAS, rank = blockIdx.x % CTAS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // remote stores come after every CTA runs
+    if (CTAS > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // remote stores come after every CTA runs
     const float* x = logits + (size_t)row * ld;
     const int begin = min(vocab, rank * share), end = min(vocab, begin + share), count = end - begin;
     const SampleParams p = params[row];
@@ -169,23 +186,23 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int s
         take_better(best, best_i, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, best_i, o));
     if (lane == 0) { s.warp_best[warp] = best; s.warp_best_i[warp] = best_i; }
     for (int i = tid; i < 2 * 2 * 256; i += kSampleThreads) (&s.hist[0][0][0])[i] = 0u;
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (CTAS > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         best = lane < kSampleWarps ? s.warp_best[lane] : -INFINITY;
         best_i = lane < kSampleWarps ? s.warp_best_i[lane] : 0x7fffffff;
         for (int o = 16; o > 0; o >>= 1)
             take_better(best, best_i, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, best_i, o));
-        if (lane < kSampleCtas) {
-            *cluster.map_shared_rank(&s.best[rank], lane) = best;
-            *cluster.map_shared_rank(&s.best_i[rank], lane) = best_i;
+        if (lane < CTAS) {
+            *of_rank<CTAS>(&s.best[rank], lane) = best;
+            *of_rank<CTAS>(&s.best_i[rank], lane) = best_i;
         }
     }
-    cluster_barrier();
+    cluster_barrier<CTAS>();
     best = s.best[0];
     best_i = s.best_i[0];
 #pragma unroll
-    for (int r = 1; r < kSampleCtas; ++r) take_better(best, best_i, s.best[r], s.best_i[r]);
+    for (int r = 1; r < CTAS; ++r) take_better(best, best_i, s.best[r], s.best_i[r]);
     const float mx = best;
     const int argmax = best_i == 0x7fffffff ? 0 : best_i;
     if (!(p.temperature > 0.f) || p.top_k == 1) {                // the same for every CTA of the row; no peer reads this one's memory any more
@@ -216,7 +233,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int s
                     else atomicAdd(reinterpret_cast<u64*>(hist) + digit, (u64)__popc(same));
                 }
             }
-            const uint32_t digit = descend<!kCached>(s, level & 1, (u64)p.top_k, above);
+            const uint32_t digit = descend<CTAS, !kCached>(s, level & 1, (u64)p.top_k, above);
             prefix |= digit << shift;
             mask |= 0xffu << shift;
             // the other parity's histogram was read before the barrier that this level has passed
@@ -244,12 +261,12 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int s
         __syncthreads();
         if (warp == 0) {
             part = warp_sum_u64(lane < kSampleWarps ? s.warp_part[lane] : 0ull);
-            if (lane < kSampleCtas) *cluster.map_shared_rank(&s.total[rank], lane) = part;
+            if (lane < CTAS) *of_rank<CTAS>(&s.total[rank], lane) = part;
         }
-        cluster_barrier();
+        cluster_barrier<CTAS>();
         u64 total = 0ull;
 #pragma unroll
-        for (int r = 0; r < kSampleCtas; ++r) total += s.total[r];
+        for (int r = 0; r < CTAS; ++r) total += s.total[r];
         const double want = (double)p.top_p * (double)total;
         u64 need = (u64)want;
         if ((double)need < want) ++need;
@@ -278,7 +295,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int s
                     atomicAdd(&hist[256 + digit], q >> 16);
                 }
             }
-            const uint32_t digit = descend<!kCached>(s, level & 1, need, above);
+            const uint32_t digit = descend<CTAS, !kCached>(s, level & 1, need, above);
             prefix |= digit << shift;
             mask |= 0xffu << shift;
             for (int i = tid; i < 512; i += kSampleThreads) (&s.hist[(level + 1) & 1][0][0])[i] = 0u;
@@ -302,12 +319,12 @@ sample_cluster_kernel(const float* __restrict__ logits, int ld, int vocab, int s
     __syncthreads();
     if (warp == 0) {
         const u64 all = warp_sum_u64(lane < kSampleWarps ? s.warp_part[lane] : 0ull);
-        if (lane < kSampleCtas) *cluster.map_shared_rank(&s.kept[rank], lane) = all;
+        if (lane < CTAS) *of_rank<CTAS>(&s.kept[rank], lane) = all;
     }
-    cluster_barrier();                                           // the last access to a peer's memory lies before it
+    cluster_barrier<CTAS>();                                           // the last access to a peer's memory lies before it
     u64 kept = 0ull, run = 0ull;
 #pragma unroll
-    for (int r = 0; r < kSampleCtas; ++r) {
+    for (int r = 0; r < CTAS; ++r) {
         if (r < rank) run += s.kept[r];
         kept += s.kept[r];
     }
@@ -434,27 +451,33 @@ extern "C" int cib_sample(const float* logits, int ld, int rows, int vocab, cons
                           cudaStream_t stream) {
     CIB_REQUIRE(rows >= 0 && vocab > 0 && ld >= vocab, "sample: bad sizes rows=%d V=%d ld=%d", rows, vocab, ld);
     if (rows == 0) return 0;
-    const int share = ((vocab + kSampleCtas - 1) / kSampleCtas + 3) & ~3;
+    const int ctas = sample_ctas(rows, vocab), share = ((vocab + ctas - 1) / ctas + 3) & ~3;
     const bool cached = share <= kSampleShareMax;
-    static SmemLimit limit;
-    if (cached && raise_smem_limit(limit, sample_cluster_kernel<true>, kSampleShareMax * sizeof(float), "sample") != 0) return -2;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(rows * kSampleCtas);
+    cfg.gridDim = dim3(rows * ctas);
     cfg.blockDim = dim3(kSampleThreads);
     cfg.dynamicSmemBytes = cached ? share * sizeof(float) : 0;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kSampleCtas;
+    attr[0].val.clusterDim.x = ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, cached ? sample_cluster_kernel<true> : sample_cluster_kernel<false>, logits, ld, vocab,
-                                             share, (const SampleParams*)params, out_ids);
-    if (e != cudaSuccess) {
+    cfg.numAttrs = ctas > 1 ? 1 : 0;
+    static SmemLimit limits[4];
+    const auto launch = [&](auto kernel, SmemLimit& limit) -> int {
+        if (cached && raise_smem_limit(limit, kernel, kSampleShareMax * sizeof(float), "sample") != 0) return -2;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, logits, ld, vocab, share, (const SampleParams*)params, out_ids);
+        if (e == cudaSuccess) return 0;
         set_error("sample: launch failed: %s", cudaGetErrorString(e));
         return -2;
+    };
+    if (!cached) return launch(sample_cluster_kernel<kSampleCtas, false>, limits[0]);      // such a row has eight
+    switch (ctas) {
+        case 1: return launch(sample_cluster_kernel<1, true>, limits[0]);
+        case 2: return launch(sample_cluster_kernel<2, true>, limits[1]);
+        case 4: return launch(sample_cluster_kernel<4, true>, limits[2]);
+        default: return launch(sample_cluster_kernel<8, true>, limits[3]);
     }
-    return 0;
 }
