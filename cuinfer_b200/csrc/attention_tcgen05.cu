@@ -485,16 +485,19 @@ extern "C" int cib_attention_tcgen05_supports(int head_dim, int nq, int nkv, int
     return 128 % g == 0 && page_size >= 8 && (page_size & (page_size - 1)) == 0;
 }
 
-// num_tiles = sum over requests of ceil(tokens_r * (nq / nkv) / 128).  error_flag: one zero int in device memory.
+// num_tiles = sum over requests of ceil(tokens_r * (nq / nkv) / 128), or more: CTAs that find no tile leave.  least_tiles: how many
+// of them the step has at least, which decides between the two variants (a recorded step is launched for the worst split of
+// its tokens over its requests).  error_flag: one zero int in device memory.
 extern "C" int cib_attention_tcgen05(const void* q, int q_stride, void* out, int out_stride, const void* cache, int num_pages,
                                      int page_size, const int* block_table, int table_stride, const int* query_start_loc,
-                                     const int* seq_lens, int num_requests, int num_tiles, int nq, int nkv, int head_dim,
-                                     float scale, int window, int joined, const float* sinks, int* error_flag,
+                                     const int* seq_lens, int num_requests, int num_tiles, int least_tiles, int nq, int nkv,
+                                     int head_dim, float scale, int window, int joined, const float* sinks, int* error_flag,
                                      cudaStream_t stream) {
     CIB_REQUIRE(cib_attention_tcgen05_supports(head_dim, nq, nkv, page_size),
                 "attention_tcgen05: head_dim %d, %d/%d heads, page size %d are not taken (head size 128, heads per kv head dividing 128, pages of 8, 16, 32, ... slots)",
                 head_dim, nq, nkv, page_size);
-    CIB_REQUIRE(num_requests >= 0 && num_tiles >= 0 && num_tiles <= 65535 && num_pages > 0 && table_stride > 0, "attention_tcgen05: bad sizes");
+    CIB_REQUIRE(num_requests >= 0 && num_tiles >= 0 && num_tiles <= 65535 && least_tiles <= num_tiles && num_pages > 0 && table_stride > 0,
+                "attention_tcgen05: bad sizes");
     CIB_REQUIRE(q_stride % 8 == 0 && ((uintptr_t)q % 16) == 0 && out_stride % 8 == 0 && ((uintptr_t)out % 16) == 0 && ((uintptr_t)cache % 16) == 0,
                 "attention_tcgen05: rows must be 16-byte aligned");
     CIB_REQUIRE(error_flag != nullptr, "attention_tcgen05: error flag missing");
@@ -504,7 +507,7 @@ extern "C" int cib_attention_tcgen05(const void* q, int q_stride, void* out, int
     const long long total_rows = (long long)num_pages * (joined ? 1 : 2) * nkv * page_size;
     CIB_REQUIRE(total_rows < (1ll << 31), "attention_tcgen05: %lld cache rows do not fit a 32-bit coordinate", total_rows);
     // few CTAs: the variant that has an SM alone (attention_tcgen05_wide.cu says why the line lies here)
-    const bool wide = (long long)nkv * num_tiles <= 3 * 148;
+    const bool wide = (long long)nkv * least_tiles <= 3 * 148;
     const int tile_keys = wide ? kWideKeys : fa::kN;
     CUtensorMap kv_map;
     const int row_values = joined ? 2 * fa::kD : fa::kD;

@@ -375,6 +375,11 @@ class ModelRunner:
         Rb = 1 << R.bit_length()
         return -(-T // step) * step, Rb, (max(Rb, 1 << (S - 1).bit_length())) if S else 0
 
+    @staticmethod
+    def step_bucket_least(T: int, R: int) -> Tuple[int, int]:
+        """The fewest (tokens, requests) of a batch whose ``step_bucket`` has ``T`` tokens and ``R`` requests."""
+        return T - max(16, 1 << max(0, (T - 1).bit_length() - 4)) + 1, R // 2
+
     def _step_graph(self, entries: Sequence[StepEntry]) -> Optional["StepGraph"]:
         if not self.config.enable_cuda_graph or len(entries) > self.STEP_GRAPH_MAX_ENTRIES or not self.model.capturable:
             return None
@@ -740,6 +745,7 @@ class StepGraph:
         ctx.seq_lens_host = None
         ctx.state_slots_host = None
         ctx.launch_query_lens = [T + 128] + [1] * (R - 1)
+        ctx.launch_least = runner.step_bucket_least(T, R)
         ctx.max_query_len = T
         ctx.max_seq_len = runner.max_model_len
         if self.graph is not None:

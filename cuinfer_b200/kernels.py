@@ -978,11 +978,13 @@ def attention_tcgen05_supports(head_dim: int, num_q_heads: int, num_kv_heads: in
 def attention_tcgen05(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
                       query_start_loc: torch.Tensor, seq_lens: torch.Tensor, query_lens_host, num_q_heads: int,
                       num_kv_heads: int, head_dim: int, scale: float, window: int = 0, *, joined: bool = False,
-                      sinks: torch.Tensor | None = None) -> None:
+                      sinks: torch.Tensor | None = None, least_tiles: int | None = None) -> None:
     """bfloat16 attention for prompt portions on tcgen05 tensor cores (head size 128, pages of 8, 16, 32, ...
     slots): scores and output accumulate in tensor memory, keys and values come page by page through TMA.
     ``cache`` is ``[pages, 2, kv heads, page, 128]`` (keys, values) or, with ``joined``, ``[pages, 1, kv heads, page, 256]``
-    with a token's key and value side by side; ``sinks`` float32 [query heads]: ``exp(sink)`` joins a row's denominator."""
+    with a token's key and value side by side; ``sinks`` float32 [query heads]: ``exp(sink)`` joins a row's denominator.
+    ``query_lens_host`` may be an upper bound; ``least_tiles`` then says how many tiles of 128 rows the step has at least
+    (``StepContext.least_row_tiles``), by which the kernel's variant is chosen."""
     T = q.shape[0]
     planes, row = (1, 2 * head_dim) if joined else (2, head_dim)
     if cache.dim() != 5 or cache.shape[1] != planes or cache.shape[2] != num_kv_heads or cache.shape[4] != row:
@@ -999,7 +1001,8 @@ def attention_tcgen05(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, b
         _cuda(q, "q", contiguous=False), q.stride(0), _cuda(out, "out", contiguous=False), out.stride(0),
         _cuda(cache, "cache"), cache.shape[0], cache.shape[3], _cuda(block_table, "block_table", torch.int32),
         block_table.stride(0), _cuda(query_start_loc, "query_start_loc", torch.int32),
-        _cuda(seq_lens, "seq_lens", torch.int32), len(query_lens_host), tiles, num_q_heads, num_kv_heads, head_dim,
+        _cuda(seq_lens, "seq_lens", torch.int32), len(query_lens_host), tiles,
+        tiles if least_tiles is None else min(least_tiles, tiles), num_q_heads, num_kv_heads, head_dim,
         float(scale), int(window), 1 if joined else 0, _cuda(sinks, "sinks") if sinks is not None else None,
         _error_flag(q.device).data_ptr(), _stream())
     _check(rc, "attention_tcgen05")

@@ -39,7 +39,8 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: PagedKV, ctx: Step
             head_dim, num_heads, num_kv_heads, kv.group.page_size) and out.stride(0) % 8 == 0 and qkv.stride(0) % 8 == 0:
         lens = ctx.query_lens_for_launch()
         kernels.attention_tcgen05(qkv, out, kv.cache, kv.group.block_table, ctx.query_start_loc, ctx.seq_lens, lens,
-                                  num_heads, num_kv_heads, head_dim, scale, window)
+                                  num_heads, num_kv_heads, head_dim, scale, window,
+                                  least_tiles=ctx.least_row_tiles(num_heads // num_kv_heads, 128))
         return
     if qkv.dtype == torch.bfloat16 and kernels.paged_attention_prefill_supports(head_dim, num_heads, num_kv_heads):
         lens = ctx.query_lens_for_launch()
@@ -124,7 +125,8 @@ def window_attention(q: torch.Tensor, out: torch.Tensor, kv: PagedKV, ctx: StepC
             and kernels.attention_tcgen05_supports(dim, num_heads, num_kv_heads, kv.group.page_size)
             and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0 and (sinks is None or sinks.dtype == torch.float32)):
         kernels.attention_tcgen05(q, out, kv.cache, kv.group.block_table, ctx.query_start_loc, ctx.seq_lens,
-                                  ctx.query_lens_for_launch(), num_heads, num_kv_heads, dim, scale, window, joined=True, sinks=sinks)
+                                  ctx.query_lens_for_launch(), num_heads, num_kv_heads, dim, scale, window, joined=True, sinks=sinks,
+                                  least_tiles=ctx.least_row_tiles(num_heads // num_kv_heads, 128))
         return
     if (q.dtype == torch.bfloat16 and not _FORCE_GENERIC_WINDOW and q.stride(0) % 8 == 0
             and kernels.window_attention_mma_supports(dim, vdim, num_heads, num_kv_heads)):

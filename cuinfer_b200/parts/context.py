@@ -9,7 +9,7 @@ state slot of every request, and the per-run cache tensors.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import Dict, List, Optional
+from typing import Dict, List, Optional, Tuple
 
 import torch
 
@@ -54,6 +54,7 @@ class StepContext:
     seq_lens_host: Optional[List[int]] = field(default_factory=list)
     state_slots_host: Optional[List[int]] = field(default_factory=list)
     launch_query_lens: Optional[List[int]] = None      # set for a captured step: see query_lens_for_launch
+    launch_least: Optional[Tuple[int, int]] = None     # the fewest (tokens, requests) of a captured step's batches
     max_query_len: int = 0
     max_seq_len: int = 0
     groups: Dict[int, GroupView] = field(default_factory=dict)
@@ -74,6 +75,14 @@ class StepContext:
             return self.launch_query_lens
         starts = self.query_start_loc_host
         return [starts[i + 1] - starts[i] for i in range(self.num_requests)]
+
+    def least_row_tiles(self, rows_per_token: int, tile_rows: int) -> Optional[int]:
+        """How many row tiles, none of which holds two requests, the step has at least: for choices between kernels that
+        depend on how many CTAs find work.  None where ``query_lens_for_launch`` is exact."""
+        if self.launch_query_lens is None or self.launch_least is None:
+            return None
+        tokens, requests = self.launch_least
+        return max(requests, -(-tokens * rows_per_token // tile_rows))
 
     def paged_kv(self, run: int) -> PagedKV:
         try:

@@ -77,6 +77,7 @@ def test_step_buckets_hold_their_batches_with_little_to_spare():
     """The sizes a step is padded to before it runs as a captured graph: never smaller than the batch, one request to
     spare for the spare tokens, at most an eighth (or 15) more tokens, and few distinct buckets."""
     from cuinfer_b200.engine.runner import ModelRunner
+    from cuinfer_b200.parts.context import StepContext
 
     rnd = random.Random(1)
     seen = set()
@@ -90,5 +91,13 @@ def test_step_buckets_hold_their_batches_with_little_to_spare():
         assert R < Rb <= 2 * R and Rb & (Rb - 1) == 0
         assert S <= Sb <= max(2 * S - 1, Rb if S else 0) and Sb & (Sb - 1) == 0
         seen.add(Tb)
+        # what a recorded step's launches are sized by: at most so many row tiles, and at least so many, in every batch
+        least_tokens, least_requests = ModelRunner.step_bucket_least(Tb, Rb)
+        assert least_tokens <= T and least_requests <= R
+        ctx = StepContext.__new__(StepContext)
+        ctx.launch_query_lens, ctx.launch_least = [Tb + 128] + [1] * (Rb - 1), (least_tokens, least_requests)
+        for g in (1, 2, 3, 4, 8, 16):
+            tiles = sum(-(-n * g // 128) for n in lens)
+            assert ctx.least_row_tiles(g, 128) <= tiles <= sum(-(-n * g // 128) for n in ctx.query_lens_for_launch())
     assert len(seen) < 120
     assert ModelRunner.step_bucket([2048], [1]) == (2048, 2, 2) and ModelRunner.step_bucket([8192], [1])[0] == 8192
