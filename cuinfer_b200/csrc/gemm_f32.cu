@@ -318,8 +318,15 @@ gemm_f32_tile_kernel(const GemmF32 p) {
     cluster.sync();                                             // a CTA's shared memory stays until the others have read it
 }
 
-// Rows up to which the few-rows kernel is taken: every pass of eight rows costs it about 6 us of reads of shared memory
-// (4096 x 1024: 10 us at 8 rows, 25 at 32), a tile of up to 64 rows takes the tile kernel 56 to 80.
+// Rows up to which the few-rows kernel may be taken, where K fits one round of its warps.  Up to one pass of eight it always
+// is; beyond, the three kernels' times are estimated (microseconds, fitted to 9 to 2 048 rows x 64 to 151 936 x 64 to 8 192
+// within 30 %) and the smallest wins:
+//   few rows: 2.5, and a pass of eight rows 1.5 and 0.57 for every warp that an SM has of it
+//   tiles: 0.08 per value of a CTA's K for each CTA that an SM has, alone on it 0.096 (0.135 where every SM has one)
+//   tiles and all sizes: 3 more
+//   all sizes: 0.0535 per value of K for each CTA that an SM has, at least 0.075
+// (64 x 151 936 x 1 024: 1 116, 716 and 972; 64 x 4 096 x 1 024: 46, 53 and 79; 64 x 64 x 64: 18, 8.8 and 7.8; 128 x 2 048 x
+// 512, K a single group of which no cluster can share the work: tiles 51, all sizes 41.)
 constexpr int kFewMaxRows = 64;
 
 bool gemm_f32_takes(const GemmF32& p, int batch) {
@@ -345,10 +352,30 @@ constexpr int kFewMaxK = 5 * kFewMaxWarps * kFewChunk;
 static_assert(kFewMaxWarps * (kFewFeatures * kFewWRow + kFewRows * kFewARow) + 5 * kFewMaxWarps * 4 * kFewRows * kFewFeatures * 4 <= 227 * 1024,
               "shared memory of the largest few-rows launch");
 
+static long long per_sm(long long ctas) { return (ctas + 147) / 148; }
+
 int gemm_f32_launch(const GemmF32& p, int batch, cudaStream_t stream) {
     CIB_REQUIRE((p.M + kTileM - 1) / kTileM <= 65535 && batch <= 65535, "gemm: M=%d or batch=%d too large for this kernel", p.M, batch);
-    const bool one_round = p.K <= kFewChunk * kFewMaxWarps;
-    if (p.K <= kFewMaxK && (p.M <= kFewRows || (p.M <= kFewMaxRows && one_round))) {
+    const int groups = f32_groups(p.K);
+    const dim3 grid((p.N + kTileN - 1) / kTileN, (p.M + kTileM - 1) / kTileM, batch);
+    // rounds of resident CTAs, in groups of K: a tile whole, or its groups apart where that fills the last round better (and
+    // the launch's z extent holds them)
+    const long long tiles = (long long)grid.x * grid.y * batch;
+    const bool split = groups > 1 && (long long)batch * groups <= 65535 && (tiles * groups + kTileCtas - 1) / kTileCtas < (tiles + kTileCtas - 1) / kTileCtas * groups;
+
+    bool few = p.K <= kFewMaxK && p.M <= kFewRows;
+    if (!few) {
+        const long long tile_ctas = tiles * (split ? groups : 1);
+        const float tile_k = split ? (float)(f32_group_slices(p.K) * kF32Slice) : (float)p.K;
+        const float t_tile = 3.f + tile_k * (tile_ctas <= 74 ? 0.096f : tile_ctas <= 148 ? 0.135f : 0.08f * per_sm(tile_ctas));
+        const long long all_ctas = (long long)((p.N + 63) / 64) * ((p.M + 63) / 64) * batch;
+        const float t_all = 3.f + p.K * fmaxf(0.075f, 0.0535f * per_sm(all_ctas));
+        const int chunks = (p.K + kFewChunk - 1) / kFewChunk, passes = (p.M + kFewRows - 1) / kFewRows;
+        const float t_few = 2.5f + passes * (1.5f + 0.57f * chunks * per_sm((long long)((p.N + kFewFeatures - 1) / kFewFeatures) * batch));
+        few = p.M <= kFewMaxRows && chunks <= kFewMaxWarps && t_few <= fminf(t_tile, t_all);
+        if (!few && t_all < t_tile) return 1;
+    }
+    if (few) {
         switch (p.M) {
             case 1: return launch_few<1>(p, batch, stream);
             case 2: return launch_few<2>(p, batch, stream);
@@ -360,12 +387,6 @@ int gemm_f32_launch(const GemmF32& p, int batch, cudaStream_t stream) {
             default: return launch_few<8>(p, batch, stream);
         }
     }
-    const int groups = f32_groups(p.K);
-    const dim3 grid((p.N + kTileN - 1) / kTileN, (p.M + kTileM - 1) / kTileM, batch);
-    // rounds of resident CTAs, in groups of K: a tile whole, or its groups apart where that fills the last round better (and
-    // the launch's z extent holds them)
-    const long long tiles = (long long)grid.x * grid.y * batch;
-    const bool split = groups > 1 && (long long)batch * groups <= 65535 && (tiles * groups + kTileCtas - 1) / kTileCtas < (tiles + kTileCtas - 1) / kTileCtas * groups;
     static SmemLimit limit_split, limit_whole;
     cudaError_t e;
     if (split) {

@@ -32,6 +32,7 @@ struct GemmF32 {
 
 // Whether the kernels of gemm_f32.cu take these operands: every row of both starts on a 16-byte boundary.
 bool gemm_f32_takes(const GemmF32& p, int batch);
+// 0: launched, 1: the all-sizes kernel is the faster one for these sizes (it adds in the same order), negative: an error.
 int gemm_f32_launch(const GemmF32& p, int batch, cudaStream_t stream);
 
 }  // namespace cib

@@ -2,16 +2,19 @@
 //
 // The reference sends every projection to cuBLAS with 32-bit accumulation
 // (csrc/ops/projection.cu:13-45).  This kernel is the fallback for shapes that the tensor-core kernels and the
-// 32-bit kernels of gemm_f32.cu refuse (rows off 16-byte boundaries).  Every output element adds in the order that
-// gemm_f32.cuh lays down, so a row's result depends neither on how many other rows are in the batch nor, in 32 bits, on
-// which kernel its address lets through.
+// 32-bit kernels of gemm_f32.cu refuse (rows off 16-byte boundaries) or would be slower at.  Every output element of 32-bit
+// operands adds in the order that gemm_f32.cuh lays down, so a row's result depends neither on how many other rows are in
+// the batch nor on which kernel its address lets through; bfloat16 operands add chains of 16 values in the order of k.
 #include "gemm_f32.cuh"
 
 namespace cib {
 
 constexpr int kBM = 64, kBN = 64, kBK = kF32Chain;
 
-template <typename TI, typename TO>
+// GROUPS: 0: every chain of 16 joins one sum (bfloat16 operands: no other kernel has to give the same bits); 1 and 2: the order
+// of gemm_f32.cuh for K of one group and of several.  The groups' sums, touched every 128 of K, lie in shared memory: in
+// registers they left an SM two CTAs instead of four (467 x 4 095 x 1 023 in 32 bits: 190 us, so 183).
+template <typename TI, typename TO, int GROUPS>
 __global__ void __launch_bounds__(256)
 gemm_generic_kernel(const TI* __restrict__ a, int lda, const TI* __restrict__ w, int ldw,
                     TO* __restrict__ out, int ldo, int M, int N, int K, long long a_batch, long long w_batch,
@@ -23,11 +26,17 @@ gemm_generic_kernel(const TI* __restrict__ a, int lda, const TI* __restrict__ w,
     out += (size_t)blockIdx.z * o_batch;
     __shared__ float As[kBK][kBM + 4];
     __shared__ float Ws[kBK][kBN + 4];
+    __shared__ float s_group[GROUPS > 0 ? 16 : 1][256], s_total[GROUPS > 1 ? 16 : 1][256];          // [output][thread]
     const int tid = threadIdx.x;
     const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
     const int tx = tid & 15, ty = tid >> 4;       // 16 x 16 threads, 4 x 4 outputs each
     const int group_k = f32_group_slices(K) * kF32Slice;
-    float slice[4][4] = {}, group[4][4] = {}, total[4][4] = {};
+    float slice[4][4] = {};
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        if (GROUPS > 0) s_group[e][tid] = 0.f;
+        if (GROUPS > 1) s_total[e][tid] = 0.f;
+    }
 
     // each thread loads 4 elements of each tile per step: row = tid / 4, k = (tid % 4) * 4 ..
     const int lrow = tid >> 2, lk = (tid & 3) * 4;
@@ -58,17 +67,18 @@ gemm_generic_kernel(const TI* __restrict__ a, int lda, const TI* __restrict__ w,
 #pragma unroll
             for (int j = 0; j < 4; ++j) slice[i][j] += part[i][j];
         const int done = k0 + kBK;
-        if (done % kF32Slice == 0 || done >= K) {
+        if (GROUPS > 0 && (done % kF32Slice == 0 || done >= K)) {
+            const bool group_ends = GROUPS > 1 && (done % group_k == 0 || done >= K);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { group[i][j] += slice[i][j]; slice[i][j] = 0.f; }
-            if (done % group_k == 0 || done >= K) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) { total[i][j] += group[i][j]; group[i][j] = 0.f; }
-            }
+                for (int j = 0; j < 4; ++j) {
+                    const int e = i * 4 + j;
+                    const float sum = s_group[e][tid] + slice[i][j];
+                    slice[i][j] = 0.f;
+                    s_group[e][tid] = group_ends ? 0.f : sum;
+                    if (group_ends) s_total[e][tid] += sum;
+                }
         }
         __syncthreads();
     }
@@ -79,7 +89,7 @@ gemm_generic_kernel(const TI* __restrict__ a, int lda, const TI* __restrict__ w,
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
-            if (n < N) out[(size_t)m * ldo + n] = from_f32<TO>(total[i][j]);
+            if (n < N) out[(size_t)m * ldo + n] = from_f32<TO>(GROUPS == 0 ? slice[i][j] : GROUPS == 1 ? s_group[i * 4 + j][tid] : s_total[i * 4 + j][tid]);
         }
     }
 }
@@ -96,16 +106,19 @@ static int gemm_generic_launch(const void* a, int lda, long long a_batch, const 
     if (M == 0) return 0;
     if (in_dtype == kF32 && out_dtype == kF32) {
         const GemmF32 p{(const float*)a, (const float*)w, (float*)out, lda, ldw, ldo, M, N, K, a_batch, w_batch, o_batch, w_constant != 0};
-        if (gemm_f32_takes(p, batch)) return gemm_f32_launch(p, batch, stream);
+        if (gemm_f32_takes(p, batch)) {
+            const int rc = gemm_f32_launch(p, batch, stream);
+            if (rc <= 0) return rc;
+        }
     }
     dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, batch);
     CIB_REQUIRE(grid.y <= 65535 && batch <= 65535, "gemm: M=%d or batch=%d too large for this kernel", M, batch);
     if (in_dtype == kF32 && out_dtype == kF32)
-        gemm_generic_kernel<float, float><<<grid, 256, 0, stream>>>((const float*)a, lda, (const float*)w, ldw, (float*)out, ldo, M, N, K, a_batch, w_batch, o_batch);
+        (f32_groups(K) == 1 ? gemm_generic_kernel<float, float, 1> : gemm_generic_kernel<float, float, 2>)<<<grid, 256, 0, stream>>>((const float*)a, lda, (const float*)w, ldw, (float*)out, ldo, M, N, K, a_batch, w_batch, o_batch);
     else if (in_dtype == kBF16 && out_dtype == kBF16)
-        gemm_generic_kernel<__nv_bfloat16, __nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw, (__nv_bfloat16*)out, ldo, M, N, K, a_batch, w_batch, o_batch);
+        gemm_generic_kernel<__nv_bfloat16, __nv_bfloat16, 0><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw, (__nv_bfloat16*)out, ldo, M, N, K, a_batch, w_batch, o_batch);
     else if (in_dtype == kBF16 && out_dtype == kF32)
-        gemm_generic_kernel<__nv_bfloat16, float><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw, (float*)out, ldo, M, N, K, a_batch, w_batch, o_batch);
+        gemm_generic_kernel<__nv_bfloat16, float, 0><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, ldw, (float*)out, ldo, M, N, K, a_batch, w_batch, o_batch);
     else
         CIB_REQUIRE(false, "gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
     CIB_LAUNCH_CHECK("gemm_generic");
