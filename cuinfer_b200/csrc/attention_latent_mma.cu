@@ -303,7 +303,9 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q_abs, int qa_stri
 // The splits' maxima and sums are read by as many threads at once and turned into weights in shared memory; the rows are then
 // a stream of independent 8-byte loads, eight in flight a thread.  (Every thread used to read the maxima one by one, twice:
 // 32 splits of 8 rows x 32 heads x 512 took 18 us.)
+// WIDE: the partials start on 8 bytes and the output rows on 4, so that a pair of columns is one access.
 constexpr int kMergeChunk = 512;
+template <bool WIDE>
 __global__ void __launch_bounds__(256)
 latent_attention_merge_kernel(const float* __restrict__ part, const float* __restrict__ sinks,
                               __nv_bfloat16* __restrict__ out, int out_stride, int H, int rk, int splits, int rows) {
@@ -334,10 +336,10 @@ latent_attention_merge_kernel(const float* __restrict__ part, const float* __res
         const int count = min(kMergeChunk, end - first);
         __syncthreads();
         for (int s = tid; s < count; s += blockDim.x) {
-            const float2 ml = *reinterpret_cast<const float2*>(p + (first + s) * stride);
-            const float f = ml.x == -INFINITY ? 0.f : exp2f(ml.x - M);
+            const float m = p[(first + s) * stride], l = p[(first + s) * stride + 1];
+            const float f = m == -INFINITY ? 0.f : exp2f(m - M);
             s_w[s] = f;
-            if (f != 0.f) L += ml.y * f;
+            if (f != 0.f) L += l * f;
         }
         __syncthreads();
         if (c < rk) {
@@ -345,7 +347,7 @@ latent_attention_merge_kernel(const float* __restrict__ part, const float* __res
 #pragma unroll 8
             for (int s = 0; s < count; ++s) {
                 const float f = s_w[s];
-                const float2 v = *reinterpret_cast<const float2*>(src + s * stride);
+                const float2 v = WIDE ? *reinterpret_cast<const float2*>(src + s * stride) : make_float2(src[s * stride], src[s * stride + 1]);
                 acc.x = fmaf(f != 0.f ? v.x : 0.f, f, acc.x);   // a split without keys may not have written its row
                 acc.y = fmaf(f != 0.f ? v.y : 0.f, f, acc.y);
             }
@@ -354,7 +356,10 @@ latent_attention_merge_kernel(const float* __restrict__ part, const float* __res
     L = block_sum(L, s_red) + (sink == -INFINITY ? 0.f : exp2f(sink - M));
     if (c < rk) {
         const float inv = L > 0.f ? 1.f / L : 0.f;
-        *reinterpret_cast<__nv_bfloat162*>(out + (size_t)token * out_stride + (size_t)head * rk + c) = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
+        __nv_bfloat16* dst = out + (size_t)token * out_stride + (size_t)head * rk + c;
+        const __nv_bfloat162 pair = __floats2bfloat162_rn(acc.x * inv, acc.y * inv);
+        if (WIDE) *reinterpret_cast<__nv_bfloat162*>(dst) = pair;
+        else { dst[0] = pair.x; dst[1] = pair.y; }
     }
 }
 
@@ -436,8 +441,9 @@ extern "C" int cib_latent_attention_mma(const void* q_abs, int qa_stride, const 
     CIB_LAUNCH_CHECK("latent_attention_mma");
     if (splits > 1) {
         const int rows = num_tokens * H;
-        latent_attention_merge_kernel<<<rows, rk > 256 ? 256 : 128, 0, stream>>>(scratch, sinks, (__nv_bfloat16*)out, out_stride, H, rk,
-                                                                           splits, rows);
+        const bool wide = (uintptr_t)scratch % 8 == 0 && (uintptr_t)out % 4 == 0;      // (rk and out_stride are even)
+        const auto merge = wide ? latent_attention_merge_kernel<true> : latent_attention_merge_kernel<false>;
+        merge<<<rows, rk > 256 ? 256 : 128, 0, stream>>>(scratch, sinks, (__nv_bfloat16*)out, out_stride, H, rk, splits, rows);
         CIB_LAUNCH_CHECK("latent_attention_merge");
     }
     return 0;

@@ -748,6 +748,26 @@ def test_paged_attention_decode_refuses_other_sizes():
                                  torch.ones(1, dtype=torch.int32, device=DEV), 6, 3, 48, 1.0, 0, 1)
 
 
+@pytest.mark.parametrize("H, rk, dr", [(8, 64, 16), (4, 288, 32)])
+def test_latent_attention_merge_into_rows_off_word_boundaries(H, rk, dr):
+    """A decode step whose keys several CTAs share, written into a column range that starts on an odd element: the merge
+    stores single values there, the same ones."""
+    k = _k()
+    R, n, dn, ps = 3, 700, 16, 16
+    P_ = n // ps + 1
+    assert k.latent_attention_splits(R, 1, n) > 1
+    cache = rand(R * P_, 1, 1, ps, rk + dr, seed=61, dtype=torch.bfloat16).to(DEV)
+    q_abs, q = rand(R, H * rk, seed=62, dtype=torch.bfloat16).to(DEV), rand(R, H * (dn + dr), seed=63, dtype=torch.bfloat16).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    bt = torch.arange(R * P_, dtype=torch.int32, device=DEV).view(R, P_)
+    outs = [torch.zeros(R, H * rk, dtype=torch.bfloat16, device=DEV), torch.full((R, H * rk + 2), 5.0, dtype=torch.bfloat16, device=DEV)]
+    for out in (outs[0], outs[1][:, 1:-1]):
+        k.latent_attention_mma(q_abs, q, out, cache, bt, i32(range(R + 1)), i32([n, 40, 333]), [1] * R, None, 0, None, H, dn, rk, dr,
+                               0.05, n, decode_only=True)
+    assert torch.equal(outs[0], outs[1][:, 1:-1]) and bool((outs[1][:, 0] == 5.0).all()) and bool((outs[1][:, -1] == 5.0).all())
+    assert float(outs[0].float().abs().max()) > 0.0
+
+
 # ---- sampling ----------------------------------------------------------------------------------------------------
 
 def _sample(k, logits, rows):
