@@ -373,9 +373,10 @@ attention_f32_tile_kernel(const AttnF32 p) {
     }
 }
 
-// Few tokens: while a CTA per (token, block of heads) is at most two for each SM, and for as many tokens as requests (a step
-// of decoded tokens: 32 requests of 1 000 keys, 12 heads of 64 over 4, 40 us, 1 760 in tiles of several requests); beyond, a key is read for one token where the tile kernel reads it for several.  As many CTAs to
-// a cluster as the SMs have room for without a second round.
+// Few tokens: while a CTA per (token, block of heads) is at most two for each SM, and for as many tokens as
+// requests (a step of decoded tokens: 32 requests of 1 000 keys, 12 heads of 64 over 4, 40 us, 1 760 in tiles of several
+// requests); beyond, a key is read for one token where the tile kernel reads it for several.  As many CTAs to a cluster as
+// the SMs have room for without a second round.
 constexpr int kFewAttnCtas = 296;
 
 template <int D, int HB>

@@ -10,7 +10,10 @@
 // A tile of 128 keys takes it about 1.9 us; one CTA of the other variant takes 2.2 us or more for 128 keys, but an SM has two
 // of them.  So this one is better while a launch has at most three CTAs for each SM and its longest row tile decides (one
 // prompt of 2 048 tokens, 256 CTAs: 31.9 us a layer against 39.8; of 2 560, 320 CTAs: 48.8 against 50.6), the other beyond
-// (one of 8 192, 1 024 CTAs: 328 us against 275).
+// (one of 8 192, 1 024 CTAs: 328 us against 275).  Around the line, this variant against the other: one prompt of 3 600 tokens
+// (450 CTAs) 80.8 / 82.2, of 3 700 (464) 83.5 / 78.4, of 4 096 (512) 96 / 77; 8 of 400 (448) 32.4 / 26.8; joined rows with sinks
+// the same within 2 %.  Steps of decoded tokens among prompts, whose row tiles are nearly empty and of very different lengths,
+// 320 to 400 CTAs: contexts up to 1 100 keys 51 / 40, up to 3 500 keys 71 / 85.
 //
 // Every mbarrier wait is bounded; on a time-out the kernel raises the error flag, stops, frees its tensor memory
 // and returns.

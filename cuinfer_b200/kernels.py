@@ -667,7 +667,8 @@ def paged_attention_decode(q: torch.Tensor, out: torch.Tensor, cache: torch.Tens
     every (request, kv head) split over ``splits`` CTAs.  Allocates the partial-result scratch with torch.
     ``tma``: let the kernel fetch the cache through TMA where the geometry allows it (default: yes).  That path
     streams faster but starts slower, so callers that know the keys per CTA pass False for short streams.
-    ``warm``: a tensor that the kernel after this one reads first; fetched into the L2 when the stream of keys ends."""
+    ``warm``: a tensor that the kernel after this one reads first; the CTAs that have keys ask for their shares of it to be
+    fetched into the L2 when their stream of keys ends."""
     R = q.shape[0]
     warm = _l2_hint(warm)
     if q.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16:

@@ -95,7 +95,8 @@ _FORCE_GENERIC_WINDOW = os.environ.get("CUINFER_B200_WINDOW_ATTENTION", "") == "
 # From how many (request, key head) pairs on a step of single tokens runs on the tcgen05 kernel too — one CTA per pair
 # walks the keys in tiles of 128 — instead of the kernel that shares a pair's key tiles out to several CTAs.  Measured
 # a call at 2 084 / 8 192 keys of 8 key heads: 1 request 37 / 124 us against 31 / 82; 8 requests 38 / 125 against 53 /
-# 163; 64 requests 151 / 494 against 438 / 1 669.
+# 163; 64 requests 151 / 494 against 438 / 1 669.  From 56 requests of 8 key heads on the launch runs on the variant of 64-key
+# tiles, which is faster still: 64 requests of 300 / 1 100 / 4 000 keys 46 / 92 / 256 us on the one of 128, 29 / 73 / 223 on it.
 TCGEN05_DECODE_MIN_CTAS = 48
 
 
