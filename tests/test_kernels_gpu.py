@@ -143,14 +143,17 @@ def test_gemm_generic(M, N, K, dtypes):
 @pytest.mark.parametrize("N, K", [(8, 16), (1001, 132), (520, 1028), (4096, 1024), (1024, 3072), (72, 5000), (40, 16384)])
 def test_gemm_32bit_paths(N, K):
     """Few rows, tiles with and without K split over a cluster, and rows off 16-byte boundaries: one order of additions, so
-    the same bits; sums of 16-long chains of K products are within (16 + 8 + 12 + 8) roundings of the exact one, each at
-    most 2^-24 of the sum of magnitudes."""
+    the same bits; a product passes 16 roundings in its chain, 8 in its slice, and one for every slice of its group and every
+    group, each at most 2^-24 of the sum of magnitudes."""
     k = _k()
     M = 700
     a, w = rand(M, K, seed=91).to(DEV), rand(N, K, seed=92).to(DEV)
     full = torch.empty(M, N, device=DEV)
     k.gemm_generic(a, w, full)
-    bound = (a.double().abs() @ w.double().abs().T) * 44 * 2.0 ** -24
+    slices = -(-K // 128)
+    per_group = max(4, -(-slices // 8))
+    depth = 16 + 8 + per_group + -(-slices // per_group)
+    bound = (a.double().abs() @ w.double().abs().T) * depth * 2.0 ** -24
     assert bool(((full.double() - a.double() @ w.double().T).abs() <= bound).all())
     for rows in (1, 3, 8, 9, 31, 33, 64, 257):
         wide = torch.full((rows, N + 3), 7.0, device=DEV)                # output rows off 16-byte boundaries
@@ -709,12 +712,33 @@ def test_paged_attention_decode_any_number_of_ctas_with_keys(nq, nkv, d, splits,
     close(out, decode_reference(case, 1.0 / math.sqrt(d)), 1.5e-2)
 
 
+@pytest.mark.parametrize("requests", [1, 2])
+@pytest.mark.parametrize("splits", [2, 5, 6, 8])
+@pytest.mark.parametrize("lens", [(1, 64), (65, 300), (320, 321), (511, 512), (700, 40), (2000, 1)])
+def test_paged_attention_decode_clusters_up_to_eight(requests, splits, lens):
+    """Launches of at most a CTA a SM meet in clusters of up to eight on both copy paths: one, some and all CTAs with keys."""
+    k = _k()
+    nq, nkv, d, ps = 16, 8, 128, 16
+    lens = list(lens)[:requests]
+    assert k.decode_merges_in_cluster(requests * nkv, splits, nq // nkv, d)
+    case = attention_case(torch.bfloat16, nq, nkv, d, lens, [1] * requests, ps, seed=splits, sharp=True, poison=True)
+    scale = 1.0 / math.sqrt(d)
+    sl = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    cache, bt, wide = case["cache"].to(DEV), case["bt"].to(DEV), case["wide"].to(DEV)
+    want = decode_reference(case, scale)
+    for tma in (True, False):
+        out = torch.full((requests, nq * d), 5.0, dtype=torch.bfloat16, device=DEV)
+        k.paged_attention_decode(wide, out, cache, bt, sl, nq, nkv, d, scale, 0, splits, tma=tma)
+        k.check_error_flags()
+        close(out, want, 1.5e-2)
+
+
 @pytest.mark.parametrize("requests", [3, 45])
 @pytest.mark.parametrize("splits", [2, 4])
 def test_paged_attention_decode_cluster_and_memory_combine(requests, splits):
-    """Two to four splits on the TMA path meet in a cluster's shared memory while all clusters of the launch run at
-    once (3 requests x 8 heads), and through the scratch buffer when they would not (45 x 8 clusters): both against the
-    plain attention, and the copy paths against each other."""
+    """Splits meet in a cluster's shared memory while all clusters of the launch run at once (3 requests x 8 heads), and
+    through the scratch buffer when they would not (45 x 8 clusters): both against the plain attention, and the copy paths
+    against each other."""
     k = _k()
     nq, nkv, d, ps = 16, 8, 128, 16
     rnd = random.Random(requests * 10 + splits)

@@ -576,6 +576,24 @@ def test_joined_rows_and_sinks_on_tcgen05(H, G):
         _close(got, want, dtype, f"query {n - 1} with key {j} standing out")
 
 
+@pytest.mark.parametrize("H,G", [(16, 8), (8, 8), (64, 8)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_joined_rows_and_sinks_on_tcgen05_in_full_launches(H, G, window):
+    """More than three CTAs a SM, the variant that walks tiles of 64 keys: contexts that end on a tile, one short of it and one
+    past it, decoded tokens beside portions, a key standing out, and sinks far above and far below every score."""
+    lengths = ([64, 65, 63, 128, 129, 1, 200, 191, 300, 192] * 6)[:58]
+    new = ([64, 1, 63, 2, 1, 1, 65, 1, 3, 1] * 6)[:58]
+    assert sum(-(-n * H // G // 128) for n in new) * G > 444
+    sink = torch.linspace(-2.0, 2.0, H, dtype=torch.float64)
+    sink[0], sink[1] = 60.0, -60.0
+    sharpen = {64: 0, 129: 100}                         # the one token of request 1, the last of request 3
+    got, want = _sink_case(torch.bfloat16, H, G, 128, lengths, new, 16, H + window, sink=sink, sharpen=sharpen, tensor_cores="tcgen05",
+                           window=window)
+    _close(got, want, torch.bfloat16, f"tcgen05 attention over joined rows in a full launch, window {window}")
+    others = [t for t in range(sum(new)) if t not in sharpen]
+    assert float(got[others, 0].float().abs().max()) < 1e-6 and float(got[:, 1].float().abs().max()) > 1e-2
+
+
 @pytest.mark.parametrize("E,top,groups,keep", [(8, 3, 2, 1), (6, 2, 3, 2), (5, 2, 1, 1), (4, 4, 2, 2), (6, 1, 6, 2), (130, 7, 10, 3),
                                                (12, 5, 4, 4), (1, 1, 1, 1), (1000, 9, 8, 2)])
 def test_scored_router(E, top, groups, keep):
