@@ -53,4 +53,4 @@ bool prompt_pdl() { return g_prompt_pdl != 0; }
 extern "C" void cib_set_prompt_pdl(int on) { cib::g_prompt_pdl = on; }
 
 // Bumped whenever an exported signature changes, so that a stale library is rebuilt, not misused.
-extern "C" int cib_abi_version() { return 2; }
+extern "C" int cib_abi_version() { return 3; }

@@ -119,7 +119,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cib_paged_attention_decode": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _I, _I, _I, _I, _F, _I, _I, _P, _P, _I, _P, _P, ctypes.c_longlong, _P],
         "cib_paged_attention_prefill": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
         "cib_attention_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P],
-        "cib_gemm_skinny": [_P, _I, _I, _I, _P, _I, _P, _P, _I, _P, _I, _F, _P, _P, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P],
+        "cib_gemm_skinny": [_P, _I, _I, _I, _P, _I, _P, _P, _I, _P, _I, _F, _P, _P, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P, _I, _P, _P, _P],
         "cib_gemm_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
         "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
         "cib_gemm_generic": [_P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P],
@@ -852,6 +852,7 @@ use_pdl = os.environ.get("CUINFER_B200_PDL", "1") != "0"
 
 EPILOGUE_BF16, EPILOGUE_F32, EPILOGUE_SILU_PAIR = 0, 1, 2
 EPILOGUE_GELU_PAIR = 3          # as the SiLU pair, with the tanh form of GELU as the gate
+EPILOGUE_STREAM = 4             # added to the 32-bit residual, which leaves with the next norm's gains
 
 
 def gemm_skinny_supports(M: int, N: int, K: int, with_norm: bool = False) -> bool:
@@ -861,17 +862,33 @@ def gemm_skinny_supports(M: int, N: int, K: int, with_norm: bool = False) -> boo
 def gemm_skinny(w: torch.Tensor, out: torch.Tensor, *, act: torch.Tensor | None = None,
                 residual: torch.Tensor | None = None, pending: torch.Tensor | None = None,
                 norm_weight: torch.Tensor | None = None, eps: float = 0.0, residual_out: torch.Tensor | None = None,
-                silu_pair: bool = False, warm: torch.Tensor | None = None) -> None:
+                silu_pair: bool = False, warm: torch.Tensor | None = None, squares: torch.Tensor | None = None,
+                stream: torch.Tensor | None = None, squares_out: torch.Tensor | None = None) -> None:
     """out = act @ w^T for at most 16 rows, bfloat16 weights.  ``warm``: a tensor that the kernel after this one
     reads first (its weights); the kernel asks for it to be fetched into the L2 while it runs.
 
     Either ``act`` [M, K] is given, or ``residual`` (float32 [M, K]) with optional ``pending``: then the rows are
     RMSNorm(residual + pending) * norm_weight, computed in the kernel, and ``residual_out`` (another buffer)
     receives residual + pending.  ``silu_pair``: ``w`` is [2I, K] = gates then ups and out [M, I] = silu(g) * u.
-    ``out`` float32 selects the 32-bit store."""
+    ``out`` float32 selects the 32-bit store.
+
+    A norm between two products is shared by them: the one before it gets ``stream`` (float32 [M, N], updated in place by its
+    result), ``norm_weight`` and ``squares_out`` (float32 [M, ceil(N / 16)]) and leaves ``out`` = bfloat16(stream * norm_weight)
+    and the sums of stream^2 over 16 columns each; the one after it gets those rows as ``act`` and the sums as ``squares``, and
+    multiplies its result rows by rsqrt(sum / K + eps)."""
     N, K = w.shape
     M = out.shape[0]
     warm = _l2_hint(warm)
+    if squares is not None and (act is None or squares.dtype != torch.float32 or squares.dim() != 2 or squares.shape[0] != M
+                                or not squares.is_contiguous()):
+        raise KernelError("gemm_skinny: squares must be contiguous float32 [M, parts] and go with act")
+    if stream is not None:
+        if silu_pair or residual is not None or out.dtype != torch.bfloat16 or norm_weight is None or norm_weight.numel() != N:
+            raise KernelError("gemm_skinny: a stream goes with plain rows, bfloat16 out and N gains")
+        if stream.dtype != torch.float32 or stream.shape != (M, N) or not stream.is_contiguous():
+            raise KernelError("gemm_skinny: stream must be contiguous float32 [M, N]")
+        if squares_out is None or squares_out.dtype != torch.float32 or squares_out.shape != (M, -(-N // 16)) or not squares_out.is_contiguous():
+            raise KernelError("gemm_skinny: squares_out must be contiguous float32 [M, ceil(N / 16)]")
     if w.dtype != torch.bfloat16 or w.stride(1) != 1:
         raise KernelError("gemm_skinny: weights must be bfloat16 with dense rows")
     if silu_pair:
@@ -881,7 +898,7 @@ def gemm_skinny(w: torch.Tensor, out: torch.Tensor, *, act: torch.Tensor | None 
     else:
         if out.shape[1] != N:
             raise KernelError(f"gemm_skinny: out must be [M, {N}]")
-        epi = EPILOGUE_F32 if out.dtype == torch.float32 else EPILOGUE_BF16
+        epi = EPILOGUE_STREAM if stream is not None else EPILOGUE_F32 if out.dtype == torch.float32 else EPILOGUE_BF16
         if out.dtype not in (torch.float32, torch.bfloat16):
             raise KernelError("gemm_skinny: out must be bfloat16 or float32")
     if out.stride(1) != 1:
@@ -909,6 +926,8 @@ def gemm_skinny(w: torch.Tensor, out: torch.Tensor, *, act: torch.Tensor | None 
         _cuda(residual_out, "residual_out") if residual_out is not None else None,
         _cuda(out, "out", contiguous=False), out.stride(0), M, epi, N // 2 if silu_pair else 0, 1 if use_pdl else 0,
         warm.data_ptr() if warm is not None else None, warm.numel() * warm.element_size() if warm is not None else 0,
+        _cuda(squares, "squares") if squares is not None else None, squares.shape[1] if squares is not None else 0,
+        _cuda(stream, "stream") if stream is not None else None, _cuda(squares_out, "squares_out") if squares_out is not None else None,
         _stream())
     _check(rc, "gemm_skinny")
     _count()

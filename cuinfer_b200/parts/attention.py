@@ -95,6 +95,12 @@ class PagedAttention(Mixer):
         return self.qkv.workspace_bytes(tokens) + tokens * self.q_size * width + self.o.workspace_bytes(tokens)
 
     def forward(self, x: torch.Tensor, ctx: StepContext, run: int) -> torch.Tensor:
+        return self.o.forward(self._attend(x, ctx, run))
+
+    def forward_deferred(self, x: torch.Tensor, ctx: StepContext, run: int):
+        return self.o.defer(self._attend(x, ctx, run))
+
+    def _attend(self, x: torch.Tensor, ctx: StepContext, run: int) -> torch.Tensor:
         kv = ctx.paged_kv(run)
         qkv = self.qkv.forward(x)
         kernels.qk_norm_rope_kv_write(
@@ -105,4 +111,4 @@ class PagedAttention(Mixer):
         out = torch.empty((qkv.shape[0], self.q_size), dtype=qkv.dtype, device=qkv.device)
         attention_dispatch.paged_attention(qkv, out, kv, ctx, self.num_heads, self.num_kv_heads, self.head_dim,
                                            self.scale, self.window, warm=self.o.weight)
-        return self.o.forward(out)
+        return out

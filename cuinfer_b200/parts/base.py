@@ -40,9 +40,12 @@ class ResidualStream:
     A layer whose two sub-layers read the same rows leaves both outputs at once: ``pending`` and ``pending_second`` (of one
     dtype) then join the residual together, and ``pending_scale`` multiplies what joins.  A norm that takes all three adds
     them in its own pass (``take_deltas``); ``settle()`` does it alone.
+
+    A plain delta may also wait as a product that has not been launched (``DeferredProduct``): whoever reads ``pending`` gets
+    its rows, and a ``LazyNorm`` whose consumer can share the norm with it takes it as it is (``deferred``).
     """
 
-    __slots__ = ("residual", "pending", "pending_norm", "extra", "_spare", "writer", "pending_second", "pending_scale")
+    __slots__ = ("residual", "_pending", "pending_norm", "extra", "_spare", "writer", "pending_second", "pending_scale")
 
     def __init__(self, residual: torch.Tensor, pending: Optional[torch.Tensor] = None) -> None:
         self.residual = residual
@@ -55,9 +58,24 @@ class ResidualStream:
         self.pending_scale = 1.0
 
     @property
+    def pending(self) -> Optional[torch.Tensor]:
+        if isinstance(self._pending, DeferredProduct):
+            self._pending = self._pending.run()
+        return self._pending
+
+    @pending.setter
+    def pending(self, delta) -> None:
+        self._pending = delta
+
+    @property
+    def deferred(self) -> Optional["DeferredProduct"]:
+        """The pending delta if it is a product that has not been launched yet."""
+        return self._pending if isinstance(self._pending, DeferredProduct) else None
+
+    @property
     def scaled(self) -> bool:
         """True when the outstanding delta is more than one plain tensor: a second one or a factor goes with it."""
-        return self.pending is not None and (self.pending_second is not None or self.pending_scale != 1.0)
+        return self._pending is not None and (self.pending_second is not None or self.pending_scale != 1.0)
 
     @property
     def plain(self) -> bool:
@@ -144,6 +162,19 @@ class ResidualStream:
         self.pending = None
 
 
+class DeferredProduct:
+    """A projection's last product, not launched yet: the next norm decides how its rows leave the kernel."""
+
+    __slots__ = ("linear", "rows")
+
+    def __init__(self, linear, rows: torch.Tensor) -> None:
+        self.linear = linear
+        self.rows = rows
+
+    def run(self) -> torch.Tensor:
+        return self.linear.forward(self.rows)
+
+
 class LazyNorm:
     """A norm of the residual stream that has not been computed yet.
 
@@ -152,16 +183,29 @@ class LazyNorm:
     ``materialize()`` gives the normed rows as a tensor, whatever happened before.
     """
 
-    __slots__ = ("stream", "norm", "_rows")
+    __slots__ = ("stream", "norm", "_rows", "_carried")
 
     def __init__(self, stream: ResidualStream, norm: "Norm") -> None:
         self.stream = stream
         self.norm = norm
         self._rows: Optional[torch.Tensor] = None
+        self._carried: Optional[tuple] = None
 
     @property
     def shape(self):
         return self.stream.residual.shape
+
+    def carried(self) -> Optional[tuple]:
+        """``(rows, squares, eps)``: the residual's rows times the norm's gains in bfloat16, and parts of their sums of squares
+        before the gains, for a product that applies the rest of the norm to its result; from the kernel of the product that
+        is pending.  None when there is no such product or norm."""
+        if self._carried is None and self._rows is None and self.stream.deferred is not None and self.stream.plain:
+            rms = self.norm.fusable_rms()
+            done = self.stream.deferred.linear.into_stream(self.stream.deferred.rows, self.stream.residual, rms[0]) if rms else None
+            if done is not None:
+                self.stream.pending = None
+                self._carried = (*done, rms[1])
+        return self._carried
 
     def materialize(self) -> torch.Tensor:
         if self._rows is None:
@@ -245,10 +289,18 @@ class Mixer(Part):
     def forward(self, x: torch.Tensor, ctx: StepContext, run: int) -> torch.Tensor:
         raise NotImplementedError
 
+    def forward_deferred(self, x: torch.Tensor, ctx: StepContext, run: int):
+        """``forward``, whose last product may be left to the next norm (a ``DeferredProduct``)."""
+        return self.forward(x, ctx, run)
+
 
 class FeedForward(Part):
     def forward(self, x: torch.Tensor, ctx: StepContext) -> torch.Tensor:
         raise NotImplementedError
+
+    def forward_deferred(self, x: torch.Tensor, ctx: StepContext):
+        """As ``Mixer.forward_deferred``."""
+        return self.forward(x, ctx)
 
 
 class Block:

@@ -44,10 +44,10 @@ class PreNormBlock(Block):
 
     def forward(self, stream: ResidualStream, ctx: StepContext, run: int) -> None:
         h = self._normed(stream, self.mixer_norm, self.mixer)
-        stream.pending = self.mixer.forward(h, ctx, run)
+        stream.pending = self.mixer.forward_deferred(h, ctx, run)
         if self.has_feed_forward:
             h = self._normed(stream, self.feed_forward_norm, self.feed_forward)
-            stream.pending = self.feed_forward.forward(h, ctx)
+            stream.pending = self.feed_forward.forward_deferred(h, ctx)
         if self.tail is not None:
             self.tail.forward(stream, ctx)
 

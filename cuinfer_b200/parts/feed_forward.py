@@ -61,6 +61,9 @@ class SwiGLU(FeedForward):
         act = self.gate_up.forward(x, silu_pair=self._pair)       # act(gate) * up, fused where the kernel allows
         return self.down.forward(act)
 
+    def forward_deferred(self, x: torch.Tensor, ctx: StepContext):
+        return self.down.defer(self.gate_up.forward(x, silu_pair=self._pair))
+
 
 @FEED_FORWARDS.register("none")
 class NoFeedForward(FeedForward):

@@ -1,8 +1,8 @@
 """Choice of the bfloat16 matrix-product kernel for a given shape.
 
 * up to 16 rows (decode steps), weights under 24 MB (every matrix of the Qwen3-0.6B layer sizes): the few-rows kernel
-  (``gemm_skinny``), weights streamed once through registers, with the norm in its prologue and the SiLU gate in its
-  epilogue; larger weights (the 8B and 32B layer sizes) go to the library, which measured faster on all of them —
+  (``gemm_skinny``), weights streamed once through registers, with a norm shared by the products on its two sides (or in its
+  prologue) and the SiLU gate in its epilogue; larger weights (the 8B and 32B layer sizes) go to the library, which measured faster on all of them —
   6144 x 4096: 11.5 us against 19.5 (few-rows) and 21.6 (weight-streaming); 24576 x 4096: 34.3 against 43.5 and 46.0;
   10240 x 5120: 22.3 against 39.6 and 33.8; 5120 x 25600: 44 against 69 (weight-streaming); 151936 x 4096: 198 against
   216 and 204 — except long K with few output features (4096 x 12288: weight-streaming tcgen05 kernel 22.4 us, library

@@ -16,7 +16,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from .. import kernels
-from .base import LazyNorm
+from .base import DeferredProduct, LazyNorm
 from .spec import TensorSpec
 
 
@@ -144,6 +144,30 @@ class Linear:
         kernels.silu_mul(y, act, gelu=silu_pair == "gelu_tanh")
         return act
 
+    def defer(self, x: torch.Tensor):
+        """The product of ``x`` as rows, or unlaunched where the norm after it may share its kernel (see ``into_stream``)."""
+        return DeferredProduct(self, x) if self._takes_skinny(x.shape[0]) and x.dtype == torch.bfloat16 else self.forward(x)
+
+    def into_stream(self, x: torch.Tensor, residual: torch.Tensor, gain: torch.Tensor) -> Optional[tuple]:
+        """Add the product of ``x`` to the 32-bit ``residual`` in place; ``(rows, squares)``: the new residual times ``gain`` in
+        bfloat16 and the sums of its squares over 16 columns each, from the product's own kernel.  None where it does not
+        take the shape (nothing has happened then)."""
+        M, N = residual.shape
+        if (not self._takes_skinny(M) or x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16
+                or not residual.is_contiguous() or gain.numel() != N or self.weight.shape[0] != N):
+            return None
+        rows = torch.empty((M, N), dtype=torch.bfloat16, device=residual.device)
+        squares = torch.empty((M, -(-N // 16)), dtype=torch.float32, device=residual.device)
+        kernels.gemm_skinny(self.weight, rows, act=x, norm_weight=gain, stream=residual, squares_out=squares, warm=self.warm_next)
+        return rows, squares
+
+    def _takes_skinny(self, M: int) -> bool:
+        """Whether ``M`` plain rows run on the few-rows kernel."""
+        from . import gemm_dispatch
+        w = self.weight
+        return (w is not None and w.dtype == torch.bfloat16 and w.is_contiguous() and 0 < M <= gemm_dispatch.FEW_ROWS
+                and gemm_dispatch.few_rows_kernel(M, *w.shape) == "skinny" and kernels.gemm_skinny_supports(M, *w.shape))
+
     def _forward_skinny(self, x, out_dtype, silu_pair) -> Optional[torch.Tensor]:
         """The few-rows kernel with the norm in its prologue and/or the gate in its epilogue, when it takes
         the shape; None otherwise."""
@@ -171,6 +195,12 @@ class Linear:
                 return None
             out = torch.empty((M, out_cols), dtype=torch.bfloat16, device=w.device)
             kernels.gemm_wstream(rows, w, out, silu_pair=True)
+            return out
+        carried = x.carried() if lazy and kernels.gemm_skinny_supports(M, N, K) else None
+        if carried is not None:
+            rows, squares, eps = carried
+            out = torch.empty((M, out_cols), dtype=out_dtype, device=w.device)
+            kernels.gemm_skinny(w, out, act=rows, squares=squares, eps=eps, silu_pair=silu_pair, warm=self.warm_next)
             return out
         if lazy and x._rows is None:
             stream = x.stream

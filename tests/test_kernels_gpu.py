@@ -338,6 +338,37 @@ def test_gemm_skinny_with_norm_and_gated_epilogue(M, H, I, pending_dtype):
     close(act2, g / (1 + torch.exp(-g)) * u, 1e-2)
 
 
+@pytest.mark.parametrize("M, N, K, I", [(1, 1024, 2048, 256), (8, 1024, 3072, 272), (9, 1000, 96, 40), (16, 48, 5120, 1024), (5, 4800, 1024, 520)])
+@pytest.mark.parametrize("gain_dtype", [torch.bfloat16, torch.float32])
+def test_two_products_share_a_norm(M, N, K, I, gain_dtype):
+    """A product that adds to the residual and leaves its rows with the next norm's gains, then products that apply the rest of
+    the norm to their results (with and without clusters, a slice of K in one, two or more rounds)."""
+    k = _k()
+    x, w = rand(M, K, seed=60, dtype=torch.bfloat16), rand(N, K, seed=61, scale=0.05, dtype=torch.bfloat16)
+    res, gain, eps = rand(M, N, seed=62, scale=2.0), (1 + rand(N, seed=63, scale=0.2)).to(gain_dtype), 1e-5
+    w2 = rand(2 * I, N, seed=64, scale=0.05, dtype=torch.bfloat16)
+    want = res.double() + x.double() @ w.double().T
+    stream, rows = res.to(DEV), torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    cols = 16
+    squares = torch.full((M, -(-N // cols)), 7.0, device=DEV)
+    k.gemm_skinny(w.to(DEV), rows, act=x.to(DEV), norm_weight=gain.to(DEV), stream=stream, squares_out=squares)
+    # a 32-bit accumulator takes 16 products a time: K / 16 additions, each off by at most 2^-23 of a sum no larger than the largest
+    bound = (K / 16 + 2) * 2.0 ** -23
+    close(stream, want, bound)
+    assert torch.equal(rows.cpu(), (stream * gain.to(DEV).float()).to(torch.bfloat16).cpu())
+    close(squares, torch.nn.functional.pad(want ** 2, (0, -N % cols)).view(M, -1, cols).sum(2), 2 * bound + 16 * 2.0 ** -23)
+    # the rows were rounded to bfloat16 once: the products of those rows are right to 32 bits but for the store
+    factor = torch.rsqrt((want ** 2).mean(1, keepdim=True) + eps)
+    gu = (rows.double().cpu() @ w2.double().T) * factor
+    g, u = gu[:, :I], gu[:, I:]
+    for silu in (False, True):
+        for dtype in (torch.bfloat16, torch.float32)[:1 if silu else 2]:
+            out = torch.full((M, I if silu else 2 * I), 7.0, dtype=dtype, device=DEV)
+            k.gemm_skinny(w2.to(DEV), out, act=rows, squares=squares, eps=eps, silu_pair=silu)
+            close(out, g / (1 + torch.exp(-g)) * u if silu else gu, 2e-5 if dtype == torch.float32 else 4e-3)
+    k.check_error_flags(force=True)
+
+
 def test_gemm_skinny_refuses_other_shapes():
     k = _k()
     assert not k.gemm_skinny_supports(17, 64, 64) and not k.gemm_skinny_supports(4, 64, 60)
