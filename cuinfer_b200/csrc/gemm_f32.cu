@@ -4,8 +4,7 @@
 //
 // Measured beside the kernel that took every size before (64 x 64 tiles of one CTA each, K in one piece, no copies ahead):
 // a decode step of 3 rows of the 0.6B layer sizes 10 to 14 us a projection instead of 160, the output head of 622 MB 170 us
-// (3.7 TB/s; 129 us at one row); 467 rows x 4096 x 1024 170 us (23 TFLOP/s: two warps a scheduler, which wait a third of
-// their time for memory).
+// (3.7 TB/s; 129 us at one row); 467 rows x 4096 x 1024 140 us (28 TFLOP/s).
 #include "gemm_f32.cuh"
 #include "mma_utils.cuh"
 
@@ -117,8 +116,10 @@ gemm_f32_few_kernel(const GemmF32 p, int rounds) {
 
 // ---- many rows ---------------------------------------------------------------------------------------------------------
 // Tiles of 64 x 128 outputs, 128 threads of 8 x 8: paired multiply-adds (fma.rn.f32x2: the same rounding as two fmaf in
-// half the issue slots) on operands read from shared memory one k ahead; the rows of `a` lie there as pairs of equal values,
-// so no register moves make them.  The next 16 of K come in through registers meanwhile.  A chain and a slice per output
+// half the issue slots) on operands read from shared memory one k ahead; a value of `a` becomes a pair of equal ones by
+// register moves, which go into the free issue slots (pairs kept in shared memory took 12 of its cycles a warp and k instead of
+// 8, with two warps a scheduler nearly as many as the multiply-adds: 467 x 4 096 x 1 024 167 us, 140 now; 2 048 rows 554 and 462).
+// The next 16 of K come in through registers meanwhile.  A chain and a slice per output
 // take 128 registers; the sums of the groups, touched every 128 of K, live in shared memory, which leaves room for two CTAs
 // a SM.  With SPLIT the groups of K go to the CTAs of a cluster, which add their tiles in order through each other's shared
 // memory: a product with fewer tiles than the SMs hold keeps them busy all the same.
@@ -126,7 +127,7 @@ constexpr int kTileM = 64, kTileN = 128, kTileThreads = 128;
 constexpr int kTileCtas = 2 * 148;                              // resident at once
 
 struct TileSmem {
-    float2 a[2][kF32Chain][kTileM + 2];                         // (v, v); + 2: the pairs of a thread's rows stay on 16 bytes
+    float a[2][kF32Chain][kTileM + 4];
     float w[2][kF32Chain][kTileN + 4];
     float part[64][kTileThreads];                               // the group's sum so far, [output][thread]; SPLIT: [64][128] at the end
     float total[64][kTileThreads];                              // the groups' sum (not with SPLIT)
@@ -140,6 +141,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t twice(float v) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
     return d;
 }
 __device__ __forceinline__ float2 unpack2(uint64_t v) {
@@ -185,10 +191,10 @@ gemm_f32_tile_kernel(const GemmF32 p) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int k = (aquad + h) * 4;
-            s.a[buffer][k][arow] = make_float2(av[h].x, av[h].x);
-            s.a[buffer][k + 1][arow] = make_float2(av[h].y, av[h].y);
-            s.a[buffer][k + 2][arow] = make_float2(av[h].z, av[h].z);
-            s.a[buffer][k + 3][arow] = make_float2(av[h].w, av[h].w);
+            s.a[buffer][k][arow] = av[h].x;
+            s.a[buffer][k + 1][arow] = av[h].y;
+            s.a[buffer][k + 2][arow] = av[h].z;
+            s.a[buffer][k + 3][arow] = av[h].w;
         }
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
@@ -199,7 +205,7 @@ gemm_f32_tile_kernel(const GemmF32 p) {
         }
     };
 
-    // outputs: rows i / 2 * 16 + ty * 2 + i % 2, columns tx * 4 + j and 64 + tx * 4 + j.  Neighbouring lanes share a place
+    // outputs: rows i / 4 * 32 + ty * 4 + i % 4, columns tx * 4 + j and 64 + tx * 4 + j.  Neighbouring lanes share a place
     // of `w` and lanes two apart one of `a`: a 16-byte read by the warp is then two wavefronts (it is four where lanes 0 to
     // 7 read eight places, whatever the other lanes read).
     const int tx = ((lane >> 1) & 7) + 8 * (warp & 1), ty = ((lane >> 4) << 1 | (lane & 1)) + 4 * (warp >> 1);
@@ -224,10 +230,11 @@ gemm_f32_tile_kernel(const GemmF32 p) {
         const bool more = k0 + kF32Chain < k_end;
         if (more) fetch(k0 + kF32Chain);
         uint64_t chain[8][4];
-        ulonglong2 x[2][4], y[2][2];
+        float4 x[2][2];
+        ulonglong2 y[2][2];
         auto operands = [&](int which, int k) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) x[which][i] = *reinterpret_cast<const ulonglong2*>(&s.a[buffer][k][i * 16 + ty * 2]);
+            for (int i = 0; i < 2; ++i) x[which][i] = *reinterpret_cast<const float4*>(&s.a[buffer][k][i * 32 + ty * 4]);
             y[which][0] = *reinterpret_cast<const ulonglong2*>(&s.w[buffer][k][tx * 4]);
             y[which][1] = *reinterpret_cast<const ulonglong2*>(&s.w[buffer][k][64 + tx * 4]);
         };
@@ -235,11 +242,11 @@ gemm_f32_tile_kernel(const GemmF32 p) {
 #pragma unroll
         for (int k = 0; k < kF32Chain; ++k) {
             if (k + 1 < kF32Chain) operands((k + 1) & 1, k + 1);
-            const ulonglong2* xk = x[k & 1];
+            const float4* xk = x[k & 1];
             const ulonglong2* yk = y[k & 1];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const uint64_t xi = i & 1 ? xk[i / 2].y : xk[i / 2].x;
+                const uint64_t xi = twice((i & 3) == 0 ? xk[i / 4].x : (i & 3) == 1 ? xk[i / 4].y : (i & 3) == 2 ? xk[i / 4].z : xk[i / 4].w);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint64_t yj = j & 1 ? yk[j / 2].y : yk[j / 2].x;
@@ -293,7 +300,7 @@ gemm_f32_tile_kernel(const GemmF32 p) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int e = i * 8 + h * 4;
-                store4(m0 + i / 2 * 16 + ty * 2 + i % 2, n0 + 64 * h + tx * 4,
+                store4(m0 + i / 4 * 32 + ty * 4 + i % 4, n0 + 64 * h + tx * 4,
                        make_float4(s.total[e][tid], s.total[e + 1][tid], s.total[e + 2][tid], s.total[e + 3][tid]));
             }
         return;
@@ -304,7 +311,7 @@ gemm_f32_tile_kernel(const GemmF32 p) {
     __syncthreads();
     float* s_part = &s.part[0][0];                              // [64][128]
 #pragma unroll
-    for (int q = 0; q < 16; ++q) *reinterpret_cast<float4*>(s_part + (q / 4 * 16 + ty * 2 + q / 2 % 2) * kTileN + 64 * (q & 1) + tx * 4) = own[q];
+    for (int q = 0; q < 16; ++q) *reinterpret_cast<float4*>(s_part + (q / 8 * 32 + ty * 4 + q / 2 % 4) * kTileN + 64 * (q & 1) + tx * 4) = own[q];
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     for (int e = group * kTileThreads + tid; e < kTileM * kTileN / 4; e += kTileThreads * groups) {
