@@ -121,7 +121,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cib_attention_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P],
         "cib_gemm_skinny": [_P, _I, _I, _I, _P, _I, _P, _P, _I, _P, _I, _F, _P, _P, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P, _I, _P, _P, _P],
         "cib_gemm_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
-        "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
+        "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, ctypes.c_longlong, _I, _P, _P],
         "cib_gemm_generic": [_P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P],
         "cib_decode_merges_in_cluster": [ctypes.c_longlong, _I, _I, _I, _I],
         "cib_sample": [_P, _I, _I, _I, _P, _P, _P],
@@ -1034,10 +1034,16 @@ def gemm_wstream_supports(M: int, N: int, K: int) -> bool:
     return bool(library().cib_gemm_wstream_supports(M, N, K))
 
 
-def gemm_wstream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, silu_pair: bool = False) -> None:
+def gemm_wstream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, silu_pair: bool = False, *, squares: torch.Tensor | None = None,
+                 eps: float = 0.0, stream: torch.Tensor | None = None, gain: torch.Tensor | None = None,
+                 squares_out: torch.Tensor | None = None, warm: torch.Tensor | None = None) -> None:
     """out[M, N] = a[M, K] @ w[N, K]^T for up to 128 rows on tcgen05 tensor cores with the weights as the streamed
     128-row operand (bfloat16 in, bfloat16 or float32 out).  ``silu_pair``: w holds N/2 gate rows then N/2 up rows and
-    out[M, N/2] = silu(gate) * up (bfloat16)."""
+    out[M, N/2] = silu(gate) * up (bfloat16).
+
+    A norm between two products is shared by them as in ``gemm_skinny``: ``stream`` (float32 [M, N], updated in place by the
+    product), ``gain`` and ``squares_out`` (float32 [M, ceil(N / 32)]) leave out = bfloat16(stream * gain); ``squares`` and
+    ``eps`` apply the rest of the norm to the product after it.  ``warm``: what the kernel after this one reads first."""
     M, K = a.shape
     N, K2 = w.shape
     out_cols = N // 2 if silu_pair else N
@@ -1047,11 +1053,25 @@ def gemm_wstream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, silu_pair:
         raise KernelError("gemm_wstream: rows must be dense and out bfloat16 or float32")
     if silu_pair and (N % 2 or out.dtype != torch.bfloat16):
         raise KernelError("gemm_wstream: the gated epilogue needs an even N and a bfloat16 result")
-    epilogue = 2 if silu_pair else (1 if out.dtype == torch.float32 else 0)
+    if squares is not None and (squares.dtype != torch.float32 or squares.dim() != 2 or squares.shape[0] != M or not squares.is_contiguous()):
+        raise KernelError("gemm_wstream: squares must be contiguous float32 [M, parts]")
+    if stream is not None:
+        if silu_pair or out.dtype != torch.bfloat16 or gain is None or gain.numel() != N:
+            raise KernelError("gemm_wstream: a stream goes with bfloat16 out and N gains")
+        if stream.dtype != torch.float32 or stream.shape != (M, N) or not stream.is_contiguous():
+            raise KernelError("gemm_wstream: stream must be contiguous float32 [M, N]")
+        if squares_out is None or squares_out.dtype != torch.float32 or squares_out.shape != (M, -(-N // 32)) or not squares_out.is_contiguous():
+            raise KernelError("gemm_wstream: squares_out must be contiguous float32 [M, ceil(N / 32)]")
+    warm = _l2_hint(warm)
+    epi = 3 if stream is not None else EPILOGUE_SILU_PAIR if silu_pair else EPILOGUE_F32 if out.dtype == torch.float32 else EPILOGUE_BF16
     rc = library().cib_gemm_wstream(
         _cuda(a, "a", contiguous=False), a.stride(0), _cuda(w, "w", contiguous=False), w.stride(0),
-        _cuda(out, "out", contiguous=False), out.stride(0), epilogue, M, N, K, 1 if use_pdl else 0,
-        _error_flag(a.device).data_ptr(), _stream())
+        _cuda(out, "out", contiguous=False), out.stride(0), epi, M, N, K,
+        _cuda(squares, "squares") if squares is not None else None, squares.shape[1] if squares is not None else 0, float(eps),
+        _cuda(stream, "stream") if stream is not None else None, _cuda(gain, "gain") if gain is not None else None,
+        _code(gain, "gain") if gain is not None else 0, _cuda(squares_out, "squares_out") if squares_out is not None else None,
+        warm.data_ptr() if warm is not None else None, warm.numel() * warm.element_size() if warm is not None else 0,
+        1 if use_pdl else 0, _error_flag(a.device).data_ptr(), _stream())
     _check(rc, "gemm_wstream")
     note_flagged_launch()
     _count()

@@ -1,12 +1,13 @@
 """Choice of the bfloat16 matrix-product kernel for a given shape.
 
-* up to 16 rows (decode steps), weights under 24 MB (every matrix of the Qwen3-0.6B layer sizes): the few-rows kernel
-  (``gemm_skinny``), weights streamed once through registers, with a norm shared by the products on its two sides (or in its
-  prologue) and the SiLU gate in its epilogue; larger weights (the 8B and 32B layer sizes) go to the library, which measured faster on all of them —
-  6144 x 4096: 11.5 us against 19.5 (few-rows) and 21.6 (weight-streaming); 24576 x 4096: 34.3 against 43.5 and 46.0;
-  10240 x 5120: 22.3 against 39.6 and 33.8; 5120 x 25600: 44 against 69 (weight-streaming); 151936 x 4096: 198 against
-  216 and 204 — except long K with few output features (4096 x 12288: weight-streaming tcgen05 kernel 22.4 us, library
-  32.2), which stay on ``gemm_wstream``;
+* up to 64 rows (decode steps): the few-rows kernel (``gemm_skinny``: weights streamed once through registers) for up to 16
+  rows of weights under 24 MB and K up to 4 096, else the weight-streaming tcgen05 kernel (``gemm_wstream``).  Both share a norm
+  with the product on its other side and have the SiLU gate in their epilogue.  A decode step of the 8B layer sizes (eight layers) with the
+  large products on ``gemm_wstream`` takes 839 / 903 / 896 / 1 006 us for 1 / 6 / 12 / 32 rows, with them on the library 963 / 999 / 990 /
+  1 046; of the 0.6B sizes 1 077 us for 20 rows at 700 keys and 1 386 for 64 at 300 (1 326 and 1 451).  One product, weights cold, library / streamed
+  / few rows: 8 x 4 096 x 4 096 11.9 / 7.8 / 8.6 us, 8 x 151 936 x 4 096 204 / 182 / 200, 8 x 24 576 x 4 096 34.4 / 35.5 / 37.4, 8 x 4 096 x 1 024
+  4.8 / 4.3 / 2.5, 16 x 24 576 x 4 096 34.7 / 35.9 / 47.7; 64 x 6 144 x 4 096 11.3 / 13.5, so from 33 rows on products that share neither a norm
+  nor a gate go to the library;
 * 128 rows and more (prompt portions): the tcgen05 / TMA / TMEM kernel (``gemm_tcgen05``), with the SiLU gate in its
   epilogue for the gate/up projection — where the product has at least ``TCGEN05_MIN_TILES`` output tiles of
   128 x 128.  With fewer, every CTA walks the whole of K alone and the library, which splits K over more CTAs, measured
@@ -15,9 +16,8 @@
   calls cuBLAS for every projection, csrc/ops/projection.cu:32-44), or the FMA kernel for shapes cuBLAS's
   tensor-core paths do not take.
 
-``CUINFER_B200_GEMM=cublas`` sends every prompt-sized product to the library, ``CUINFER_B200_GEMM=tcgen05`` every one
-that the kernel takes to the kernel, ``CUINFER_B200_GEMM=own`` keeps the decode steps' large products on this package's
-kernels as well (for comparisons).
+``CUINFER_B200_GEMM=cublas`` sends every product of more than 16 rows to the library, ``CUINFER_B200_GEMM=tcgen05`` every
+prompt-sized one that the kernel takes to the kernel (for comparisons).
 """
 from __future__ import annotations
 
@@ -34,24 +34,28 @@ torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 TCGEN05_MIN_ROWS = 128
 TCGEN05_MIN_TILES = 296          # output tiles of 128 x 128 from which the tcgen05 kernel is chosen over the library
 FEW_ROWS = 16
+MANY_ROWS = 64                   # rows up to which the weight-streaming kernel is taken, and of products on their own
+MANY_ROWS_PLAIN = 32
 FUSED_NORM_MAX_K = 2048          # the norm prologue keeps 32-bit rows of all of K in shared memory: beyond this one CTA per SM
-FEW_ROWS_LONG_K = 4096           # above it the few-rows kernel is down to one CTA per SM (measured: 1.9 TB/s at K = 12288)
-FEW_ROWS_LIBRARY_BYTES = 24 << 20   # weights from this size on: the library product, unless K is long and N small
-WSTREAM_MIN_K, WSTREAM_MAX_N = 12288, 4096
+FEW_ROWS_LONG_K = 4096           # the few-rows kernel up to here, and for weights below
+FEW_ROWS_MAX_BYTES = 24 << 20
 _FORCE_CUBLAS = os.environ.get("CUINFER_B200_GEMM", "") == "cublas"
 _FORCE_TCGEN05 = os.environ.get("CUINFER_B200_GEMM", "") == "tcgen05"
-_FORCE_OWN = os.environ.get("CUINFER_B200_GEMM", "") in ("own", "tcgen05")       # decode steps too stay on this package's kernels
 
 
 def few_rows_kernel(M: int, N: int, K: int) -> str:
-    """Which kernel multiplies ``M <= 16`` rows with an [N, K] weight: "skinny", "wstream" or "library"."""
-    if N * K * 2 >= FEW_ROWS_LIBRARY_BYTES and not _FORCE_OWN:
-        if K >= WSTREAM_MIN_K and N <= WSTREAM_MAX_N and kernels.gemm_wstream_supports(M, N, K):
-            return "wstream"
-        return "library"
-    if K > FEW_ROWS_LONG_K and kernels.gemm_wstream_supports(M, N, K):
+    """Which kernel multiplies ``M <= 64`` rows with an [N, K] weight: "skinny", "wstream" or "library"."""
+    if M <= FEW_ROWS and N * K * 2 < FEW_ROWS_MAX_BYTES and K <= FEW_ROWS_LONG_K:
+        return "skinny"
+    if kernels.gemm_wstream_supports(M, N, K) and not (M > FEW_ROWS and _FORCE_CUBLAS):
         return "wstream"
-    return "skinny"
+    return "skinny" if M <= FEW_ROWS else "library"
+
+
+def wstream_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether the rows of both operands lie as ``gemm_wstream`` fetches them: apart, and on 16-byte boundaries."""
+    K = x.shape[1]
+    return all(t.stride(1) == 1 and t.stride(0) >= K and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (x, weight))
 
 
 def takes_tcgen05(x: torch.Tensor, weight: torch.Tensor, fused: bool = False) -> bool:
@@ -83,9 +87,9 @@ def bf16_matmul_nt(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> 
     """out[M, N] = x[M, K] @ weight[N, K]^T; x and weight bfloat16, out bfloat16 or float32."""
     M, K = x.shape
     N = weight.shape[0]
-    if M <= FEW_ROWS and weight.stride(1) == 1 and x.stride(1) == 1:
+    if M <= MANY_ROWS_PLAIN and weight.stride(1) == 1 and x.stride(1) == 1:
         choice = few_rows_kernel(M, N, K)
-        if choice == "wstream" and x.stride(0) % 8 == 0 and weight.stride(0) % 8 == 0:
+        if choice == "wstream" and wstream_takes(x, weight) and out.stride(1) == 1 and out.stride(0) >= N:
             kernels.gemm_wstream(x, weight, out)
             return
         if choice == "skinny" and weight.is_contiguous() and kernels.gemm_skinny_supports(M, N, K):

@@ -146,27 +146,40 @@ class Linear:
 
     def defer(self, x: torch.Tensor):
         """The product of ``x`` as rows, or unlaunched where the norm after it may share its kernel (see ``into_stream``)."""
-        return DeferredProduct(self, x) if self._takes_skinny(x.shape[0]) and x.dtype == torch.bfloat16 else self.forward(x)
+        if x.dtype == torch.bfloat16 and self.weight is not None and self._few_rows_kernel(x.shape[0]) != "library":
+            return DeferredProduct(self, x)
+        return self.forward(x)
 
     def into_stream(self, x: torch.Tensor, residual: torch.Tensor, gain: torch.Tensor) -> Optional[tuple]:
         """Add the product of ``x`` to the 32-bit ``residual`` in place; ``(rows, squares)``: the new residual times ``gain`` in
-        bfloat16 and the sums of its squares over 16 columns each, from the product's own kernel.  None where it does not
+        bfloat16 and parts of the sums of its squares, from the product's own kernel.  None where it does not
         take the shape (nothing has happened then)."""
         M, N = residual.shape
-        if (not self._takes_skinny(M) or x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16
-                or not residual.is_contiguous() or gain.numel() != N or self.weight.shape[0] != N):
+        from . import gemm_dispatch
+        if (x.dtype != torch.bfloat16 or not gemm_dispatch.wstream_takes(x, self.weight) or not residual.is_contiguous()
+                or gain.numel() != N or self.weight.shape[0] != N):
             return None
+        kernel = self._few_rows_kernel(M)
+        if kernel == "library":
+            return None
+        cols = 16 if kernel == "skinny" else 32
         rows = torch.empty((M, N), dtype=torch.bfloat16, device=residual.device)
-        squares = torch.empty((M, -(-N // 16)), dtype=torch.float32, device=residual.device)
-        kernels.gemm_skinny(self.weight, rows, act=x, norm_weight=gain, stream=residual, squares_out=squares, warm=self.warm_next)
+        squares = torch.empty((M, -(-N // cols)), dtype=torch.float32, device=residual.device)
+        if kernel == "skinny":
+            kernels.gemm_skinny(self.weight, rows, act=x, norm_weight=gain, stream=residual, squares_out=squares, warm=self.warm_next)
+        else:
+            kernels.gemm_wstream(x, self.weight, rows, stream=residual, gain=gain, squares_out=squares, warm=self.warm_next)
         return rows, squares
 
-    def _takes_skinny(self, M: int) -> bool:
-        """Whether ``M`` plain rows run on the few-rows kernel."""
+    def _few_rows_kernel(self, M: int) -> str:
+        """Which kernel multiplies ``M`` plain rows (``gemm_dispatch.few_rows_kernel``), "library" for more than 64."""
         from . import gemm_dispatch
         w = self.weight
-        return (w is not None and w.dtype == torch.bfloat16 and w.is_contiguous() and 0 < M <= gemm_dispatch.FEW_ROWS
-                and gemm_dispatch.few_rows_kernel(M, *w.shape) == "skinny" and kernels.gemm_skinny_supports(M, *w.shape))
+        if w is None or w.dtype != torch.bfloat16 or not w.is_contiguous() or not 0 < M <= gemm_dispatch.MANY_ROWS:
+            return "library"
+        choice = gemm_dispatch.few_rows_kernel(M, *w.shape)
+        takes = {"skinny": kernels.gemm_skinny_supports, "wstream": kernels.gemm_wstream_supports}.get(choice)
+        return choice if takes is not None and takes(M, *w.shape) and w.stride(0) % 8 == 0 else "library"
 
     def _forward_skinny(self, x, out_dtype, silu_pair) -> Optional[torch.Tensor]:
         """The few-rows kernel with the norm in its prologue and/or the gate in its epilogue, when it takes
@@ -177,24 +190,27 @@ class Linear:
         lazy = isinstance(x, LazyNorm)
         M = x.shape[0]
         N, K = w.shape
-        if M == 0 or M > 16:
+        from . import gemm_dispatch
+        if M == 0 or M > gemm_dispatch.MANY_ROWS:
             return None
         out_dtype = out_dtype or torch.bfloat16
         if silu_pair and out_dtype != torch.bfloat16:
             return None
         out_cols = N // 2 if silu_pair else N
-        from . import gemm_dispatch
         choice = gemm_dispatch.few_rows_kernel(M, N, K)
         if choice == "library":
             return None           # the library product (and the activation kernel after it) in forward()
         if choice == "wstream":
-            # long K: the weight-streaming kernel (no norm prologue; the gate is in its epilogue)
-            rows = x.materialize() if lazy else x
-            if (silu_pair is not True or rows.dtype != torch.bfloat16 or rows.stride(1) != 1 or rows.stride(0) % 8 or w.stride(0) % 8
-                    or not kernels.gemm_wstream_supports(M, N, K)):
+            if self._few_rows_kernel(M) != "wstream" or silu_pair == "gelu_tanh" or not (lazy or silu_pair):
+                return None           # plain rows: matmul_nt decides
+            carried = x.carried() if lazy else None
+            if carried is None and not silu_pair and M > gemm_dispatch.MANY_ROWS_PLAIN:
+                return None           # nothing shared
+            rows, squares, eps = carried or (x.materialize() if lazy else x, None, 0.0)
+            if rows.dtype != torch.bfloat16 or not gemm_dispatch.wstream_takes(rows, w):
                 return None
-            out = torch.empty((M, out_cols), dtype=torch.bfloat16, device=w.device)
-            kernels.gemm_wstream(rows, w, out, silu_pair=True)
+            out = torch.empty((M, out_cols), dtype=out_dtype, device=w.device)
+            kernels.gemm_wstream(rows, w, out, silu_pair=bool(silu_pair), squares=squares, eps=eps, warm=self.warm_next)
             return out
         carried = x.carried() if lazy and kernels.gemm_skinny_supports(M, N, K) else None
         if carried is not None:
