@@ -19,8 +19,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int encode_tensor_map_bf16_2d(void* map, const void* base, unsigned long long rows, int cols, int ld, int box_cols,
-                              int box_rows, const char* who) {
+static int encode_tensor_map_2d(CUtensorMapDataType type, int width, void* map, const void* base, unsigned long long rows, int cols,
+                                int ld, int box_cols, int box_rows, const char* who) {
     // the driver's encoder, looked up through the runtime so that nothing links against the driver library
     static EncodeTiledFn fn = nullptr;
     if (fn == nullptr) {
@@ -31,15 +31,25 @@ int encode_tensor_map_bf16_2d(void* map, const void* base, unsigned long long ro
     }
     CIB_REQUIRE(fn != nullptr, "%s: the driver does not give cuTensorMapEncodeTiled", who);
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * width};
     cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(reinterpret_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims,
+    CUresult r = fn(reinterpret_cast<CUtensorMap*>(map), type, 2, const_cast<void*>(base), dims,
                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     CIB_REQUIRE(r == CUDA_SUCCESS, "%s: cuTensorMapEncodeTiled failed with code %d (rows=%llu cols=%d ld=%d box=%dx%d)", who, (int)r,
                 rows, cols, ld, box_cols, box_rows);
     return 0;
+}
+
+int encode_tensor_map_bf16_2d(void* map, const void* base, unsigned long long rows, int cols, int ld, int box_cols,
+                              int box_rows, const char* who) {
+    return encode_tensor_map_2d(CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, map, base, rows, cols, ld, box_cols, box_rows, who);
+}
+
+int encode_tensor_map_f32_2d(void* map, const void* base, unsigned long long rows, int cols, int ld, int box_cols,
+                             int box_rows, const char* who) {
+    return encode_tensor_map_2d(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, map, base, rows, cols, ld, box_cols, box_rows, who);
 }
 
 }  // namespace cib

@@ -33,6 +33,9 @@ bool prompt_pdl();
 // issue TMA copies include the driver header).  0, or -1 with the error text set.
 int encode_tensor_map_bf16_2d(void* map, const void* base, unsigned long long rows, int cols, int ld, int box_cols,
                               int box_rows, const char* who);
+// The same over 32-bit rows.
+int encode_tensor_map_f32_2d(void* map, const void* base, unsigned long long rows, int cols, int ld, int box_cols,
+                             int box_rows, const char* who);
 
 // The larger limit on dynamic shared memory is a property of a kernel on ONE device: it is set the first time the kernel
 // is launched on each device, under a mutex (the entry points may be called from several threads).  A launcher keeps one

@@ -120,7 +120,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cib_paged_attention_prefill": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
         "cib_attention_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P],
         "cib_gemm_skinny": [_P, _I, _I, _I, _P, _I, _P, _P, _I, _P, _I, _F, _P, _P, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P, _I, _P, _P, _P],
-        "cib_gemm_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
+        "cib_gemm_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, _P],
         "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, ctypes.c_longlong, _I, _P, _P],
         "cib_gemm_generic": [_P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P],
         "cib_decode_merges_in_cluster": [ctypes.c_longlong, _I, _I, _I, _I],
@@ -151,6 +151,8 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.cib_paged_attention_decode_supports.restype = _I
     lib.cib_gemm_tcgen05_supports.argtypes = [_I, _I, _I]
     lib.cib_gemm_tcgen05_supports.restype = _I
+    lib.cib_gemm_tcgen05_stream_cols.argtypes = [_I, _I, _I]
+    lib.cib_gemm_tcgen05_stream_cols.restype = _I
     lib.cib_attention_tcgen05_supports.argtypes = [_I, _I, _I, _I]
     lib.cib_attention_tcgen05_supports.restype = _I
     lib.cib_gemm_wstream_supports.argtypes = [_I, _I, _I]
@@ -1081,9 +1083,21 @@ def gemm_tcgen05_supports(M: int, N: int, K: int) -> bool:
     return bool(library().cib_gemm_tcgen05_supports(M, N, K))
 
 
-def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, silu_pair: bool = False) -> None:
+def gemm_tcgen05_stream_cols(M: int, N: int, K: int) -> int:
+    """Columns of a tile of the product that adds to the residual (``gemm_tcgen05(stream=...)``), 0 where it does not take the
+    shape."""
+    return int(library().cib_gemm_tcgen05_stream_cols(M, N, K))
+
+
+def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, silu_pair: bool = False, *, squares: torch.Tensor | None = None,
+                 eps: float = 0.0, stream: torch.Tensor | None = None, gain: torch.Tensor | None = None,
+                 squares_out: torch.Tensor | None = None) -> None:
     """out[M, N] = a[M, K] @ w[N, K]^T on tcgen05 tensor cores (bfloat16 in, bfloat16 or float32 out).
-    ``silu_pair``: w holds N/2 gate rows then N/2 up rows and out[M, N/2] = silu(gate) * up (bfloat16)."""
+    ``silu_pair``: w holds N/2 gate rows then N/2 up rows and out[M, N/2] = silu(gate) * up (bfloat16).
+
+    A norm between two products is shared by them as in ``gemm_skinny``: ``stream`` (float32 [M, N], updated in place by the
+    product), ``gain`` and ``squares_out`` (float32 [M, ceil(N / gemm_tcgen05_stream_cols)]) leave out = bfloat16(stream * gain);
+    ``squares`` and ``eps`` apply the rest of the norm to the product after it."""
     M, K = a.shape
     N, K2 = w.shape
     out_cols = N // 2 if silu_pair else N
@@ -1093,10 +1107,24 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, silu_pair:
         raise KernelError("gemm_tcgen05: rows must be dense and out bfloat16 or float32")
     if silu_pair and (N % 2 or out.dtype != torch.bfloat16 or out.stride(0) % 8 or out.data_ptr() % 16):
         raise KernelError("gemm_tcgen05: the gated epilogue needs an even N and 16-byte aligned bfloat16 rows")
+    if squares is not None and (squares.dtype != torch.float32 or squares.dim() != 2 or squares.shape[0] != M or not squares.is_contiguous()):
+        raise KernelError("gemm_tcgen05: squares must be contiguous float32 [M, parts]")
+    if stream is not None:
+        cols = gemm_tcgen05_stream_cols(M, N, K)
+        if not cols or silu_pair or out.dtype != torch.bfloat16 or gain is None or gain.numel() != N:
+            raise KernelError(f"gemm_tcgen05: a stream of {M} rows of {N} (K={K}) is not taken, or without bfloat16 out or {N} gains")
+        if stream.dtype != torch.float32 or stream.shape != (M, N) or not stream.is_contiguous():
+            raise KernelError("gemm_tcgen05: stream must be contiguous float32 [M, N]")
+        if squares_out is None or squares_out.dtype != torch.float32 or squares_out.shape != (M, -(-N // cols)) or not squares_out.is_contiguous():
+            raise KernelError(f"gemm_tcgen05: squares_out must be contiguous float32 [M, {-(-N // cols)}]")
     rc = library().cib_gemm_tcgen05(
         _cuda(a, "a", contiguous=False), a.stride(0), _cuda(w, "w", contiguous=False), w.stride(0),
         _cuda(out, "out", contiguous=False), out.stride(0), 1 if out.dtype == torch.float32 else 0,
-        (2 if silu_pair == "gelu_tanh" else 1) if silu_pair else 0, M, N, K, _error_flag(a.device).data_ptr(), _stream())
+        (2 if silu_pair == "gelu_tanh" else 1) if silu_pair else 0, M, N, K,
+        _cuda(squares, "squares") if squares is not None else None, squares.shape[1] if squares is not None else 0, float(eps),
+        _cuda(stream, "stream") if stream is not None else None, _cuda(gain, "gain") if gain is not None else None,
+        _code(gain, "gain") if gain is not None else 0, _cuda(squares_out, "squares_out") if squares_out is not None else None,
+        _error_flag(a.device).data_ptr(), _stream())
     _check(rc, "gemm_tcgen05")
     note_flagged_launch()
     _count()

@@ -33,6 +33,7 @@ torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 TCGEN05_MIN_ROWS = 128
 TCGEN05_MIN_TILES = 296          # output tiles of 128 x 128 from which the tcgen05 kernel is chosen over the library
+STREAM_MIN_ROWS = 2048           # from here on a product adds to the residual itself and leaves the next norm to its reader
 FEW_ROWS = 16
 MANY_ROWS = 64                   # rows up to which the weight-streaming kernel is taken, and of products on their own
 MANY_ROWS_PLAIN = 32
@@ -47,6 +48,8 @@ def few_rows_kernel(M: int, N: int, K: int) -> str:
     """Which kernel multiplies ``M <= 64`` rows with an [N, K] weight: "skinny", "wstream" or "library"."""
     if M <= FEW_ROWS and N * K * 2 < FEW_ROWS_MAX_BYTES and K <= FEW_ROWS_LONG_K:
         return "skinny"
+    if M > MANY_ROWS_PLAIN and N * K * 2 >= FEW_ROWS_MAX_BYTES:
+        return "library"          # (8B sizes, eight layers, 64 rows: a step 1 330 us on the library, 1 387 streamed; 48 rows the same on both)
     if kernels.gemm_wstream_supports(M, N, K) and not (M > FEW_ROWS and _FORCE_CUBLAS):
         return "wstream"
     return "skinny" if M <= FEW_ROWS else "library"
@@ -61,10 +64,14 @@ def wstream_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
 def takes_tcgen05(x: torch.Tensor, weight: torch.Tensor, fused: bool = False) -> bool:
     """``fused``: the product carries an epilogue (the SiLU gate) that the library call would need another kernel for;
     it stays on the tcgen05 kernel whatever its size."""
-    M, K = x.shape
-    N = weight.shape[0]
-    if not (M >= TCGEN05_MIN_ROWS and not _FORCE_CUBLAS and x.stride(1) == 1 and weight.stride(1) == 1
-            and x.stride(0) % 8 == 0 and weight.stride(0) % 8 == 0 and kernels.gemm_tcgen05_supports(M, N, K)):
+    return x.stride(1) == 1 and x.stride(0) % 8 == 0 and shape_takes_tcgen05(x.shape[0], weight, fused)
+
+
+def shape_takes_tcgen05(M: int, weight: torch.Tensor, fused: bool = False) -> bool:
+    """``takes_tcgen05`` for ``M`` dense rows."""
+    N, K = weight.shape
+    if not (M >= TCGEN05_MIN_ROWS and not _FORCE_CUBLAS and weight.stride(1) == 1 and weight.stride(0) % 8 == 0
+            and kernels.gemm_tcgen05_supports(M, N, K)):
         return False
     if fused or _FORCE_TCGEN05 or K % 8 or N % 8:
         return True

@@ -131,6 +131,9 @@ class Linear:
         if fused is not None:
             return fused
         if isinstance(x, LazyNorm):
+            y = self._forward_carried(x, out_dtype, silu_pair)
+            if y is not None:
+                return y
             x = x.materialize()
         if silu_pair and x.dtype == torch.bfloat16 and x.shape[0] > 0:
             from . import gemm_dispatch
@@ -144,15 +147,32 @@ class Linear:
         kernels.silu_mul(y, act, gelu=silu_pair == "gelu_tanh")
         return act
 
+    def _forward_carried(self, x: LazyNorm, out_dtype, silu_pair) -> Optional[torch.Tensor]:
+        """The prompt-sized product of rows that carry their norm; None where there are none or another kernel would take them."""
+        from . import gemm_dispatch
+        w = self.weight
+        M, K = x.shape
+        out_cols = w.shape[0] // 2 if silu_pair else w.shape[0]
+        if (M < gemm_dispatch.STREAM_MIN_ROWS or w.dtype != torch.bfloat16 or w.shape[1] != K or (silu_pair and w.shape[0] % 16)
+                or not gemm_dispatch.shape_takes_tcgen05(M, w, fused=bool(silu_pair))):
+            return None
+        carried = x.carried()
+        if carried is None:
+            return None
+        rows, squares, eps = carried
+        out = torch.empty((M, out_cols), dtype=torch.bfloat16 if silu_pair else out_dtype or torch.bfloat16, device=w.device)
+        kernels.gemm_tcgen05(rows, w, out, silu_pair=silu_pair, squares=squares, eps=eps)
+        return out
+
     def defer(self, x: torch.Tensor):
         """The product of ``x`` as rows, or unlaunched where the norm after it may share its kernel (see ``into_stream``)."""
-        if x.dtype == torch.bfloat16 and self.weight is not None and self._few_rows_kernel(x.shape[0]) != "library":
+        if x.dtype == torch.bfloat16 and self.weight is not None and (self._few_rows_kernel(x.shape[0]) != "library" or self._stream_cols(x)):
             return DeferredProduct(self, x)
         return self.forward(x)
 
     def into_stream(self, x: torch.Tensor, residual: torch.Tensor, gain: torch.Tensor) -> Optional[tuple]:
         """Add the product of ``x`` to the 32-bit ``residual`` in place; ``(rows, squares)``: the new residual times ``gain`` in
-        bfloat16 and parts of the sums of its squares, from the product's own kernel.  None where it does not
+        bfloat16 and the sums of its squares over 16 columns each, from the product's own kernel.  None where it does not
         take the shape (nothing has happened then)."""
         M, N = residual.shape
         from . import gemm_dispatch
@@ -160,16 +180,26 @@ class Linear:
                 or gain.numel() != N or self.weight.shape[0] != N):
             return None
         kernel = self._few_rows_kernel(M)
-        if kernel == "library":
+        cols = {"skinny": 16, "wstream": 32}.get(kernel) or self._stream_cols(x)
+        if not cols:
             return None
-        cols = 16 if kernel == "skinny" else 32
         rows = torch.empty((M, N), dtype=torch.bfloat16, device=residual.device)
         squares = torch.empty((M, -(-N // cols)), dtype=torch.float32, device=residual.device)
         if kernel == "skinny":
             kernels.gemm_skinny(self.weight, rows, act=x, norm_weight=gain, stream=residual, squares_out=squares, warm=self.warm_next)
-        else:
+        elif kernel == "wstream":
             kernels.gemm_wstream(x, self.weight, rows, stream=residual, gain=gain, squares_out=squares, warm=self.warm_next)
+        else:
+            kernels.gemm_tcgen05(x, self.weight, rows, stream=residual, gain=gain, squares_out=squares)
         return rows, squares
+
+    def _stream_cols(self, x: torch.Tensor) -> int:
+        """``kernels.gemm_tcgen05_stream_cols`` where the prompt-sized product of ``x`` may add to the residual, else 0."""
+        from . import gemm_dispatch
+        w = self.weight
+        if x.shape[0] < gemm_dispatch.STREAM_MIN_ROWS or w.dtype != torch.bfloat16 or not gemm_dispatch.takes_tcgen05(x, w, fused=True):
+            return 0
+        return kernels.gemm_tcgen05_stream_cols(x.shape[0], *w.shape)
 
     def _few_rows_kernel(self, M: int) -> str:
         """Which kernel multiplies ``M`` plain rows (``gemm_dispatch.few_rows_kernel``), "library" for more than 64."""

@@ -341,24 +341,26 @@ def test_gemm_skinny_with_norm_and_gated_epilogue(M, H, I, pending_dtype):
 @pytest.mark.parametrize("kind, M, N, K, I", [
     ("skinny", 1, 1024, 2048, 256), ("skinny", 8, 1024, 3072, 272), ("skinny", 9, 1000, 96, 40), ("skinny", 16, 48, 5120, 1024),
     ("skinny", 5, 4800, 1024, 520), ("wstream", 1, 4096, 4096, 64), ("wstream", 16, 1024, 3072, 96), ("wstream", 17, 1000, 200, 1536),
-    ("wstream", 33, 1024, 2048, 1536), ("wstream", 64, 19200, 72, 40), ("wstream", 100, 1024, 1024, 9600)])
+    ("wstream", 33, 1024, 2048, 1536), ("wstream", 64, 19200, 72, 40), ("wstream", 100, 1024, 1024, 9600), ("tcgen05", 300, 7680, 72, 128),
+    ("tcgen05", 2400, 1000, 512, 136), ("tcgen05", 2561, 1024, 2048, 1536), ("tcgen05", 600, 3208, 200, 64)])
 @pytest.mark.parametrize("gain_dtype", [torch.bfloat16, torch.float32])
 def test_two_products_share_a_norm(kind, M, N, K, I, gain_dtype):
     """A product that adds to the residual and leaves its rows with the next norm's gains, then products that apply the rest of
     the norm to their results: the few-rows kernel (with and without clusters, a slice of K in one, two or more rounds), the
-    weight-streaming one (K in 1 to 8 CTAs of a cluster, shares of K without a step, every row tile); ragged edges."""
+    weight-streaming one (K in 1 to 8 CTAs of a cluster, shares of K without a step, every row tile), and prompt sizes (tiles of
+    128 and 256 columns); ragged edges."""
     k = _k()
     x, w = rand(M, K, seed=60, dtype=torch.bfloat16), rand(N, K, seed=61, scale=0.05, dtype=torch.bfloat16)
     res, gain, eps = rand(M, N, seed=62, scale=2.0), (1 + rand(N, seed=63, scale=0.2)).to(gain_dtype), 1e-5
     w2 = rand(2 * I, N, seed=64, scale=0.05, dtype=torch.bfloat16)
     want = res.double() + x.double() @ w.double().T
     stream, rows = res.to(DEV), torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV)
-    cols = {"skinny": 16, "wstream": 32}[kind]
+    cols = {"skinny": 16, "wstream": 32}.get(kind) or k.gemm_tcgen05_stream_cols(M, N, K)
     squares = torch.full((M, -(-N // cols)), 7.0, device=DEV)
     if kind == "skinny":
         k.gemm_skinny(w.to(DEV), rows, act=x.to(DEV), norm_weight=gain.to(DEV), stream=stream, squares_out=squares)
     else:
-        k.gemm_wstream(x.to(DEV), w.to(DEV), rows, stream=stream, gain=gain.to(DEV), squares_out=squares)
+        (k.gemm_wstream if kind == "wstream" else k.gemm_tcgen05)(x.to(DEV), w.to(DEV), rows, stream=stream, gain=gain.to(DEV), squares_out=squares)
     # a 32-bit accumulator takes 16 products a time: K / 16 additions, each off by at most 2^-23 of a sum no larger than the largest
     bound = (K / 16 + 2) * 2.0 ** -23
     close(stream, want, bound)
@@ -374,7 +376,7 @@ def test_two_products_share_a_norm(kind, M, N, K, I, gain_dtype):
             if kind == "skinny":
                 k.gemm_skinny(w2.to(DEV), out, act=rows, squares=squares, eps=eps, silu_pair=silu)
             else:
-                k.gemm_wstream(rows, w2.to(DEV), out, silu_pair=silu, squares=squares, eps=eps)
+                (k.gemm_wstream if kind == "wstream" else k.gemm_tcgen05)(rows, w2.to(DEV), out, silu_pair=silu, squares=squares, eps=eps)
             close(out, g / (1 + torch.exp(-g)) * u if silu else gu, 2e-5 if dtype == torch.float32 else 4e-3)
     k.check_error_flags(force=True)
 
