@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(kDecWarps * 32)
 paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, __nv_bfloat16* __restrict__ out,
                               int out_stride, const __nv_bfloat16* __restrict__ cache, int num_pages, int page_size,
                               const int* __restrict__ block_table, int table_stride,
-                              const int* __restrict__ seq_lens, int nq, int nkv, float scale_log2, int window,
-                              int splits, float* __restrict__ part_o, float* __restrict__ part_ml,
+                              const int* __restrict__ seq_lens, const int* __restrict__ query_start_loc, int nq, int nkv,
+                              float scale_log2, int window, int splits, float* __restrict__ part_o, float* __restrict__ part_ml,
                               int* __restrict__ counters, const __grid_constant__ CUtensorMap kv_map,
                               int* __restrict__ error_flag, const void* __restrict__ warm, unsigned long long warm_bytes,
                               int inbox_offset) {
@@ -154,6 +154,15 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     const int quad = lane & 3, qrow = lane >> 2;
 
     const int seq_len = seq_lens[r];
+    // a step of several kinds: this kernel takes the requests that bring one token, whose row is the request's first
+    int token = r;
+    if (query_start_loc != nullptr) {
+        token = query_start_loc[r];
+        if (query_start_loc[r + 1] - token != 1) {
+            griddep_wait();          // (a launch none of whose CTAs waits would be over before the kernel in front of it)
+            return;
+        }
+    }
     // (while that load is on its way)
     if (TMA) {
         if (threadIdx.x == 0) {
@@ -243,7 +252,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
     // ---- query fragments: rows 0..g-1 are the heads of this kv head, the rest are zero ----
     uint32_t qf[D / 16][4];
     {
-        const __nv_bfloat16* qp = q + (size_t)r * q_stride + (size_t)kvh * g * D;
+        const __nv_bfloat16* qp = q + (size_t)token * q_stride + (size_t)kvh * g * D;
 #pragma unroll
         for (int kt = 0; kt < D / 16; ++kt) {
             const int c0 = kt * 16 + quad * 2;
@@ -416,7 +425,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
             }
         }
         if (alone) {
-            out[(size_t)r * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+            out[(size_t)token * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
         } else if (CL) {
             inbox_o[row * D + dim] = O;
             if (dim == 0) {
@@ -454,7 +463,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
                 L = fmaf(all_ml[(sp * g + row) * 2 + 1], f, L);
                 O = fmaf(all_o[((size_t)sp * g + row) * D + dim], f, O);
             }
-            out[(size_t)r * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+            out[(size_t)token * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
         }
         return;
     }
@@ -514,7 +523,7 @@ paged_attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,
         }
         if (active - sp > 4) O = add_last_splits<16>(O, part_o + ((base + sp) * g + row) * D + dim, (size_t)g * D, sm_w + row * active + sp, active - sp);
         else if (active > sp) O = add_last_splits<4>(O, part_o + ((base + sp) * g + row) * D + dim, (size_t)g * D, sm_w + row * active + sp, active - sp);
-        out[(size_t)r * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(O * sm_inv[row]);
+        out[(size_t)token * out_stride + (size_t)(kvh * g + row) * D + dim] = __float2bfloat16_rn(O * sm_inv[row]);
     }
     if (threadIdx.x == 0) counters[r * nkv + kvh] = 0;
 }
@@ -552,7 +561,7 @@ static int max_resident_clusters(int cluster_x, size_t smem) {
 template <int D>
 static int launch_decode(const void* q, int q_stride, void* out, int out_stride, const void* cache, int num_pages,
                          int page_size, const int* block_table, int table_stride, const int* seq_lens,
-                         int num_requests, int nq, int nkv, float scale, int window, int splits, float* part_o,
+                         const int* query_start_loc, int num_requests, int nq, int nkv, float scale, int window, int splits, float* part_o,
                          float* part_ml, int* counters, cudaStream_t stream, bool use_pdl = false,
                          int* error_flag = nullptr, const void* warm = nullptr, unsigned long long warm_bytes = 0) {
     const int g = nq / nkv;
@@ -592,7 +601,7 @@ static int launch_decode(const void* q, int q_stride, void* out, int out_stride,
         if (raise_smem_limit(limit, kernel, 225 * 1024, "paged_attention_decode") != 0) return cudaErrorUnknown;
         return launch_pdl_cluster(kernel, grid, dim3(kDecWarps * 32), smem, stream, use_pdl, cluster ? splits : 1,
                                   (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride,
-                                  (const __nv_bfloat16*)cache, num_pages, page_size, block_table, table_stride, seq_lens, nq,
+                                  (const __nv_bfloat16*)cache, num_pages, page_size, block_table, table_stride, seq_lens, query_start_loc, nq,
                                   nkv, scale_log2, window, splits, part_o, part_ml, counters, kv_map, error_flag, warm,
                                   warm_bytes, inbox_offset);
     };
@@ -639,7 +648,8 @@ extern "C" long long cib_paged_attention_decode_scratch_floats(int num_requests,
     return (long long)num_requests * nq * splits * (head_dim + 2);
 }
 
-// One query token per request.  `scratch` holds cib_paged_attention_decode_scratch_floats floats (unused when
+// One query token per request.  With query_start_loc [num_requests + 1] (or null) the requests bring any number of tokens: those
+// that bring one are computed (q and out then have a row for every token), the others' rows are left as they are.  `scratch` holds cib_paged_attention_decode_scratch_floats floats (unused when
 // splits == 1); `counters` holds num_requests * nkv ints that are zero before the first call (the kernel leaves
 // them zero).  `error_flag` (one zero int in device memory, or null) lets the kernel fetch the cache through TMA
 // where the geometry allows it: a copy that does not land in time sets the flag instead of hanging the kernel.
@@ -649,8 +659,8 @@ extern "C" long long cib_paged_attention_decode_scratch_floats(int num_requests,
 // instead of 17.95).
 extern "C" int cib_paged_attention_decode(const void* q, int q_stride, void* out, int out_stride, const void* cache,
                                           int num_pages, int page_size, const int* block_table, int table_stride,
-                                          const int* seq_lens, int num_requests, int nq, int nkv, int head_dim,
-                                          float scale, int window, int splits, float* scratch, int* counters,
+                                          const int* seq_lens, const int* query_start_loc, int num_requests, int nq, int nkv,
+                                          int head_dim, float scale, int window, int splits, float* scratch, int* counters,
                                           int use_pdl, int* error_flag, const void* warm, long long warm_bytes,
                                           cudaStream_t stream) {
     CIB_REQUIRE(cib_paged_attention_decode_supports(head_dim, nq, nkv),
@@ -668,9 +678,9 @@ extern "C" int cib_paged_attention_decode(const void* q, int q_stride, void* out
     if (((uintptr_t)warm % 16) != 0 || warm_bytes <= 0) { warm = nullptr; warm_bytes = 0; }
     const unsigned long long wb = (unsigned long long)warm_bytes;
     switch (head_dim) {
-        case 64: return launch_decode<64>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream, use_pdl != 0, error_flag, warm, wb);
-        case 128: return launch_decode<128>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream, use_pdl != 0, error_flag, warm, wb);
-        case 256: return launch_decode<256>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream, use_pdl != 0, error_flag, warm, wb);
+        case 64: return launch_decode<64>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, query_start_loc, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream, use_pdl != 0, error_flag, warm, wb);
+        case 128: return launch_decode<128>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, query_start_loc, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream, use_pdl != 0, error_flag, warm, wb);
+        case 256: return launch_decode<256>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, query_start_loc, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream, use_pdl != 0, error_flag, warm, wb);
     }
     return -1;
 }
@@ -744,9 +754,9 @@ extern "C" int cib_paged_attention_decode_static(const void* q, int q_stride, vo
         }
     }
     switch (head_dim) {
-        case 64: return launch_decode<64>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream);
-        case 128: return launch_decode<128>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream);
-        case 256: return launch_decode<256>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream);
+        case 64: return launch_decode<64>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, nullptr, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream);
+        case 128: return launch_decode<128>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, nullptr, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream);
+        case 256: return launch_decode<256>(q, q_stride, out, out_stride, cache, num_pages, page_size, block_table, table_stride, seq_lens, nullptr, num_requests, nq, nkv, scale, window, splits, part_o, part_ml, counters, stream);
     }
     return -1;
 }

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pages, const __nv_bfloat16* __restrict__ q, int q_stride,
                          __nv_bfloat16* __restrict__ out, int out_stride, int page_size,
                          const int* __restrict__ block_table, int table_stride, const int* __restrict__ query_start_loc,
-                         const int* __restrict__ seq_lens, int num_requests, int nq, int nkv, float scale_log2, int window,
+                         const int* __restrict__ seq_lens, int num_requests, int least_query, int nq, int nkv, float scale_log2, int window,
                          int joined, const float* __restrict__ sinks, int* __restrict__ error_flag) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -120,7 +120,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pag
         for (int r0 = 0; r0 < num_requests; r0 += 32) {
             const int r = r0 + lane;
             int tiles = 0;
-            if (r < num_requests) tiles = ((query_start_loc[r + 1] - query_start_loc[r]) * g + kM - 1) / kM;
+            if (r < num_requests) {
+                const int n = query_start_loc[r + 1] - query_start_loc[r];
+                tiles = n < least_query ? 0 : (n * g + kM - 1) / kM;
+            }
             int upto = tiles;                   // tiles of the requests r0 .. r
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -487,10 +490,11 @@ extern "C" int cib_attention_tcgen05_supports(int head_dim, int nq, int nkv, int
 
 // num_tiles = sum over requests of ceil(tokens_r * (nq / nkv) / 128), or more: CTAs that find no tile leave.  least_tiles: how many
 // of them the step has at least, which decides between the two variants (a recorded step is launched for the worst split of
-// its tokens over its requests).  error_flag: one zero int in device memory.
+// its tokens over its requests).  least_query: requests that bring fewer tokens have no tiles (1: all have; 2: those of one token are
+// left to another kernel).  error_flag: one zero int in device memory.
 extern "C" int cib_attention_tcgen05(const void* q, int q_stride, void* out, int out_stride, const void* cache, int num_pages,
                                      int page_size, const int* block_table, int table_stride, const int* query_start_loc,
-                                     const int* seq_lens, int num_requests, int num_tiles, int least_tiles, int nq, int nkv,
+                                     const int* seq_lens, int num_requests, int num_tiles, int least_tiles, int least_query, int nq, int nkv,
                                      int head_dim, float scale, int window, int joined, const float* sinks, int* error_flag,
                                      cudaStream_t stream) {
     CIB_REQUIRE(cib_attention_tcgen05_supports(head_dim, nq, nkv, page_size),
@@ -517,13 +521,13 @@ extern "C" int cib_attention_tcgen05(const void* q, int q_stride, void* out, int
     const float scale_log2 = scale * 1.4426950408889634f;
     if (wide)
         return attention_tcgen05_wide(kv_map, num_pages, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride, page_size, block_table,
-                                      table_stride, query_start_loc, seq_lens, num_requests, num_tiles, nq, nkv, scale_log2, window, joined,
+                                      table_stride, query_start_loc, seq_lens, num_requests, least_query, num_tiles, nq, nkv, scale_log2, window, joined,
                                       sinks, error_flag, stream);
     static SmemLimit limit;
     if (int rc = raise_smem_limit(limit, fa::attention_tcgen05_kernel, fa::kSmemBytes, "attention_tcgen05")) return rc;
     const cudaError_t e = launch_pdl(fa::attention_tcgen05_kernel, dim3(nkv, num_tiles), dim3(fa::kThreads), (size_t)fa::kSmemBytes, stream,
                                      prompt_pdl(), kv_map, num_pages, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, out_stride,
-                                     page_size, block_table, table_stride, query_start_loc, seq_lens, num_requests, nq, nkv, scale_log2,
+                                     page_size, block_table, table_stride, query_start_loc, seq_lens, num_requests, least_query, nq, nkv, scale_log2,
                                      window, joined, sinks, error_flag);
     CIB_REQUIRE(e == cudaSuccess, "attention_tcgen05: launch failed: %s", cudaGetErrorString(e));
     return 0;

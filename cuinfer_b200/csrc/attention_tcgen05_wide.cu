@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kThreads)
 attention_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap kv_map, int num_pages, const __nv_bfloat16* __restrict__ q, int q_stride,
                          __nv_bfloat16* __restrict__ out, int out_stride, int page_size,
                          const int* __restrict__ block_table, int table_stride, const int* __restrict__ query_start_loc,
-                         const int* __restrict__ seq_lens, int num_requests, int nq, int nkv, float scale_log2, int window,
+                         const int* __restrict__ seq_lens, int num_requests, int least_query, int nq, int nkv, float scale_log2, int window,
                          int joined, const float* __restrict__ sinks, int* __restrict__ error_flag) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -117,7 +117,10 @@ attention_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap kv_map, int nu
         for (int r0 = 0; r0 < num_requests; r0 += 32) {
             const int r = r0 + lane;
             int tiles = 0;
-            if (r < num_requests) tiles = ((query_start_loc[r + 1] - query_start_loc[r]) * g + kM - 1) / kM;
+            if (r < num_requests) {
+                const int n = query_start_loc[r + 1] - query_start_loc[r];
+                tiles = n < least_query ? 0 : (n * g + kM - 1) / kM;
+            }
             int upto = tiles;                   // tiles of the requests r0 .. r
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -519,13 +522,13 @@ attention_tcgen05_wide_kernel(const __grid_constant__ CUtensorMap kv_map, int nu
 }  // namespace fw
 int attention_tcgen05_wide(const CUtensorMap& kv_map, int num_pages, const __nv_bfloat16* q, int q_stride, __nv_bfloat16* out,
                            int out_stride, int page_size, const int* block_table, int table_stride, const int* query_start_loc,
-                           const int* seq_lens, int num_requests, int num_tiles, int nq, int nkv, float scale_log2, int window,
+                           const int* seq_lens, int num_requests, int least_query, int num_tiles, int nq, int nkv, float scale_log2, int window,
                            int joined, const float* sinks, int* error_flag, cudaStream_t stream) {
     static SmemLimit limit;
     if (int rc = raise_smem_limit(limit, fw::attention_tcgen05_wide_kernel, fw::kSmemBytes, "attention_tcgen05")) return rc;
     const cudaError_t e = launch_pdl(fw::attention_tcgen05_wide_kernel, dim3(nkv, num_tiles), dim3(fw::kThreads), (size_t)fw::kSmemBytes, stream,
                                      prompt_pdl(), kv_map, num_pages, q, q_stride, out, out_stride, page_size, block_table, table_stride,
-                                     query_start_loc, seq_lens, num_requests, nq, nkv, scale_log2, window, joined, sinks, error_flag);
+                                     query_start_loc, seq_lens, num_requests, least_query, nq, nkv, scale_log2, window, joined, sinks, error_flag);
     CIB_REQUIRE(e == cudaSuccess, "attention_tcgen05: launch failed: %s", cudaGetErrorString(e));
     return 0;
 }

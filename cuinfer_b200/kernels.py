@@ -116,9 +116,9 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cib_silu_mul": [_P, _P, _I, _I, _I, _I, _P],
         "cib_qk_norm_rope_kv_write": [_P, _I, _I, _P, _P, _P, _P, _I, _I, _F, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "cib_paged_attention_generic": [_P, _I, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
-        "cib_paged_attention_decode": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _I, _I, _I, _I, _F, _I, _I, _P, _P, _I, _P, _P, ctypes.c_longlong, _P],
+        "cib_paged_attention_decode": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _F, _I, _I, _P, _P, _I, _P, _P, ctypes.c_longlong, _P],
         "cib_paged_attention_prefill": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P],
-        "cib_attention_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P],
+        "cib_attention_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P],
         "cib_gemm_skinny": [_P, _I, _I, _I, _P, _I, _P, _P, _I, _P, _I, _F, _P, _P, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P, _I, _P, _P, _P],
         "cib_gemm_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, _P],
         "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, ctypes.c_longlong, _I, _P, _P],
@@ -664,18 +664,24 @@ def _l2_hint(warm: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
 
 def paged_attention_decode(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
                            seq_lens: torch.Tensor, num_q_heads: int, num_kv_heads: int, head_dim: int, scale: float,
-                           window: int, splits: int, tma: bool | None = None, warm: torch.Tensor | None = None) -> None:
+                           window: int, splits: int, tma: bool | None = None, warm: torch.Tensor | None = None,
+                           query_start_loc: torch.Tensor | None = None) -> None:
     """bfloat16 attention of one query token per request (``q[r, :nq*d]``) over the paged cache, the keys of
     every (request, kv head) split over ``splits`` CTAs.  Allocates the partial-result scratch with torch.
     ``tma``: let the kernel fetch the cache through TMA where the geometry allows it (default: yes).  That path
     streams faster but starts slower, so callers that know the keys per CTA pass False for short streams.
     ``warm``: a tensor that the kernel after this one reads first; the CTAs that have keys ask for their shares of it to be
-    fetched into the L2 when their stream of keys ends."""
-    R = q.shape[0]
+    fetched into the L2 when their stream of keys ends.
+    ``query_start_loc`` int32 [R + 1]: the requests of ``seq_lens`` bring any number of tokens, ``q`` and ``out`` have a row for
+    every token, and only the requests that bring one are computed (the other rows of ``out`` are left as they are)."""
+    R = q.shape[0] if query_start_loc is None else seq_lens.numel()
+    T = q.shape[0]
     warm = _l2_hint(warm)
+    if query_start_loc is not None and (query_start_loc.numel() != R + 1 or block_table.shape[0] < R):
+        raise KernelError("paged_attention_decode: query_start_loc must be [R + 1] for R requests of seq_lens and block_table")
     if q.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16:
         raise KernelError("paged_attention_decode: bfloat16 only")
-    if q.stride(1) != 1 or out.stride(1) != 1 or out.shape != (R, num_q_heads * head_dim):
+    if q.stride(1) != 1 or out.stride(1) != 1 or out.shape != (T, num_q_heads * head_dim):
         raise KernelError("paged_attention_decode: q/out rows must be dense and out [R, nq*d]")
     scratch = None
     counters = None
@@ -695,8 +701,9 @@ def paged_attention_decode(q: torch.Tensor, out: torch.Tensor, cache: torch.Tens
     rc = library().cib_paged_attention_decode(
         _cuda(q, "q", contiguous=False), q.stride(0), _cuda(out, "out", contiguous=False), out.stride(0),
         _cuda(cache, "cache"), cache.shape[0], cache.shape[3], _cuda(block_table, "block_table", torch.int32),
-        block_table.stride(0), _cuda(seq_lens, "seq_lens", torch.int32), R, num_q_heads, num_kv_heads, head_dim,
-        float(scale), int(window), int(splits), scratch.data_ptr() if scratch is not None else None,
+        block_table.stride(0), _cuda(seq_lens, "seq_lens", torch.int32),
+        _cuda(query_start_loc, "query_start_loc", torch.int32) if query_start_loc is not None else None, R, num_q_heads, num_kv_heads,
+        head_dim, float(scale), int(window), int(splits), scratch.data_ptr() if scratch is not None else None,
         counters.data_ptr() if counters is not None else None, 1 if use_pdl else 0,
         _error_flag(q.device).data_ptr() if decode_tma and tma is not False else None,
         warm.data_ptr() if warm is not None else None, warm.numel() * warm.element_size() if warm is not None else 0,
@@ -1000,13 +1007,14 @@ def attention_tcgen05_supports(head_dim: int, num_q_heads: int, num_kv_heads: in
 def attention_tcgen05(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
                       query_start_loc: torch.Tensor, seq_lens: torch.Tensor, query_lens_host, num_q_heads: int,
                       num_kv_heads: int, head_dim: int, scale: float, window: int = 0, *, joined: bool = False,
-                      sinks: torch.Tensor | None = None, least_tiles: int | None = None) -> None:
+                      sinks: torch.Tensor | None = None, least_tiles: int | None = None, least_query: int = 1) -> None:
     """bfloat16 attention for prompt portions on tcgen05 tensor cores (head size 128, pages of 8, 16, 32, ...
     slots): scores and output accumulate in tensor memory, keys and values come page by page through TMA.
     ``cache`` is ``[pages, 2, kv heads, page, 128]`` (keys, values) or, with ``joined``, ``[pages, 1, kv heads, page, 256]``
     with a token's key and value side by side; ``sinks`` float32 [query heads]: ``exp(sink)`` joins a row's denominator.
     ``query_lens_host`` may be an upper bound; ``least_tiles`` then says how many tiles of 128 rows the step has at least
-    (``StepContext.least_row_tiles``), by which the kernel's variant is chosen."""
+    (``StepContext.least_row_tiles``), by which the kernel's variant is chosen.  ``least_query`` 2: the rows of requests that
+    bring a single token are left as they are (``paged_attention_decode`` with ``query_start_loc`` computes those)."""
     T = q.shape[0]
     planes, row = (1, 2 * head_dim) if joined else (2, head_dim)
     if cache.dim() != 5 or cache.shape[1] != planes or cache.shape[2] != num_kv_heads or cache.shape[4] != row:
@@ -1018,13 +1026,13 @@ def attention_tcgen05(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, b
     if q.stride(1) != 1 or out.stride(1) != 1 or out.shape != (T, num_q_heads * head_dim) or not cache.is_contiguous():
         raise KernelError("attention_tcgen05: q/out rows must be dense, out [T, nq*d], cache contiguous")
     g = num_q_heads // num_kv_heads
-    tiles = sum((n * g + 127) // 128 for n in query_lens_host)
+    tiles = sum((n * g + 127) // 128 for n in query_lens_host if n >= least_query or least_tiles is not None)
     rc = library().cib_attention_tcgen05(
         _cuda(q, "q", contiguous=False), q.stride(0), _cuda(out, "out", contiguous=False), out.stride(0),
         _cuda(cache, "cache"), cache.shape[0], cache.shape[3], _cuda(block_table, "block_table", torch.int32),
         block_table.stride(0), _cuda(query_start_loc, "query_start_loc", torch.int32),
         _cuda(seq_lens, "seq_lens", torch.int32), len(query_lens_host), tiles,
-        tiles if least_tiles is None else min(least_tiles, tiles), num_q_heads, num_kv_heads, head_dim,
+        tiles if least_tiles is None else min(least_tiles, tiles), int(least_query), num_q_heads, num_kv_heads, head_dim,
         float(scale), int(window), 1 if joined else 0, _cuda(sinks, "sinks") if sinks is not None else None,
         _error_flag(q.device).data_ptr(), _stream())
     _check(rc, "attention_tcgen05")

@@ -19,6 +19,12 @@ from .context import PagedKV, StepContext
 
 
 _FORCE_MMA = os.environ.get("CUINFER_B200_ATTENTION", "") == "mma"
+# From how many (request, key head) pairs on the single tokens of a mixed step leave the prompt kernel, where a CTA walks all of a
+# token's keys, for the split-KV one.  A recorded step does not know its contexts, so the line lies where every length gains:
+# recorded for 32 requests of 8 key heads, a portion of 300 tokens beside 23 decoded ones of 300 / 1 100 / 3 500 keys 22.5 / 40.9 /
+# 96.7 us together, 21.0 / 33.3 / 73.5 apart; for 16 requests 12.0 / 22.0 / 56.2 and 17.6 / 22.8 / 43.5; for 4 10.8 / 17.8 / 42.7 and
+# 17.4 / 18.2 / 23.1 (the second launch costs some 5 us).
+SINGLES_APART_MIN_PAIRS = 256
 
 
 def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: PagedKV, ctx: StepContext, num_heads: int,
@@ -27,20 +33,19 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: PagedKV, ctx: Step
     asks for it to be fetched into the L2 when its stream of keys ends."""
     if (qkv.dtype == torch.bfloat16 and ctx.decode_only
             and kernels.paged_attention_decode_supports(head_dim, num_heads, num_kv_heads)):
-        longest = max(1, ctx.max_seq_len)
-        tma = kernels.decode_tma_takes(kv.group.page_size, head_dim, window)
-        splits = kernels.decode_splits(ctx.num_requests, num_kv_heads, longest, kernels.decode_slots(head_dim), tma=tma,
-                                       head_dim=head_dim, group=num_heads // num_kv_heads)
-        tma = tma and kernels.decode_uses_tma(longest, splits)
-        kernels.paged_attention_decode(qkv, out, kv.cache, kv.group.block_table, ctx.seq_lens, num_heads,
-                                       num_kv_heads, head_dim, scale, window, splits, tma=tma, warm=warm)
+        _decode(qkv, out, kv, ctx, num_heads, num_kv_heads, head_dim, scale, window, warm)
         return
     if qkv.dtype == torch.bfloat16 and not _FORCE_MMA and kernels.attention_tcgen05_supports(
             head_dim, num_heads, num_kv_heads, kv.group.page_size) and out.stride(0) % 8 == 0 and qkv.stride(0) % 8 == 0:
         lens = ctx.query_lens_for_launch()
+        apart = (ctx.num_requests * num_kv_heads >= SINGLES_APART_MIN_PAIRS and (ctx.launch_query_lens is not None or 1 in lens)
+                 and kernels.paged_attention_decode_supports(head_dim, num_heads, num_kv_heads))
+        if apart:
+            _decode(qkv, out, kv, ctx, num_heads, num_kv_heads, head_dim, scale, window, None, ctx.query_start_loc)
         kernels.attention_tcgen05(qkv, out, kv.cache, kv.group.block_table, ctx.query_start_loc, ctx.seq_lens, lens,
                                   num_heads, num_kv_heads, head_dim, scale, window,
-                                  least_tiles=ctx.least_row_tiles(num_heads // num_kv_heads, 128))
+                                  least_tiles=ctx.least_row_tiles(num_heads // num_kv_heads, 128, apart),
+                                  least_query=2 if apart else 1)
         return
     if qkv.dtype == torch.bfloat16 and kernels.paged_attention_prefill_supports(head_dim, num_heads, num_kv_heads):
         lens = ctx.query_lens_for_launch()
@@ -50,6 +55,17 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: PagedKV, ctx: Step
     kernels.paged_attention_generic(
         qkv, out, kv.cache, kv.group.block_table, ctx.query_start_loc, ctx.seq_lens, ctx.token_request,
         num_heads, num_kv_heads, head_dim, scale, window)
+
+
+def _decode(qkv, out, kv, ctx, num_heads, num_kv_heads, head_dim, scale, window, warm, query_start_loc=None) -> None:
+    """The split-KV kernel over the step's requests, or over those that bring one token."""
+    longest = max(1, ctx.max_seq_len)
+    tma = kernels.decode_tma_takes(kv.group.page_size, head_dim, window)
+    splits = kernels.decode_splits(ctx.num_requests, num_kv_heads, longest, kernels.decode_slots(head_dim), tma=tma,
+                                   head_dim=head_dim, group=num_heads // num_kv_heads)
+    tma = tma and kernels.decode_uses_tma(longest, splits)
+    kernels.paged_attention_decode(qkv, out, kv.cache, kv.group.block_table, ctx.seq_lens, num_heads,
+                                   num_kv_heads, head_dim, scale, window, splits, tma=tma, warm=warm, query_start_loc=query_start_loc)
 
 
 _FORCE_GENERIC_LATENT = os.environ.get("CUINFER_B200_LATENT_ATTENTION", "") == "generic"

@@ -76,12 +76,15 @@ class StepContext:
         starts = self.query_start_loc_host
         return [starts[i + 1] - starts[i] for i in range(self.num_requests)]
 
-    def least_row_tiles(self, rows_per_token: int, tile_rows: int) -> Optional[int]:
+    def least_row_tiles(self, rows_per_token: int, tile_rows: int, without_single: bool = False) -> Optional[int]:
         """How many row tiles, none of which holds two requests, the step has at least: for choices between kernels that
-        depend on how many CTAs find work.  None where ``query_lens_for_launch`` is exact."""
+        depend on how many CTAs find work.  None where ``query_lens_for_launch`` is exact.  ``without_single``: requests that
+        bring one token have no tiles."""
         if self.launch_query_lens is None or self.launch_least is None:
             return None
         tokens, requests = self.launch_least
+        if without_single:
+            return -(-max(0, tokens - self.num_requests + 1) * rows_per_token // tile_rows)
         return max(requests, -(-tokens * rows_per_token // tile_rows))
 
     def paged_kv(self, run: int) -> PagedKV:

@@ -711,6 +711,32 @@ def test_attention_tcgen05(nq, nkv, ps, window):
     assert not k.attention_tcgen05_supports(128, 8, 8, 5) and not k.attention_tcgen05_supports(128, 8, 8, 4)
 
 
+@pytest.mark.parametrize("nq, nkv, ps, splits", [(16, 8, 16, 1), (16, 8, 16, 4), (32, 2, 64, 16), (16, 1, 8, 5)])
+@pytest.mark.parametrize("wide", [True, False])
+def test_single_tokens_of_a_mixed_step_apart(nq, nkv, ps, splits, wide):
+    """Decoded tokens beside prompt portions: the split-key kernel computes the requests of one token (in clusters, through
+    memory, alone; the first, the last, neighbours), the prompt kernel the others, and neither touches the other's rows."""
+    k = _k()
+    d, lens = 128, [300, 37, 1, 130, 1000, 300, 70, 1000, 128, 513]
+    new = [1, 37, 1, 2, 1, 300, 1, 129, 128, 1]
+    if not wide:
+        lens, new = lens + [1000] * (1 + 420 // nkv), new + [128 * nkv // nq + 1] * (1 + 420 // nkv)
+    case = attention_case(torch.bfloat16, nq, nkv, d, lens, new, ps, seed=82, sharp=True, poison=True)
+    scale = 1.0 / math.sqrt(d)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    q, cache, bt, qsl, sl = case["wide"].to(DEV), case["cache"].to(DEV), case["bt"].to(DEV), i32(case["qsl"]), i32(lens)
+    out = torch.full((sum(new), nq * d), 5.0, dtype=torch.bfloat16, device=DEV)
+    single = torch.tensor([n == 1 for n in new for _ in range(n)], device=DEV)
+    for tma in (False, True):
+        k.paged_attention_decode(q, out, cache, bt, sl, nq, nkv, d, scale, 0, splits, tma=tma, query_start_loc=qsl)
+        assert bool((out[~single] == 5.0).all())
+    before = out.clone()
+    k.attention_tcgen05(q, out, cache, bt, qsl, sl, new, nq, nkv, d, scale, 0, least_query=2)
+    k.check_error_flags(force=True)
+    assert torch.equal(out[single], before[single])
+    close(out, attention_reference(case, lens, new, scale, None), 1.5e-2)
+
+
 @pytest.mark.parametrize("seed", [1, 2])
 def test_attention_tcgen05_random_batches(seed):
     """Drawn batches: 1 to 70 requests (more than the 32 that one pass of the request search takes), portions of 1 to
