@@ -36,6 +36,7 @@ struct Args {
     void* out; int ldo; int M, N, K, up_offset;
     const float* squares_in; int squares_in_n; float eps;      // rows that carry a norm still to be applied, or null
     AnyVec gain; float* stream; float* squares_out;            // kStream; squares_out [M][ceil(N / 32)]
+    const float* bias; int squared_relu;                       // kBf16, kF32: added to every row (or null), then relu(y)^2
     const void* warm; unsigned long long warm_bytes;           // what the kernel after this one reads first (or null)
     int* error_flag;
 };
@@ -132,6 +133,8 @@ gemm_wstream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const int n = n0 + feature;
     float gain = 0.f, old[C];
     if (EPI == kStream && epilogue_thread && n < a.N) gain = a.gain[n];
+    float bias = 0.f;
+    if ((EPI == kBf16 || EPI == kF32) && a.bias != nullptr && epilogue_thread && n < a.N) bias = a.bias[n];
     auto fetch_old = [&](int c) {
 #pragma unroll
         for (int i = 0; i < C; ++i) {
@@ -307,6 +310,11 @@ gemm_wstream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                             if (lane == 0) a.squares_out[(size_t)m * parts + n / 32] = sq;
                         }
                     } else if (ok) {
+                        v[i] += bias;
+                        if (a.squared_relu) {
+                            v[i] = fmaxf(v[i], 0.f);
+                            v[i] *= v[i];
+                        }
                         if (EPI == kF32) reinterpret_cast<float*>(a.out)[(size_t)m * a.ldo + n] = v[i];
                         else reinterpret_cast<__nv_bfloat16*>(a.out)[(size_t)m * a.ldo + n] = __float2bfloat16_rn(v[i]);
                     }
@@ -375,13 +383,14 @@ extern "C" int cib_gemm_wstream_supports(int M, int N, int K) {
 // out[M, N]; 2 = rows [0, N / 2) of w are gates and rows [N / 2, N) the matching ups: out[M, N / 2] = silu(gate) * up in
 // bfloat16; 3 = stream_rows[M, N] (32-bit, dense) += the product, out = bfloat16(stream_rows * gain), squares_out
 // [M][ceil(N / 32)] = the sums of stream_rows^2 over 32 columns each.
+// bias [N] (epilogues 0 and 1, or null) is added to every row; squared_relu: then y = relu(y)^2.
 // squares_in: [M][squares_in_n] (or null): every result row is multiplied by rsqrt(sum(squares_in[row]) / K + eps).
 // warm / warm_bytes: memory that the kernel after this one reads first, or null: fetched into the L2 meanwhile.
 // error_flag: one zero int in device memory.
 extern "C" int cib_gemm_wstream(const void* act, int lda, const void* w, int ldw, void* out, int ldo, int epilogue, int M,
                                 int N, int K, const float* squares_in, int squares_in_n, float eps, float* stream_rows,
-                                const void* gain, int gain_dtype, float* squares_out, const void* warm, long long warm_bytes,
-                                int use_pdl, int* error_flag, cudaStream_t stream) {
+                                const void* gain, int gain_dtype, float* squares_out, const float* bias, int squared_relu,
+                                const void* warm, long long warm_bytes, int use_pdl, int* error_flag, cudaStream_t stream) {
     CIB_REQUIRE(cib_gemm_wstream_supports(M, N, K), "gemm_wstream: M=%d N=%d K=%d is not taken (at most 128 rows, K a multiple of 8)", M, N, K);
     CIB_REQUIRE(lda >= K && ldw >= K && lda % 8 == 0 && ldw % 8 == 0 && ((uintptr_t)act % 16) == 0 && ((uintptr_t)w % 16) == 0,
                 "gemm_wstream: rows must be 16-byte aligned");
@@ -390,6 +399,7 @@ extern "C" int cib_gemm_wstream(const void* act, int lda, const void* w, int ldw
     CIB_REQUIRE(ldo >= (epilogue == ws::kSilu ? N / 2 : N), "gemm_wstream: ldo too small");
     CIB_REQUIRE(epilogue != ws::kStream || (stream_rows != nullptr && gain != nullptr && squares_out != nullptr),
                 "gemm_wstream: the stream epilogue needs the residual, the norm's gains and room for the squares");
+    CIB_REQUIRE((bias == nullptr && !squared_relu) || epilogue == ws::kBf16 || epilogue == ws::kF32, "gemm_wstream: a bias goes with plain rows");
     CIB_REQUIRE(squares_in == nullptr || squares_in_n > 0, "gemm_wstream: sums of squares without parts");
     CUtensorMap mw, mx;
     if (tc_make_map(&mw, w, N, K, ldw, epilogue == ws::kSilu ? 64 : 128, "gemm_wstream") != 0) return -1;
@@ -397,7 +407,7 @@ extern "C" int cib_gemm_wstream(const void* act, int lda, const void* w, int ldw
     if (tc_make_map(&mx, act, M, K, lda, bx, "gemm_wstream") != 0) return -1;
     if (((uintptr_t)warm % 16) != 0 || warm_bytes <= 0) { warm = nullptr; warm_bytes = 0; }
     const ws::Args a = {out, ldo, M, N, K, N / 2, squares_in, squares_in_n, eps, AnyVec{gain, gain_dtype == kBF16}, stream_rows, squares_out,
-                        warm, (unsigned long long)warm_bytes, error_flag};
+                        bias, squared_relu, warm, (unsigned long long)warm_bytes, error_flag};
     switch (bx) {
         case 16: return ws::dispatch<16>(mw, mx, a, epilogue, use_pdl != 0, stream);
         case 32: return ws::dispatch<32>(mw, mx, a, epilogue, use_pdl != 0, stream);

@@ -121,7 +121,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "cib_attention_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P],
         "cib_gemm_skinny": [_P, _I, _I, _I, _P, _I, _P, _P, _I, _P, _I, _F, _P, _P, _I, _I, _I, _I, _I, _P, ctypes.c_longlong, _P, _I, _P, _P, _P],
         "cib_gemm_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, _P],
-        "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, ctypes.c_longlong, _I, _P, _P],
+        "cib_gemm_wstream": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, _I, _P, ctypes.c_longlong, _I, _P, _P],
         "cib_gemm_generic": [_P, _I, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _P],
         "cib_decode_merges_in_cluster": [ctypes.c_longlong, _I, _I, _I, _I],
         "cib_sample": [_P, _I, _I, _I, _P, _P, _P],
@@ -1046,17 +1046,23 @@ def gemm_wstream_supports(M: int, N: int, K: int) -> bool:
 
 def gemm_wstream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, silu_pair: bool = False, *, squares: torch.Tensor | None = None,
                  eps: float = 0.0, stream: torch.Tensor | None = None, gain: torch.Tensor | None = None,
-                 squares_out: torch.Tensor | None = None, warm: torch.Tensor | None = None) -> None:
+                 squares_out: torch.Tensor | None = None, warm: torch.Tensor | None = None, bias: torch.Tensor | None = None,
+                 squared_relu: bool = False) -> None:
     """out[M, N] = a[M, K] @ w[N, K]^T for up to 128 rows on tcgen05 tensor cores with the weights as the streamed
     128-row operand (bfloat16 in, bfloat16 or float32 out).  ``silu_pair``: w holds N/2 gate rows then N/2 up rows and
     out[M, N/2] = silu(gate) * up (bfloat16).
 
     A norm between two products is shared by them as in ``gemm_skinny``: ``stream`` (float32 [M, N], updated in place by the
     product), ``gain`` and ``squares_out`` (float32 [M, ceil(N / 32)]) leave out = bfloat16(stream * gain); ``squares`` and
-    ``eps`` apply the rest of the norm to the product after it.  ``warm``: what the kernel after this one reads first."""
+    ``eps`` apply the rest of the norm to the product after it.  ``warm``: what the kernel after this one reads first.
+    ``bias`` float32 [N] is added in 32 bits; ``squared_relu``: then out = relu(y)^2."""
     M, K = a.shape
     N, K2 = w.shape
     out_cols = N // 2 if silu_pair else N
+    if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N or not bias.is_contiguous()):
+        raise KernelError("gemm_wstream: bias must be contiguous float32 [N]")
+    if (bias is not None or squared_relu) and (silu_pair or stream is not None):
+        raise KernelError("gemm_wstream: a bias goes with plain rows")
     if K != K2 or out.shape != (M, out_cols) or a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise KernelError(f"gemm_wstream: a {list(a.shape)} {a.dtype}, w {list(w.shape)} {w.dtype}, out {list(out.shape)} do not fit")
     if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1 or out.dtype not in (torch.bfloat16, torch.float32):
@@ -1080,6 +1086,7 @@ def gemm_wstream(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, silu_pair:
         _cuda(squares, "squares") if squares is not None else None, squares.shape[1] if squares is not None else 0, float(eps),
         _cuda(stream, "stream") if stream is not None else None, _cuda(gain, "gain") if gain is not None else None,
         _code(gain, "gain") if gain is not None else 0, _cuda(squares_out, "squares_out") if squares_out is not None else None,
+        _cuda(bias, "bias") if bias is not None else None, 1 if squared_relu else 0,
         warm.data_ptr() if warm is not None else None, warm.numel() * warm.element_size() if warm is not None else 0,
         1 if use_pdl else 0, _error_flag(a.device).data_ptr(), _stream())
     _check(rc, "gemm_wstream")

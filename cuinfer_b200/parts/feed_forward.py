@@ -113,12 +113,9 @@ class SquaredReluFeedForward(FeedForward):
         return 2 * self.up.workspace_bytes(tokens) + self.down.workspace_bytes(tokens)
 
     def forward(self, x: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        y = self.up.forward(x)
         if self.up_bias is not None:
-            kernels.bias_rows(y, self.up_bias, y, squared_relu=True)
-            out = self.down.forward(y)
-            kernels.bias_rows(out, self.down_bias, out)
-            return out
+            return self.down.forward_biased(self.up.forward_biased(x, self.up_bias, squared_relu=True), self.down_bias)
+        y = self.up.forward(x)
         act = torch.empty_like(y)
         kernels.relu_squared(y, act)
         return self.down.forward(act)

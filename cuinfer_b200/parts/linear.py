@@ -201,6 +201,20 @@ class Linear:
             return 0
         return kernels.gemm_tcgen05_stream_cols(x.shape[0], *w.shape)
 
+    def forward_biased(self, x: torch.Tensor, bias: torch.Tensor, squared_relu: bool = False) -> torch.Tensor:
+        """``x W^T + bias`` (``bias`` 32-bit), or relu of it squared: in the product's epilogue in decode steps on the
+        weight-streaming kernel, else by a kernel of its own."""
+        from . import gemm_dispatch
+        M = x.shape[0]
+        if (x.dtype == torch.bfloat16 and M <= gemm_dispatch.MANY_ROWS_PLAIN and self._few_rows_kernel(M) == "wstream"
+                and gemm_dispatch.wstream_takes(x, self.weight)):
+            out = torch.empty((M, self.weight.shape[0]), dtype=torch.bfloat16, device=x.device)
+            kernels.gemm_wstream(x, self.weight, out, bias=bias, squared_relu=squared_relu, warm=self.warm_next)
+            return out
+        y = self.forward(x)
+        kernels.bias_rows(y, bias, y, squared_relu=squared_relu)
+        return y
+
     def _few_rows_kernel(self, M: int) -> str:
         """Which kernel multiplies ``M`` plain rows (``gemm_dispatch.few_rows_kernel``), "library" for more than 64."""
         from . import gemm_dispatch

@@ -381,6 +381,21 @@ def test_two_products_share_a_norm(kind, M, N, K, I, gain_dtype):
     k.check_error_flags(force=True)
 
 
+@pytest.mark.parametrize("M, N, K", [(1, 4096, 1024), (9, 1000, 4096), (32, 328, 72), (100, 4100, 512)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gemm_wstream_bias_and_squared_relu(M, N, K, dtype):
+    k = _k()
+    x, w, bias = rand(M, K, seed=70, dtype=torch.bfloat16), rand(N, K, seed=71, scale=0.05, dtype=torch.bfloat16), rand(N, seed=72)
+    want = x.double() @ w.double().T + bias.double()
+    # 32-bit sums as in test_two_products_share_a_norm; the square doubles a relative error
+    tol = (K / 16 + 2) * 2.0 ** -23 if dtype == torch.float32 else 2.0 ** -8
+    for relu in (False, True):
+        out = torch.full((M, N), 7.0, dtype=dtype, device=DEV)
+        k.gemm_wstream(x.to(DEV), w.to(DEV), out, bias=bias.to(DEV), squared_relu=relu)
+        close(out, torch.relu(want) ** 2 if relu else want, 2 * tol)
+    k.check_error_flags(force=True)
+
+
 def test_gemm_skinny_refuses_other_shapes():
     k = _k()
     assert not k.gemm_skinny_supports(17, 64, 64) and not k.gemm_skinny_supports(4, 64, 60)
