@@ -46,11 +46,11 @@ struct TcSmem {
 // PAIR: launched as clusters of two CTAs that share each 256 x BN tile (see the helpers above).  Per 64-k step a CTA
 // then fetches 16 KB of activations and BN / 2 weight rows instead of BN: the kernel is bound by what an SM can fetch
 // from the L2, so fewer bytes per flop is what makes it faster.
-// STREAM: the result joins the 32-bit residual (`map_res`, updated in place) and what is stored to `out` is the new residual times
-// the next norm's gains; `norm.squares_out` [M][tiles along N] gets the sums of the new residual's squares over a tile's columns.  A
-// norm kernel of its own read and wrote 100 MB for 8 192 rows of 1 024 (33 us); here 80 of them pass under the MMAs, in pieces of 32
+// STREAM: the result joins the 32-bit residual (`extra.res`, updated in place) and what is stored to `out` is the new residual times
+// the next norm's gains; `squares_out` [M][tiles along N] gets the sums of the new residual's squares over a tile's columns.  A
+// norm kernel of its own read and wrote 100 MB for 8 192 rows of 1 024 (21 us alone); here 84 of them pass under the MMAs, in pieces of 32
 // columns that a seventh warp brings by TMA before the epilogue needs them and stores behind it.  The product after the norm gets
-// those sums (`norm.squares_in`) and multiplies its rows by rsqrt(mean square + eps).
+// those sums (`squares_in`; NORMED) and multiplies its rows by rsqrt(mean square + eps).
 struct TcNorm {
     const float* squares_in; int squares_in_n; float eps;      // null: rows without a norm
     AnyVec gain; float* squares_out;                           // STREAM
@@ -62,7 +62,7 @@ template <> struct TcExtra<true, false> { CUtensorMap res; TcNorm norm; };
 template <> struct TcExtra<false, false> {};
 
 template <int BN, int STAGES, bool F32OUT, bool TMA_STORE, int SILU = 0, bool PAIR = false, bool STREAM = false, bool NORMED = false>
-__global__ void __launch_bounds__(STREAM ? 224 : 192, STREAM ? 1 : 0)
+__global__ void __launch_bounds__(STREAM ? 224 : 192)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_out, const __grid_constant__ TcExtra<STREAM, NORMED> extra,
                     void* __restrict__ out, int ldo, int M, int N, int K, int up_offset, int* __restrict__ error_flag) {

@@ -11,7 +11,11 @@
 * 128 rows and more (prompt portions): the tcgen05 / TMA / TMEM kernel (``gemm_tcgen05``), with the SiLU gate in its
   epilogue for the gate/up projection — where the product has at least ``TCGEN05_MIN_TILES`` output tiles of
   128 x 128.  With fewer, every CTA walks the whole of K alone and the library, which splits K over more CTAs, measured
-  1.3 to 2.7 times faster (2048 x 1024 x 2048: 8.8 us against 14.9), so those go to cuBLAS;
+  1.3 to 2.7 times faster (2048 x 1024 x 2048: 8.8 us against 14.9), so those go to cuBLAS.  A product on the kernel that is followed by
+  a norm adds to the residual itself; the line is the same: prompt steps of the 0.6B sizes with 2 400 / 2 919 / 3 500 / 4 096 tokens, whose
+  output and down projections have 152 to 256 tiles, 4.11 / 4.81 / 5.72 / 6.07 ms on cuBLAS with norm kernels and 4.85 / 5.45 / 6.27 / 6.17 that
+  way, with 4 700 / 8 192 (296 / 512 tiles) 8.02 / 14.83 and 7.96 / 14.41; of the 8B sizes 600 / 1 024 / 2 048 / 4 096 tokens (160 / 256 / 512 /
+  1 024 tiles) 2.19 / 3.13 / 5.84 / 11.93 and 2.37 / 3.17 / 5.78 / 11.75;
 * in between, and for K that is not a multiple of 8: the library product (cuBLAS via ``torch.mm``; the reference
   calls cuBLAS for every projection, csrc/ops/projection.cu:32-44), or the FMA kernel for shapes cuBLAS's
   tensor-core paths do not take.
@@ -33,7 +37,6 @@ torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 TCGEN05_MIN_ROWS = 128
 TCGEN05_MIN_TILES = 296          # output tiles of 128 x 128 from which the tcgen05 kernel is chosen over the library
-STREAM_MIN_ROWS = 2048           # from here on a product adds to the residual itself and leaves the next norm to its reader
 FEW_ROWS = 16
 MANY_ROWS = 64                   # rows up to which the weight-streaming kernel is taken, and of products on their own
 MANY_ROWS_PLAIN = 32

@@ -153,7 +153,7 @@ class Linear:
         w = self.weight
         M, K = x.shape
         out_cols = w.shape[0] // 2 if silu_pair else w.shape[0]
-        if (M < gemm_dispatch.STREAM_MIN_ROWS or w.dtype != torch.bfloat16 or w.shape[1] != K or (silu_pair and w.shape[0] % 16)
+        if (M <= gemm_dispatch.MANY_ROWS or w.dtype != torch.bfloat16 or w.shape[1] != K or (silu_pair and w.shape[0] % 16)
                 or not gemm_dispatch.shape_takes_tcgen05(M, w, fused=bool(silu_pair))):
             return None
         carried = x.carried()
@@ -197,7 +197,7 @@ class Linear:
         """``kernels.gemm_tcgen05_stream_cols`` where the prompt-sized product of ``x`` may add to the residual, else 0."""
         from . import gemm_dispatch
         w = self.weight
-        if x.shape[0] < gemm_dispatch.STREAM_MIN_ROWS or w.dtype != torch.bfloat16 or not gemm_dispatch.takes_tcgen05(x, w, fused=True):
+        if x.shape[0] <= gemm_dispatch.MANY_ROWS or w.dtype != torch.bfloat16 or not gemm_dispatch.takes_tcgen05(x, w):
             return 0
         return kernels.gemm_tcgen05_stream_cols(x.shape[0], *w.shape)
 
