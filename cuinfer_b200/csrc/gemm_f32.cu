@@ -329,10 +329,11 @@ gemm_f32_tile_kernel(const GemmF32 p) {
 // is; beyond, the three kernels' times are estimated (microseconds, fitted to 9 to 2 048 rows x 64 to 151 936 x 64 to 8 192
 // within 30 %) and the smallest wins:
 //   few rows: 2.5, and a pass of eight rows 1.5 and 0.57 for every warp that an SM has of it
-//   tiles: 0.08 per value of a CTA's K for each CTA that an SM has, alone on it 0.096 (0.135 where every SM has one)
+//   tiles: 0.067 per value of a CTA's K for each CTA that an SM has, alone on it 0.096 (0.115 where every SM has one)
 //   tiles and all sizes: 3 more
 //   all sizes: 0.0535 per value of K for each CTA that an SM has, at least 0.075
-// (64 x 151 936 x 1 024: 1 116, 716 and 972; 64 x 4 096 x 1 024: 46, 53 and 79; 64 x 64 x 64: 18, 8.8 and 7.8; 128 x 2 048 x
+// (64 x 151 936 x 1 024: 1 116, 597 and 972; 64 x 4 096 x 1 024: 44, 49 and 79; 64 x 6 144 x
+// 1 024: 60, 52 and more; 64 x 64 x 64: 18, 8.8 and 7.8; 128 x 2 048 x
 // 512, K a single group of which no cluster can share the work: tiles 51, all sizes 41.)
 constexpr int kFewMaxRows = 64;
 
@@ -374,7 +375,7 @@ int gemm_f32_launch(const GemmF32& p, int batch, cudaStream_t stream) {
     if (!few) {
         const long long tile_ctas = tiles * (split ? groups : 1);
         const float tile_k = split ? (float)(f32_group_slices(p.K) * kF32Slice) : (float)p.K;
-        const float t_tile = 3.f + tile_k * (tile_ctas <= 74 ? 0.096f : tile_ctas <= 148 ? 0.135f : 0.08f * per_sm(tile_ctas));
+        const float t_tile = 3.f + tile_k * (tile_ctas <= 74 ? 0.096f : tile_ctas <= 148 ? 0.115f : 0.067f * per_sm(tile_ctas));
         const long long all_ctas = (long long)((p.N + 63) / 64) * ((p.M + 63) / 64) * batch;
         const float t_all = 3.f + p.K * fmaxf(0.075f, 0.0535f * per_sm(all_ctas));
         const int chunks = (p.K + kFewChunk - 1) / kFewChunk, passes = (p.M + kFewRows - 1) / kFewRows;
