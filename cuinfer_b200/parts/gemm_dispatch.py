@@ -7,7 +7,7 @@
   1 046; of the 0.6B sizes 1 077 us for 20 rows at 700 keys and 1 386 for 64 at 300 (1 326 and 1 451).  One product, weights cold, library / streamed
   / few rows: 8 x 4 096 x 4 096 11.9 / 7.8 / 8.6 us, 8 x 151 936 x 4 096 204 / 182 / 200, 8 x 24 576 x 4 096 34.4 / 35.5 / 37.4, 8 x 4 096 x 1 024
   4.8 / 4.3 / 2.5, 16 x 24 576 x 4 096 34.7 / 35.9 / 47.7; 64 x 6 144 x 4 096 11.3 / 13.5, so from 33 rows on products that share neither a norm
-  nor a gate go to the library;
+  nor a gate go to the library, and from 17 rows on those of them that it multiplies faster (``plain_takes_wstream``);
 * 128 rows and more (prompt portions): the tcgen05 / TMA / TMEM kernel (``gemm_tcgen05``), with the SiLU gate in its
   epilogue for the gate/up projection — where the product has at least ``TCGEN05_MIN_TILES`` output tiles of
   128 x 128.  With fewer, every CTA walks the whole of K alone and the library, which splits K over more CTAs, measured
@@ -58,6 +58,16 @@ def few_rows_kernel(M: int, N: int, K: int) -> str:
     return "skinny" if M <= FEW_ROWS else "library"
 
 
+def plain_takes_wstream(M: int, N: int, K: int, out_dtype: torch.dtype) -> bool:
+    """Whether rows that share neither a norm nor a gate stay on the weight-streaming kernel where ``few_rows_kernel`` says so.  Up
+    to 16 rows always; to 32 rows where the library has to split K and add the parts up in a kernel of its own (at least two
+    of K to a feature, or a few features), and for 32-bit rows; else the library is the faster one.  Inside decode steps of
+    24 rows, streamed less library, us a product: 1 024 x 3 072 -2.4, 2 048 x 6 144 -1.6, 4 096 x 12 288 -2.8, 64 x 2 048 in 32
+    bits -4.7, 32 768 x 4 096 in 32 bits -3; 4 096 x 1 024 +1.7, 6 144 x 1 024 +2.0, 12 288 x 2 048 +2.4, 2 048 x 2 048 between
+    -0.8 and +1.4."""
+    return M <= FEW_ROWS or (M <= MANY_ROWS_PLAIN and (K >= 2 * N or N <= 256 or out_dtype == torch.float32))
+
+
 def wstream_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether the rows of both operands lie as ``gemm_wstream`` fetches them: apart, and on 16-byte boundaries."""
     K = x.shape[1]
@@ -99,7 +109,8 @@ def bf16_matmul_nt(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> 
     N = weight.shape[0]
     if M <= MANY_ROWS_PLAIN and weight.stride(1) == 1 and x.stride(1) == 1:
         choice = few_rows_kernel(M, N, K)
-        if choice == "wstream" and wstream_takes(x, weight) and out.stride(1) == 1 and out.stride(0) >= N:
+        if (choice == "wstream" and plain_takes_wstream(M, N, K, out.dtype) and wstream_takes(x, weight)
+                and out.stride(1) == 1 and out.stride(0) >= N):
             kernels.gemm_wstream(x, weight, out)
             return
         if choice == "skinny" and weight.is_contiguous() and kernels.gemm_skinny_supports(M, N, K):

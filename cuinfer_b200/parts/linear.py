@@ -248,7 +248,7 @@ class Linear:
             if self._few_rows_kernel(M) != "wstream" or silu_pair == "gelu_tanh" or not (lazy or silu_pair):
                 return None           # plain rows: matmul_nt decides
             carried = x.carried() if lazy else None
-            if carried is None and not silu_pair and M > gemm_dispatch.MANY_ROWS_PLAIN:
+            if carried is None and not silu_pair and not gemm_dispatch.plain_takes_wstream(M, N, K, out_dtype):
                 return None           # nothing shared
             rows, squares, eps = carried or (x.materialize() if lazy else x, None, 0.0)
             if rows.dtype != torch.bfloat16 or not gemm_dispatch.wstream_takes(rows, w):

@@ -101,3 +101,23 @@ def test_step_buckets_hold_their_batches_with_little_to_spare():
             assert ctx.least_row_tiles(g, 128) <= tiles <= sum(-(-n * g // 128) for n in ctx.query_lens_for_launch())
     assert len(seen) < 120
     assert ModelRunner.step_bucket([2048], [1]) == (2048, 2, 2) and ModelRunner.step_bucket([8192], [1])[0] == 8192
+
+
+def test_decode_products_that_share_nothing_leave_the_library_only_where_it_is_slower(monkeypatch):
+    """17 to 32 rows whose product has neither a norm nor a gate beside it: streamed where the library has to split K, or for
+    32-bit rows; everything else goes to the library, up to 16 rows nothing does."""
+    from cuinfer_b200.parts import gemm_dispatch
+    streamed = []
+    monkeypatch.setattr(kernels, "gemm_wstream", lambda x, w, out: streamed.append(w.shape))
+    for M, N, K, dtype, own in [(24, 192, 64, torch.bfloat16, True), (32, 256, 512, torch.bfloat16, True), (17, 512, 1024, torch.bfloat16, True),
+                                (24, 512, 512, torch.bfloat16, False), (32, 1024, 256, torch.bfloat16, False), (17, 1024, 1024, torch.bfloat16, False),
+                                (24, 264, 520, torch.bfloat16, False), (33, 512, 1024, torch.bfloat16, False), (24, 1024, 256, torch.float32, True),
+                                (9, 128, 4104, torch.bfloat16, True)]:
+        x, w = torch.ones(M, K, dtype=torch.bfloat16), torch.ones(N, K, dtype=torch.bfloat16)
+        if dtype == torch.bfloat16 or own:                      # (the library's 32-bit store of bfloat16 rows is for CUDA tensors)
+            out = torch.zeros(M, N, dtype=dtype)
+            streamed.clear()
+            gemm_dispatch.bf16_matmul_nt(x, w, out)
+            assert streamed == ([w.shape] if own else []), (M, N, K)
+            assert own or bool((out == K).all())
+        assert gemm_dispatch.plain_takes_wstream(M, N, K, dtype) is own
