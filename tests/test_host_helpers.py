@@ -121,3 +121,23 @@ def test_decode_products_that_share_nothing_leave_the_library_only_where_it_is_s
             assert streamed == ([w.shape] if own else []), (M, N, K)
             assert own or bool((out == K).all())
         assert gemm_dispatch.plain_takes_wstream(M, N, K, dtype) is own
+
+
+def test_gated_decode_products_without_a_shared_norm_are_streamed_up_to_32_rows(monkeypatch):
+    from cuinfer_b200.parts.base import LazyNorm, ResidualStream
+    from cuinfer_b200.parts.linear import Linear
+
+    class PlainNorm:
+        def add_norm(self, stream):
+            return stream.residual.to(torch.bfloat16)
+
+    called = []
+    monkeypatch.setattr(kernels, "gemm_wstream", lambda x, w, out, silu_pair=False, **kw: called.append(("streamed", bool(silu_pair))))
+    monkeypatch.setattr(kernels, "silu_mul", lambda y, act, gelu=False: called.append(("gate", gelu)))
+    product = Linear(["w"], [1024], 256, torch.bfloat16)
+    product.weight = torch.ones(1024, 256, dtype=torch.bfloat16)
+    for M, own in [(17, True), (32, True), (33, False), (64, False)]:
+        for x in (torch.ones(M, 256, dtype=torch.bfloat16), LazyNorm(ResidualStream(torch.ones(M, 256)), PlainNorm())):
+            called.clear()
+            assert product.forward(x, silu_pair=True).shape == (M, 512)
+            assert called == ([("streamed", True)] if own else [("gate", False)]), (M, type(x))
