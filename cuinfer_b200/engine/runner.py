@@ -386,7 +386,7 @@ class ModelRunner:
         lens = tuple(len(e.tokens) for e in entries)
         if sum(lens) < self.STEP_GRAPH_MIN_TOKENS:
             return None
-        key = self.step_bucket(lens, [len(e.want) for e in entries])
+        key = (*self.step_bucket(lens, [len(e.want) for e in entries]), self.model.single_token_class(lens.count(1)))
         if key[0] > self.STEP_GRAPH_MAX_TOKENS:
             return None
         graph = self._step_graphs.get(key)
@@ -706,7 +706,8 @@ class DecodeGraph:
 
 
 class StepGraph:
-    """A CUDA graph of one step of fixed sizes: so many tokens, requests and wanted rows (``ModelRunner.step_bucket``).
+    """A CUDA graph of one step of fixed sizes: so many tokens, requests and wanted rows (``ModelRunner.step_bucket``), and at
+    least so many requests of a single token, where a mixer launches those differently (``DecoderModel.single_token_class``).
 
     Positions, cache slots, block tables, token ids, the requests' boundaries and the indices of the wanted rows are
     data in the graph's own device arena (packed by ``ModelRunner.build_context`` as for an eager step, padded to the
@@ -718,10 +719,10 @@ class StepGraph:
     engine samples from it, on the same stream, before it launches another step.
     """
 
-    def __init__(self, runner: "ModelRunner", key: Tuple[int, int, int]) -> None:
+    def __init__(self, runner: "ModelRunner", key: Tuple[int, int, int, int]) -> None:
         self._runner = weakref.ref(runner)
-        self.key = key
-        T, R, S = key
+        self.key = key                           # ``ModelRunner.step_bucket`` and the class of its single tokens
+        T, R, S = key[:3]
         G = len(runner.groups)
         self.stride = (runner.max_model_len + runner.page_size - 1) // runner.page_size
         total = 3 * T + (R + 1) + 2 * R + S + G * (T + R * self.stride)
@@ -736,9 +737,9 @@ class StepGraph:
         runner = self._runner()
         if runner is None:
             raise RuntimeError("the engine of this step graph is gone")
-        T, R, S = self.key
+        T, R, S, singles = self.key
         wanted = sum(len(e.want) for e in entries)
-        ctx, want = runner.build_context(entries, table_stride=self.stride, arena=self.arena, pad=self.key)
+        ctx, want = runner.build_context(entries, table_stride=self.stride, arena=self.arena, pad=self.key[:3])
         # what a replay cannot know stays off the host side of the context: launches are sized for the worst split of
         # the graph's tokens over its requests (one more 128-row tile than the tokens fill, one tile per further request)
         ctx.query_start_loc_host = None
@@ -746,6 +747,7 @@ class StepGraph:
         ctx.state_slots_host = None
         ctx.launch_query_lens = [T + 128] + [1] * (R - 1)
         ctx.launch_least = runner.step_bucket_least(T, R)
+        ctx.launch_singles = singles
         ctx.max_query_len = T
         ctx.max_seq_len = runner.max_model_len
         if self.graph is not None:

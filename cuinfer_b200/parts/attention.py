@@ -12,7 +12,7 @@ position=PartSpec(...))``; ``scale`` None means ``head_dim ** -0.5``; ``window``
 """
 from __future__ import annotations
 
-from typing import List, Optional
+from typing import List, Optional, Tuple
 
 import torch
 
@@ -88,6 +88,10 @@ class PagedAttention(Mixer):
     @property
     def capturable(self) -> bool:
         return self.position.capturable
+
+    def single_token_lines(self) -> Tuple[int, ...]:
+        line = attention_dispatch.singles_apart_from(self.dtype, self.num_heads, self.num_kv_heads, self.head_dim)
+        return () if line is None else (line,)
 
     def workspace_bytes(self, tokens: int) -> int:
         # q/k/v rows, the attention output, the projection's output

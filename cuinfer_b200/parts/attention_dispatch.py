@@ -11,6 +11,7 @@ portions off the tcgen05 kernel (for comparisons).
 from __future__ import annotations
 
 import os
+from typing import Optional
 
 import torch
 
@@ -19,13 +20,38 @@ from .context import PagedKV, StepContext
 
 
 _FORCE_MMA = os.environ.get("CUINFER_B200_ATTENTION", "") == "mma"
-# From how many (request, key head) pairs on the single tokens of a mixed step leave the prompt kernel, where a CTA walks all of a
-# token's keys, for the split-KV one.  A recorded step does not know its contexts, so the line lies where every length gains:
-# recorded for 32 requests of 8 key heads, a portion of 300 tokens beside 23 decoded ones of 300 / 1 100 / 3 500 keys 22.5 / 40.9 /
-# 96.7 us together, 21.0 / 33.3 / 73.5 apart; for 16 requests 12.0 / 22.0 / 56.2 and 17.6 / 22.8 / 43.5; for 4 10.8 / 17.8 / 42.7 and
-# 17.4 / 18.2 / 23.1 (the second launch costs some 5 us).
-SINGLES_APART_MIN_PAIRS = 256
+# When the single tokens of a mixed step leave the prompt kernel, where a CTA walks all of a token's keys, for the split-KV one.
+# From as many (request, key head) pairs on as the prompt kernel's CTAs of one token no longer fit the 148 SMs at once: recorded
+# for 8 key heads beside three portions of 60 tokens, us a layer for 18 tokens (144 pairs) of 300 / 1 100 / 3 500 keys 64.3 / 75.7 /
+# 108.7 together and 62.8 / 77.4 / 119.0 apart, for 19 (152 pairs) 67.5 / 89.8 / 156.5 and 63.0 / 77.4 / 118.9; for no single
+# token at all the second launch costs 2.3.
+SINGLES_APART_MIN_PAIRS = 149
+# Beside more row tiles than three to an SM the single tokens' CTAs fill the gaps of the portions' when the contexts are short: with
+# 23 of them beside a portion of 3 800 tokens (480 CTAs) 215 / 236 / 299 us a layer together and 221 / 241 / 285 apart (a portion of 3 400:
+# 3 / 9 / 32 less apart).  So apart only where the contexts are known to be long, which a recorded step's are not.
+SINGLES_APART_MAX_CTAS = 3 * 148
+SINGLES_APART_LONG_KEYS = 2048
 
+
+def singles_apart_from(dtype: torch.dtype, num_heads: int, num_kv_heads: int, head_dim: int) -> Optional[int]:
+    """The fewest single tokens of a mixed step that may be computed apart (a recorded step has to say that it has so many)."""
+    if dtype != torch.bfloat16 or _FORCE_MMA or not kernels.paged_attention_decode_supports(head_dim, num_heads, num_kv_heads):
+        return None
+    return -(-SINGLES_APART_MIN_PAIRS // num_kv_heads)
+
+
+def _singles_apart(ctx: StepContext, lens, num_heads: int, num_kv_heads: int, head_dim: int, window: int) -> bool:
+    least = singles_apart_from(torch.bfloat16, num_heads, num_kv_heads, head_dim)
+    if least is None or ctx.least_singles() < least:
+        return False
+    g = num_heads // num_kv_heads
+    tiles = ctx.least_row_tiles(g, 128, True)
+    if tiles is None:
+        tiles = sum(-(-n * g // 128) for n in lens if n > 1)
+    if tiles * num_kv_heads <= SINGLES_APART_MAX_CTAS:
+        return True
+    longest = 0 if ctx.launch_query_lens is not None else max(keys for keys, n in zip(ctx.seq_lens_host, lens) if n == 1)
+    return min(longest, window or longest) >= SINGLES_APART_LONG_KEYS
 
 def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: PagedKV, ctx: StepContext, num_heads: int,
                     num_kv_heads: int, head_dim: int, scale: float, window: int, warm: torch.Tensor | None = None) -> None:
@@ -38,8 +64,7 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: PagedKV, ctx: Step
     if qkv.dtype == torch.bfloat16 and not _FORCE_MMA and kernels.attention_tcgen05_supports(
             head_dim, num_heads, num_kv_heads, kv.group.page_size) and out.stride(0) % 8 == 0 and qkv.stride(0) % 8 == 0:
         lens = ctx.query_lens_for_launch()
-        apart = (ctx.num_requests * num_kv_heads >= SINGLES_APART_MIN_PAIRS and (ctx.launch_query_lens is not None or 1 in lens)
-                 and kernels.paged_attention_decode_supports(head_dim, num_heads, num_kv_heads))
+        apart = _singles_apart(ctx, lens, num_heads, num_kv_heads, head_dim, window)
         if apart:
             _decode(qkv, out, kv, ctx, num_heads, num_kv_heads, head_dim, scale, window, None, ctx.query_start_loc)
         kernels.attention_tcgen05(qkv, out, kv.cache, kv.group.block_table, ctx.query_start_loc, ctx.seq_lens, lens,

@@ -16,7 +16,7 @@ Block           ``forward(stream, ctx, run)``: arranges norms, mixer and feed-fo
 """
 from __future__ import annotations
 
-from typing import List, Optional
+from typing import List, Optional, Tuple
 
 import torch
 
@@ -292,6 +292,12 @@ class Mixer(Part):
     def forward_deferred(self, x: torch.Tensor, ctx: StepContext, run: int):
         """``forward``, whose last product may be left to the next norm (a ``DeferredProduct``)."""
         return self.forward(x, ctx, run)
+
+
+    def single_token_lines(self) -> Tuple[int, ...]:
+        """From how many requests with a single token on the mixer launches a step of several kinds differently: a recorded step
+        of as many or more is another one than a step of fewer."""
+        return ()
 
 
 class FeedForward(Part):

@@ -55,6 +55,7 @@ class StepContext:
     state_slots_host: Optional[List[int]] = field(default_factory=list)
     launch_query_lens: Optional[List[int]] = None      # set for a captured step: see query_lens_for_launch
     launch_least: Optional[Tuple[int, int]] = None     # the fewest (tokens, requests) of a captured step's batches
+    launch_singles: int = 0                            # the fewest requests with a single token of a captured step's batches
     max_query_len: int = 0
     max_seq_len: int = 0
     groups: Dict[int, GroupView] = field(default_factory=dict)
@@ -86,6 +87,12 @@ class StepContext:
         if without_single:
             return -(-max(0, tokens - self.num_requests + 1) * rows_per_token // tile_rows)
         return max(requests, -(-tokens * rows_per_token // tile_rows))
+
+    def least_singles(self) -> int:
+        """How many requests bring a single token, at least in a captured step, exactly in an eager one."""
+        if self.launch_query_lens is not None:
+            return self.launch_singles
+        return self.query_lens_for_launch().count(1)
 
     def paged_kv(self, run: int) -> PagedKV:
         try:

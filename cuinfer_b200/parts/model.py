@@ -51,6 +51,7 @@ class DecoderModel:
         self.tied = spec.lm_head_name is None
         self.lm_head = Linear([spec.lm_head_name or spec.embedding_name], [spec.vocab_size], spec.hidden_size, dtype)
         self._bad_id_flag: Optional[torch.Tensor] = None
+        self._single_lines: Optional[set] = None
 
     # ---- weights ------------------------------------------------------------------------------
     def _embedding_spec(self) -> TensorSpec:
@@ -138,6 +139,13 @@ class DecoderModel:
     def capturable(self) -> bool:
         """True when every part's and block's ``forward`` may be replayed from a CUDA graph (Part.capturable)."""
         return all(block.capturable for block in self.blocks) and all(part.capturable for part in self.parts())
+
+    def single_token_class(self, singles: int) -> int:
+        """The largest line (``Mixer.single_token_lines``) that ``singles`` reaches, 0 below all of them: recorded steps of one
+        class launch the same kernels."""
+        if self._single_lines is None:
+            self._single_lines = {line for block in self.blocks for line in block.mixer.single_token_lines()}
+        return max((line for line in self._single_lines if line <= singles), default=0)
 
     def workspace_bytes(self, tokens: int, rows: int) -> int:
         """Device memory a step of ``tokens`` rows with ``rows`` wanted logits needs beside weights and cache: the

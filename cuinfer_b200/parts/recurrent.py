@@ -571,6 +571,9 @@ class SideBySide(Mixer):
         needs = [m.cache_need() for m in self.sides.values()]
         return needs[0] if needs[0] is not None else needs[1]
 
+    def single_token_lines(self) -> tuple:
+        return tuple(line for m in self.sides.values() for line in m.single_token_lines())
+
     def _state_needs(self, side: str) -> tuple:
         need = self.sides[side].state_need()
         return () if need is None else tuple(need) if isinstance(need, (tuple, list)) else (need,)

@@ -141,3 +141,56 @@ def test_gated_decode_products_without_a_shared_norm_are_streamed_up_to_32_rows(
             called.clear()
             assert product.forward(x, silu_pair=True).shape == (M, 512)
             assert called == ([("streamed", True)] if own else [("gate", False)]), (M, type(x))
+
+
+def test_row_tiles_without_the_requests_of_one_token():
+    """What a recorded step says that it has at least when another kernel takes its single tokens."""
+    from cuinfer_b200.engine.runner import ModelRunner
+    from cuinfer_b200.parts import StepContext
+    rnd = random.Random(4)
+    for _ in range(3000):
+        R = rnd.choice([1, 2, 3, 8, 17, 33, 100, 255])
+        lens = [rnd.choice([1, 1, 1, 1, 2, 7, 60, 500]) for _ in range(R)]
+        Tb, Rb, _ = ModelRunner.step_bucket(lens, [1] * R)
+        ctx = StepContext.__new__(StepContext)
+        ctx.num_requests = Rb
+        ctx.launch_query_lens, ctx.launch_least = [Tb + 128] + [1] * (Rb - 1), ModelRunner.step_bucket_least(Tb, Rb)
+        for g in (1, 2, 4, 16):
+            assert ctx.least_row_tiles(g, 128, True) <= sum(-(-n * g // 128) for n in lens if n > 1), (lens, g)
+    ctx.num_requests, ctx.launch_least = 32, (2017, 16)
+    assert ctx.least_row_tiles(2, 128, True) == 32 and ctx.least_row_tiles(2, 128) == 32 and ctx.least_row_tiles(16, 128, True) == 249
+
+
+def test_single_tokens_of_a_mixed_step_are_computed_apart_only_where_that_pays(monkeypatch):
+    """Recorded steps that do not say that they hold many single tokens launch the prompt kernel alone; so do steps whose single
+    tokens fit the SMs beside the portions, and long portions beside short contexts."""
+    from cuinfer_b200.parts import GroupView, PagedKV, StepContext, attention_dispatch
+    launched = []
+    monkeypatch.setattr(kernels, "attention_tcgen05", lambda *a, least_tiles, least_query: launched.append(("prompt", least_tiles, least_query)))
+    monkeypatch.setattr(kernels, "paged_attention_decode", lambda *a, query_start_loc=None, **kw: launched.append(("single", query_start_loc is not None)))
+    assert attention_dispatch.singles_apart_from(torch.bfloat16, 16, 8, 128) == 19
+    assert attention_dispatch.singles_apart_from(torch.float32, 16, 8, 128) is None
+
+    def kinds(lens, keys=300, recorded=None, window=0):
+        starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32)
+        held = [keys if n == 1 else n for n in lens]
+        ctx = StepContext(starts[-1], len(lens), None, None, None, i32(starts), i32(held), None, query_start_loc_host=starts, seq_lens_host=held,
+                          max_seq_len=max(held))
+        if recorded is not None:
+            ctx.query_start_loc_host = ctx.seq_lens_host = None
+            ctx.num_requests, ctx.launch_singles, ctx.launch_least = 32, recorded, (max(1, sum(lens) - 15), 16)
+            ctx.launch_query_lens = [sum(lens) + 128] + [1] * 31
+        rows = torch.empty(starts[-1], 32 * 128, dtype=torch.bfloat16)
+        kv = PagedKV(torch.empty(2, 2, 8, 16, 128, dtype=torch.bfloat16), GroupView(16, i32([[0]] * len(lens)), None))
+        launched.clear()
+        attention_dispatch.paged_attention(rows, torch.empty(starts[-1], 16 * 128, dtype=torch.bfloat16), kv, ctx, 16, 8, 128, 0.1, window)
+        assert launched[-1][0] == "prompt" and launched[-1][2] == len(launched)
+        return len(launched)
+
+    assert kinds([60] * 24, recorded=0) == 1 and kinds([1] * 18 + [60] * 3, recorded=0) == 1       # (recorded for fewer than 19)
+    assert kinds([1] * 19 + [60] * 3, recorded=19) == 2 and launched == [("single", True), ("prompt", 3, 2)]
+    assert kinds([60] * 24) == 1 and kinds([1] * 18 + [60] * 3) == 1 and kinds([1] * 19 + [60] * 3) == 2
+    # more than three row tiles an SM: by the contexts, where they are known
+    assert kinds([1] * 23 + [3400]) == 2 and kinds([1] * 23 + [5000]) == 1 and kinds([1] * 23 + [5000], keys=2048) == 2
+    assert kinds([1] * 23 + [5000], keys=4000, window=1024) == 1 and kinds([1] * 23 + [3900], recorded=19) == 1

@@ -306,3 +306,66 @@ def test_a_context_of_eight_thousand_tokens(dtype, tmp_path):
             worst = max(worst, err)
             assert err <= TOLERANCE[dtype], f"request {rid}: position {place} is off by {err:.3e} of the largest logit"
     note_error(dtype, "a context of 8 230 tokens", worst)
+
+
+@pytest.mark.parametrize("cuda_graph", [False, True])
+def test_many_decoded_tokens_beside_portions(cuda_graph, tmp_path, monkeypatch):
+    """Steps of 22 requests with eight key heads: prompts alone, fewer decoded tokens than leave the prompt kernel, as many and
+    more beside one and two portions, with exactly one spare token in the recorded steps and with several row tiles; eager and,
+    in the third pass, replayed.  Single tokens go to a kernel of their own only where there are enough of them."""
+    from cuinfer_b200 import kernels
+    from cuinfer_b200.engine.runner import ModelRunner
+    from cuinfer_b200.weights import write_random_model
+    from conftest import GAINS, TINY_D
+
+    monkeypatch.setattr(ModelRunner, "STEP_GRAPH_MIN_TOKENS", 2)
+    cfg = dict(TINY_D, num_hidden_layers=2, hidden_size=128, num_attention_heads=16, num_key_value_heads=8, intermediate_size=256,
+               vocab_size=300, max_position_embeddings=512)
+    folder = str(tmp_path / "model")
+    write_random_model(folder, cfg, 31, std=0.05, gain_std=0.1, dtype="bfloat16", gains=GAINS["bfloat16"])
+    requests = _requests(cfg, [12 + 3 * i for i in range(22)] + [37, 362], seed=31)
+    ids, done, steps = list(requests), {}, []
+
+    def step(takes, end=()):
+        entries = []
+        for rid, n in takes:
+            at = done.get(rid, 0)
+            done[rid] = at + n
+            entries.append({"id": rid, "tokens": requests[rid][at:at + n], "want": [n - 1]})
+        steps.append({"step": len(steps), "entries": entries, "end": list(end)})
+        return len(steps) - 1
+
+    olds, new, long = ids[:22], ids[22], ids[23]
+    step([(r, len(requests[r]) - 6) for r in olds])                          # no single token
+    few = [step([(r, 1) for r in olds[:18]] + [(long, 29)])]                 # 18: 47 tokens, one to spare
+    many = [step([(r, 1) for r in olds] + [(new, 25)]),                      # 22 of 47 tokens
+            step([(r, 1) for r in olds[:19]] + [(new, 10), (long, 18)]),     # 19 of 47
+            step([(r, 1) for r in olds[1:21]] + [(long, 300)])]              # 20 beside five row tiles
+    step([(new, 2), (long, 15)] + [(r, 2) for r in olds], ids)               # no single token again
+    apart, calls = [], [0]
+    original, forward = kernels.paged_attention_decode, ModelRunner.step
+
+    def counted(*args, **kw):
+        calls[0] += kw.get("query_start_loc") is not None
+        return original(*args, **kw)
+
+    def noted(self, entries):
+        calls[0] = 0
+        out = forward(self, entries)
+        apart.append(calls[0])
+        return out
+
+    monkeypatch.setattr(kernels, "paged_attention_decode", counted)
+    monkeypatch.setattr(ModelRunner, "step", noted)
+    out = str(tmp_path / "out")
+    runner = traces.replay_in_process(folder, "bfloat16", steps, out, traces.live_token_peak(steps), 16, cuda_graph=cuda_graph,
+                                      passes=3 if cuda_graph else 1, max_live=32)
+    for i in range(len(steps)):
+        counts = apart[i::len(steps)]
+        assert all(n == 0 for n in counts) if i not in many else counts[0] >= 2, (i, counts)
+    if cuda_graph:                                   # "few" and the first two of "many" share a bucket of sizes
+        assert runner.step_graph_replays >= len(steps) and len(runner._step_graphs) == 5
+        keys = sorted(runner._step_graphs)
+        assert sum(key[:2] == (48, 32) for key in keys) == 2 and {key[3] for key in keys} == {0, 19}
+    traces.compare_with_plain(folder, requests, traces.collect(steps, out, cfg["vocab_size"]), TOLERANCE["bfloat16"],
+                              label="decoded tokens beside portions")
