@@ -9,7 +9,7 @@ what is compared is one design against the other at the same sizes, and every ke
 
 Kernel times are taken in place: while one eager step runs, every call through ``cuinfer_b200.kernels`` is made once
 for its result and then repeated between two CUDA events on the same arguments (the repeats change nothing that later
-kernels read differently: a norm that adds into the residual is repeated on a copy).  The roofline of a call is the larger
+kernels read differently: a norm or a product that adds into the residual is repeated on a copy).  The roofline of a call is the larger
 of its algorithmic bytes over the measured copy bandwidth and its FLOPs over the measured bfloat16 peak
 (``MEASURED_PEAKS.json``, else the fallback figures).
 """
@@ -218,12 +218,17 @@ class KernelTimes:
                 rep_args = (args[0].clone(),) + tuple(args[1:])
             if name == "bias_rows":                                                                # may run in place
                 rep_args = (args[0], args[1], torch.empty_like(args[2]))
+            rep_kw = kw
+            if kw.get("stream") is not None:                       # a product that adds to the residual: rows, sums and residual of its own
+                at = 1 if name == "gemm_skinny" else 2
+                rep_args = args[:at] + (torch.empty_like(args[at]),) + args[at + 1:]
+                rep_kw = dict(kw, stream=kw["stream"].clone(), squares_out=torch.empty_like(kw["squares_out"]))
             # the repeats are recorded into a CUDA graph and the graph is timed: the device's time, not Python's
             torch.cuda.synchronize()
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph):
                 for _ in range(self.reps):
-                    fn(*rep_args, **kw)
+                    fn(*rep_args, **rep_kw)
             graph.replay()
             torch.cuda.synchronize()
             a.record()
@@ -314,9 +319,9 @@ class KernelTimes:
                 (2.0 * h.shape[0] * table.shape[1] * (gate_up.shape[1] + down.shape[2]) * h.shape[1],
                  min(h.shape[0] * table.shape[1], gate_up.shape[0]) * (gate_up.shape[1] + down.shape[2]) * h.shape[1] * 2 + 3 * _nbytes(h)),
             "gemm_generic_batched": lambda a, w, out, **k: (2.0 * a.shape[0] * a.shape[1] * a.shape[2] * w.shape[1], _nbytes(a, w, out)),
-            "gemm_tcgen05": lambda a, w, out, **k: (2.0 * a.shape[0] * a.shape[1] * w.shape[0], _nbytes(a, w, out)),
-            "gemm_skinny": lambda w, out, **k: (2.0 * out.shape[0] * w.shape[0] * w.shape[1], _nbytes(w, out)),
-            "gemm_wstream": lambda a, w, out, **k: (2.0 * a.shape[0] * a.shape[1] * w.shape[0], _nbytes(a, w, out)),
+            "gemm_tcgen05": lambda a, w, out, *p, **k: (2.0 * a.shape[0] * a.shape[1] * w.shape[0], _nbytes(a, w, out) + 2 * _nbytes(k.get("stream"))),
+            "gemm_skinny": lambda w, out, **k: (2.0 * out.shape[0] * w.shape[0] * w.shape[1], _nbytes(w, out) + 2 * _nbytes(k.get("stream"))),
+            "gemm_wstream": lambda a, w, out, *p, **k: (2.0 * a.shape[0] * a.shape[1] * w.shape[0], _nbytes(a, w, out) + 2 * _nbytes(k.get("stream"))),
         }
         for name, cost in costs.items():
             self._saved[name] = getattr(kernels, name)

@@ -1016,3 +1016,29 @@ def test_gated_epilogues_agree_on_large_gates():
             fn(x[:M].to(DEV), w.to(DEV), out, silu_pair=True)
         assert bool(torch.isfinite(out.float()).all())
         close(out, want[:M], 4e-3)
+
+
+@pytest.mark.parametrize("kind, M, N, K", [("gemm_skinny", 4, 256, 128), ("gemm_wstream", 20, 256, 128), ("gemm_tcgen05", 2400, 1000, 72)])
+def test_timed_products_that_add_to_the_residual_add_once(kind, M, N, K):
+    """``bench_designs.KernelTimes`` repeats every call for its time; what the step goes on with is the one call's result."""
+    from cuinfer_b200.bench_designs import KernelTimes
+    k = _k()
+    x, w, gain = rand(M, K, seed=90, dtype=torch.bfloat16).to(DEV), rand(N, K, seed=91, dtype=torch.bfloat16).to(DEV), rand(N, seed=92).to(DEV)
+    cols = {"gemm_skinny": 16, "gemm_wstream": 32}.get(kind) or k.gemm_tcgen05_stream_cols(M, N, K)
+
+    def product():
+        stream, rows = rand(M, N, seed=93).to(DEV), torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        squares = torch.empty(M, -(-N // cols), device=DEV)
+        if kind == "gemm_skinny":
+            k.gemm_skinny(w, rows, act=x, norm_weight=gain, stream=stream, squares_out=squares)
+        else:
+            getattr(k, kind)(x, w, rows, stream=stream, gain=gain, squares_out=squares)
+        return stream, rows, squares
+
+    want = product()
+    with KernelTimes({"q": [M], "k": [M]}, reps=2) as times:
+        got = product()
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
+    assert len(times.rows) == 1 and times.rows[0]["kernel"] == kind and times.rows[0]["bytes"] >= 2 * 4 * M * N
+    k.check_error_flags(force=True)
