@@ -490,6 +490,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
 }
 
+// CUINFER_B200_GEMM_PAIR=0 keeps one CTA per tile, for comparisons (and no product adds to the residual: that takes pairs).
+static bool pair_allowed() {
+    static const bool allowed = [] { const char* e = getenv("CUINFER_B200_GEMM_PAIR"); return !(e && e[0] == '0'); }();
+    return allowed;
+}
+
 static int make_map(CUtensorMap* map, const void* base, int rows, int K, int ld, int box_rows) {
     return tc_make_map(map, base, rows, K, ld, box_rows, "gemm_tcgen05");
 }
@@ -564,7 +570,7 @@ extern "C" int cib_gemm_tcgen05_supports(int M, int N, int K) {
 // The columns of a tile of the product that adds to the residual (squares_out has ceil(N / that) sums a row), or 0 where it does not
 // take the shape: it runs as pairs of CTAs.
 extern "C" int cib_gemm_tcgen05_stream_cols(int M, int N, int K) {
-    if (!cib_gemm_tcgen05_supports(M, N, K) || M < 256 || N % 8 != 0) return 0;
+    if (!cib_gemm_tcgen05_supports(M, N, K) || !pair_allowed() || M < 256 || N % 8 != 0) return 0;
     const int m_pairs = (M + 255) / 256;
     if (m_pairs * ((N + 127) / 128) < 74) return 0;
     return N % 256 == 0 && (N / 256) * m_pairs >= 60 ? 256 : 128;
@@ -587,11 +593,10 @@ extern "C" int cib_gemm_tcgen05(const void* a, int lda, const void* w, int ldw, 
     CIB_REQUIRE(squares_in == nullptr || (squares_in_n > 0 && ((uintptr_t)squares_in % 16) == 0), "gemm_tcgen05: sums of squares without parts, or not on 16 bytes");
     const TcNorm norm = {squares_in, squares_in_n, eps, AnyVec{gain, gain_dtype == kBF16}, squares_out};
     CUtensorMap ma, mw;
-    // From 256 rows on, pairs of CTAs share 256-row tiles (CUINFER_B200_GEMM_PAIR=0 keeps one CTA per tile, for comparisons).
-    static const bool pair_allowed = [] { const char* e = getenv("CUINFER_B200_GEMM_PAIR"); return !(e && e[0] == '0'); }();
+    // From 256 rows on, pairs of CTAs share 256-row tiles
     // (only when there are enough 256-row tiles for every pair of SMs: with fewer, one CTA per 128-row tile measured faster)
     const int pair_tiles = ((M + 255) / 256) * (((silu_pair ? N / 2 : N) + 127) / 128);
-    const bool pair = pair_allowed && M >= 256 && pair_tiles >= 74;
+    const bool pair = pair_allowed() && M >= 256 && pair_tiles >= 74;
     if (stream_rows != nullptr) {
         const int bn = cib_gemm_tcgen05_stream_cols(M, N, K);
         CIB_REQUIRE(bn > 0 && !out_f32 && !silu_pair && gain != nullptr && squares_out != nullptr && ldo % 8 == 0 && ((uintptr_t)out % 16) == 0 &&

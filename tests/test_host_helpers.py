@@ -2,7 +2,10 @@
 sampling, the size limit of the L2 hints."""
 from __future__ import annotations
 
+import os
 import random
+import subprocess
+import sys
 
 import torch
 
@@ -194,3 +197,11 @@ def test_single_tokens_of_a_mixed_step_are_computed_apart_only_where_that_pays(m
     # more than three row tiles an SM: by the contexts, where they are known
     assert kinds([1] * 23 + [3400]) == 2 and kinds([1] * 23 + [5000]) == 1 and kinds([1] * 23 + [5000], keys=2048) == 2
     assert kinds([1] * 23 + [5000], keys=4000, window=1024) == 1 and kinds([1] * 23 + [3900], recorded=19) == 1
+
+
+def test_no_product_runs_as_pairs_of_ctas_when_they_are_switched_off():
+    code = "from cuinfer_b200 import kernels; print(kernels.gemm_tcgen05_stream_cols(8192, 1024, 1024))"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    cols = [subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, CUINFER_B200_GEMM_PAIR=on), capture_output=True, text=True,
+                           timeout=600, check=True).stdout.split() for on in ("1", "0")]
+    assert cols == [["256"], ["0"]]
