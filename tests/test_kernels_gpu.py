@@ -1042,3 +1042,44 @@ def test_timed_products_that_add_to_the_residual_add_once(kind, M, N, K):
         assert torch.equal(a, b)
     assert len(times.rows) == 1 and times.rows[0]["kernel"] == kind and times.rows[0]["bytes"] >= 2 * 4 * M * N
     k.check_error_flags(force=True)
+
+
+@pytest.mark.parametrize("kind, M, N, K, I", [
+    ("skinny", 5, 2560, 4096, 640), ("skinny", 9, 2560, 4096, 640), ("skinny", 16, 2000, 2088, 640),
+    ("skinny", 16, 2088, 2088, 2400), ("skinny", 9, 4800, 2088, 40), ("skinny", 3, 4800, 2088, 2400),
+    ("tcgen05", 4900, 1024, 72, 600), ("tcgen05", 8257, 1024, 1032, 1536)])
+def test_two_products_share_a_norm_at_longer_slices_and_more_tiles(kind, M, N, K, I):
+    """As above where a few-rows CTA's slice of K takes more than two chunks, without a cluster (75 to 296 row tiles, eight rows
+    and sixteen, whose activations have one buffer) and with two row tiles a CTA; and residual tiles of 256 columns with four sums
+    a row, several tiles a worker, rows that end inside the first and the second half of a pair."""
+    for gain_dtype in (torch.bfloat16, torch.float32)[:1 if kind == "tcgen05" else 2]:
+        test_two_products_share_a_norm(kind, M, N, K, I, gain_dtype)
+
+
+@pytest.mark.parametrize("N, K", [(2560, 4096), (2000, 2088), (4800, 2088), (1024, 3072), (1184, 2048), (48, 96)])
+def test_few_rows_results_do_not_depend_on_the_rows_beside_them(N, K):
+    """Every row of 16 and of 5 as it is alone, bit for bit, in every epilogue."""
+    k = _k()
+    x, w = rand(16, K, seed=95, dtype=torch.bfloat16).to(DEV), rand(N, K, seed=96, scale=0.05, dtype=torch.bfloat16).to(DEV)
+    gain, squares = rand(N, seed=97).to(DEV), rand(16, 5, seed=98).abs().to(DEV)
+
+    def products(rows):
+        m = rows.numel()
+        out = {}
+        for name, dtype, cols, kw in [("bf16", torch.bfloat16, N, {}), ("f32", torch.float32, N, {}),
+                                      ("normed", torch.float32, N, dict(squares=squares[rows], eps=1e-5)),
+                                      ("gated", torch.bfloat16, N // 2, dict(silu_pair=True, squares=squares[rows], eps=1e-5))]:
+            out[name] = torch.empty(m, cols, dtype=dtype, device=DEV)
+            k.gemm_skinny(w, out[name], act=x[rows], **kw)
+        out["stream"], out["rows"] = rand(16, N, seed=99).to(DEV)[rows], torch.empty(m, N, dtype=torch.bfloat16, device=DEV)
+        out["squares"] = torch.empty(m, -(-N // 16), device=DEV)
+        k.gemm_skinny(w, out["rows"], act=x[rows], norm_weight=gain, stream=out["stream"], squares_out=out["squares"])
+        return out
+
+    rows = torch.arange(16, device=DEV)
+    whole, five = products(rows), products(rows[:5])
+    for r in (0, 4, 7, 8, 15):
+        alone = products(rows[r:r + 1])
+        for name, values in alone.items():
+            assert torch.equal(values[0], whole[name][r]), (name, r)
+            assert r >= 5 or torch.equal(values[0], five[name][r]), (name, r)

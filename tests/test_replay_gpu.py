@@ -369,3 +369,48 @@ def test_many_decoded_tokens_beside_portions(cuda_graph, tmp_path, monkeypatch):
         assert sum(key[:2] == (48, 32) for key in keys) == 2 and {key[3] for key in keys} == {0, 19}
     traces.compare_with_plain(folder, requests, traces.collect(steps, out, cfg["vocab_size"]), TOLERANCE["bfloat16"],
                               label="decoded tokens beside portions")
+
+
+def test_products_that_share_norms_through_the_engine(tmp_path):
+    """A prompt step of as many output tiles as the products that add to the residual are chosen from (1 300 tokens: pairs of
+    tiles, the last one with 20 rows), prompts of a few, and decode steps of 1, 20 and 40 requests, replayed, against the plain
+    implementation; with counts of the products that added to the residual in place."""
+    from cuinfer_b200 import kernels
+    from cuinfer_b200.parts import gemm_dispatch
+    from cuinfer_b200.weights import write_random_model
+    from conftest import GAINS, TINY_D
+
+    H, heads, kv, I = 3456, 24, 2, 256
+    cfg = dict(TINY_D, num_hidden_layers=2, hidden_size=H, num_attention_heads=heads, num_key_value_heads=kv, intermediate_size=I,
+               vocab_size=300, max_position_embeddings=2048)
+    assert 11 * (H // 128) >= gemm_dispatch.TCGEN05_MIN_TILES > 10 * (H // 128)
+    folder = str(tmp_path / "model")
+    write_random_model(folder, cfg, 41, std=0.02, gain_std=0.1, dtype="bfloat16", gains=GAINS["bfloat16"])
+    requests = _requests(cfg, [1303] + [9 + i % 7 for i in range(40)], seed=41)
+    ids, steps = list(requests), []
+
+    def step(takes, end=()):
+        steps.append({"step": len(steps), "end": list(end), "entries": [
+            {"id": rid, "tokens": requests[rid][lo:hi], "want": sorted({0, (hi - lo) // 2, hi - lo - 1})} for rid, lo, hi in takes]})
+
+    step([(ids[0], 0, 1300)])
+    for i in range(3):
+        step([(ids[0], 1300 + i, 1301 + i)], ids[:1] if i == 2 else ())
+    step([(r, 0, len(requests[r]) - 4) for r in ids[1:]])
+    for i in range(4):
+        live = ids[1:41] if i % 2 == 0 else ids[1:21]
+        step([(r, len(requests[r]) - 4 + done, len(requests[r]) - 3 + done) for r in live for done in [i if r in ids[1:21] else i // 2]])
+    steps[-1]["end"] = ids[1:]
+    streams = {"gemm_skinny": 0, "gemm_wstream": 0, "gemm_tcgen05": 0}
+    with pytest.MonkeyPatch.context() as patch:
+        for name in streams:
+            def counted(*args, _name=name, _call=getattr(kernels, name), **kw):
+                streams[_name] += kw.get("stream") is not None
+                return _call(*args, **kw)
+            patch.setattr(kernels, name, counted)
+        out = str(tmp_path / "out")
+        traces.replay_in_process(folder, "bfloat16", steps, out, traces.live_token_peak(steps), 16, cuda_graph=True, max_live=64)
+    # two layers' output projection and feed-forward, but for the last one, whose rows the output head gathers
+    assert streams["gemm_tcgen05"] == 3 and streams["gemm_skinny"] >= 2 * 3 and streams["gemm_wstream"] >= 2 * 2 * 3, streams
+    traces.compare_with_plain(folder, requests, traces.collect(steps, out, cfg["vocab_size"]), TOLERANCE["bfloat16"],
+                              label="products that share norms")
