@@ -592,7 +592,9 @@ static int dispatch_skinny(SkinnyArgs& a, int epilogue, int use_pdl, cudaStream_
 
 using namespace cib;
 
-// with_norm: the activations are normalised in the kernel (needs room for the 32-bit rows as well).
+// with_norm: the activations are normalised in the kernel, which keeps them in shared memory, the 32-bit rows as well.  Plain
+// rows need no such room; the limit on their K (about 6 000 for 16 rows, 12 000 for 8) is part of what callers of the kernel
+// rely on being refused; the engine gives it 4 096 at most (more only for fewer than eight features).
 extern "C" int cib_gemm_skinny_supports(int M, int N, int K, int with_norm) {
     if (!(M >= 1 && M <= 16 && N >= 1 && K >= 32 && K % 8 == 0)) return 0;
     const size_t rows = M <= 8 ? 8 : 16;

@@ -504,7 +504,8 @@ template <int BN, int STAGES, bool F32OUT, bool TMA_STORE, int SILU = 0, bool PA
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mo, const TcNorm& norm, void* out, int ldo, int M,
                      int N, int K, int* error_flag, cudaStream_t stream, int up_offset = 0, const CUtensorMap* mr = nullptr) {
     // (a kernel of its own for rows that carry a norm: two more multiplications a value cost the gated epilogue, which its tiles wait
-    // for, 1.6 us a layer at 2 048 rows)
+    // for, 1.6 us a layer at 2 048 rows.  All stores and tile forms have it: a reader of such rows may have few features, a number of
+    // them that is not a multiple of eight, or 32-bit results)
     if constexpr (!NORMED && !STREAM)
         if (norm.squares_in != nullptr)
             return launch_tc<BN, STAGES, F32OUT, TMA_STORE, SILU, PAIR, STREAM, true>(ma, mw, mo, norm, out, ldo, M, N, K, error_flag, stream, up_offset, mr);

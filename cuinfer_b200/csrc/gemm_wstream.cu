@@ -19,8 +19,11 @@
 //     holds 64 gate features and the 64 matching up features), or the residual and the next norm's rows (`stream`: see
 //     gemm_skinny.cu, whose description of a norm shared by two products holds here too).
 //
-// Every mbarrier wait is bounded; on a time-out the kernel raises the error flag, skips its stores, frees its tensor
-// memory and returns.
+// The engine takes it up to 64 rows; 65 to 128 rows (one CTA an SM) are for callers of the kernel itself: the library is faster there.
+//
+// Every mbarrier wait is bounded; on a time-out the kernel raises the error flag, frees its tensor memory and returns.  The CTA
+// whose wait ran out stores nothing; the others of its cluster have its unfinished sums among theirs, so no row of a flagged launch
+// counts, the residual's neither.
 #include "tcgen05_utils.cuh"
 
 #include "mma_utils.cuh"
@@ -340,8 +343,8 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& a, i
     return 0;
 }
 
-// K is split over the CTAs of a cluster until there is about a CTA for every SM, as long as every one keeps two steps.  By the
-// weight's sizes alone: a row's result does not depend on how many rows are beside it.
+// K is split over the CTAs of a cluster until there is about a CTA for every SM, as long as there are two steps a CTA (the shares are
+// rounded up, so the last CTAs may have less, or none: 17 steps over eight are 3, 3, 3, 3, 3, 2, 0, 0).  By the weight's sizes alone: a row's result does not depend on how many rows are beside it.
 static int k_splits(int n_out, int K, bool pair) {
     const int tiles = (n_out + (pair ? 63 : 127)) / (pair ? 64 : 128), steps = (K + kTcBK - 1) / kTcBK;
     int s = 1;

@@ -21,7 +21,8 @@
   tensor-core paths do not take.
 
 ``CUINFER_B200_GEMM=cublas`` sends every product of more than 16 rows to the library, ``CUINFER_B200_GEMM=tcgen05`` every
-prompt-sized one that the kernel takes to the kernel (for comparisons).
+prompt-sized one that the kernel takes to the kernel (for comparisons); ``own`` (decode products of up to 16 rows on this
+package's kernels) asks for what is always so.
 """
 from __future__ import annotations
 

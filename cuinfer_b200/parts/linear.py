@@ -172,8 +172,8 @@ class Linear:
 
     def into_stream(self, x: torch.Tensor, residual: torch.Tensor, gain: torch.Tensor) -> Optional[tuple]:
         """Add the product of ``x`` to the 32-bit ``residual`` in place; ``(rows, squares)``: the new residual times ``gain`` in
-        bfloat16 and the sums of its squares over 16 columns each, from the product's own kernel.  None where it does not
-        take the shape (nothing has happened then)."""
+        bfloat16 and parts of the sums of its squares (over 16, 32, 128 or 256 columns each, by the kernel), from the product's own
+        kernel.  None where it does not take the shape (nothing has happened then)."""
         M, N = residual.shape
         from . import gemm_dispatch
         if (x.dtype != torch.bfloat16 or not gemm_dispatch.wstream_takes(x, self.weight) or not residual.is_contiguous()

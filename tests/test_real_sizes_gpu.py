@@ -2,8 +2,8 @@
 the Qwen3-0.6B, 8B and 32B shapes (hidden 1024 / 4096 / 5120, 16-8 / 32-8 / 64-8 heads of 128, feed-forward 3072 /
 12288 / 25600, vocabulary 151 936, tied / untied) through the replay path, against the plain implementation on the
 CPU.  Fewer layers than the shapes have (2 of 28 / 36 / 64), not smaller layers: every projection, the attention
-and the output head take the kernels that the dispatch rules choose at these sizes — the norm folded into the
-few-rows projection up to K = 2048, the plain few-rows kernel at 4096, the weight-streaming kernel above, CTA-pair
+and the output head take the kernels that the dispatch rules choose at these sizes — the few-rows kernel (weights under
+24 MB, K up to 4096) and the weight-streaming one in decode steps, each sharing the norms with the product on the other side, CTA-pair
 tiles and the library product for prompt-sized steps, the 151 936-wide head — in the order a benchmark step runs them.
 """
 from __future__ import annotations
