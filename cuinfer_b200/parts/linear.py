@@ -206,8 +206,8 @@ class Linear:
         weight-streaming kernel, else by a kernel of its own."""
         from . import gemm_dispatch
         M = x.shape[0]
-        if (x.dtype == torch.bfloat16 and M <= gemm_dispatch.MANY_ROWS_PLAIN and self._few_rows_kernel(M) == "wstream"
-                and gemm_dispatch.wstream_takes(x, self.weight)):
+        if (isinstance(x, torch.Tensor) and x.dtype == torch.bfloat16 and M <= gemm_dispatch.MANY_ROWS_PLAIN
+                and self._few_rows_kernel(M) == "wstream" and gemm_dispatch.wstream_takes(x, self.weight)):
             out = torch.empty((M, self.weight.shape[0]), dtype=torch.bfloat16, device=x.device)
             kernels.gemm_wstream(x, self.weight, out, bias=bias, squared_relu=squared_relu, warm=self.warm_next)
             return out

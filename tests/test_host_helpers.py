@@ -205,3 +205,16 @@ def test_no_product_runs_as_pairs_of_ctas_when_they_are_switched_off():
     cols = [subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, CUINFER_B200_GEMM_PAIR=on), capture_output=True, text=True,
                            timeout=600, check=True).stdout.split() for on in ("1", "0")]
     assert cols == [["256"], ["0"]]
+
+
+def test_a_product_with_a_bias_takes_a_norm_that_has_not_been_computed(monkeypatch):
+    """As every projection does: the rows are normed first."""
+    from cuinfer_b200.parts.base import LazyNorm, ResidualStream
+    from cuinfer_b200.parts.linear import Linear
+    added = []
+    monkeypatch.setattr(Linear, "forward", lambda self, x: torch.zeros(x.shape[0], 8192, dtype=torch.bfloat16))
+    monkeypatch.setattr(kernels, "bias_rows", lambda y, bias, out, squared_relu=False: added.append((tuple(y.shape), squared_relu)))
+    product = Linear(["w"], [8192], 4096, torch.bfloat16)
+    product.weight = torch.zeros(8192, 4096, dtype=torch.bfloat16)
+    product.forward_biased(LazyNorm(ResidualStream(torch.zeros(3, 4096)), None), torch.zeros(8192), squared_relu=True)
+    assert added == [((3, 8192), True)]
